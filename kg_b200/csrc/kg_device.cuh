@@ -62,6 +62,9 @@ __device__ __forceinline__ long long off3(const Grid& g, int ii, int jj, int k) 
 __device__ __forceinline__ int off2(const Grid& g, int ii, int jj) { return jj * g.PI + ii; }
 
 __device__ __forceinline__ double2 ldf(const double2* __restrict__ f, long long o) { return __ldg(f + o); }
+// state data in a kernel that may start under the tail of the one that writes it:
+// not the read-only path, which wants data that no one writes while the kernel lives
+__device__ __forceinline__ double2 lds(const double2* f, long long o) { return f[o]; }
 __device__ __forceinline__ double ldm(const double* __restrict__ t, int o) { return __ldg(t + o); }
 
 // one-sided and centred building blocks, written exactly as the Fortran

@@ -161,11 +161,10 @@ __global__ void __launch_bounds__(NTH, 2)
   const bool vcol = c >= 0 && c <= n;
   const bool own = vcol && tx >= 1 && tx <= FO;
   const int k0 = blockIdx.z * a.kchunk;
-  if (k0 >= g.NK) return;
   const int k1 = min(k0 + a.kchunk, g.NK);
   const int NP = (k1 - k0) + 2;
   const long long fs = g.fs;
-  const double2* __restrict__ U = a.U;
+  const double2* U = a.U;
 
   if (tid == 0) {
     for (int s = 0; s < NSTF; ++s) mbar_init(&bars[s], 1);
@@ -508,7 +507,7 @@ bool encode_box(CUtensorMap* tm, const Grid& g, const double2* base, int nvars, 
 }
 
 template <int MK>
-int fused_launch(const CUtensorMap* tms, const FusedArgs& a, cudaStream_t st) {
+int fused_launch(const CUtensorMap* tms, FusedArgs a, cudaStream_t st) {
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(pirk_s1_fused_kernel<MK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) !=
@@ -518,7 +517,9 @@ int fused_launch(const CUtensorMap* tms, const FusedArgs& a, cudaStream_t st) {
   }
   const Grid& g = a.g;
   const int tiles_x = (g.NI <= FO) ? 1 : (g.NI + FO - 1) / FO;
-  dim3 grid(tiles_x, (g.NJ + FJ - 1) / FJ, (g.NK + a.kchunk - 1) / a.kchunk);
+  dim3 grid(tiles_x, (g.NJ + FJ - 1) / FJ, 1);
+  a.kchunk = phi_chunk(g.NK, (long long)grid.x * grid.y, 148 * 2, 64);
+  grid.z = (g.NK + a.kchunk - 1) / a.kchunk;
   pirk_s1_fused_kernel<MK><<<grid, dim3(FL, FJ, 1), SMEM, st>>>(tms[0], tms[1], tms[2], tms[3], a);
   return 0;
 }
@@ -542,9 +543,7 @@ int launch_pirk_s1_fused(const Grid& g, const Metric& m, int mk, const double2* 
   a.S = S;
   a.Snew = Snew;
   a.err = err;
-  // long chunks: each chunk reads two planes beyond its own
-  const int nch = (g.NK + 63) / 64;
-  a.kchunk = (g.NK + nch - 1) / nch;
+  a.kchunk = 0;  // set at the launch, from the tiles of the grid
   return mk == MK_KS ? fused_launch<MK_KS>(tms, a, st) : fused_launch<MK_SCHW>(tms, a, st);
 }
 

@@ -113,7 +113,6 @@ struct MxArgs {
   Grid g;
   Metric m;
   const double* rsg;
-  const void* in;       // stencil input, 5 variables (stride g.fs complex): double2 in stage 1, float2 after
   const double2* base;  // u^n
   float2* acc;          // k1 + 2 k2 + 2 k3
   float2* outf;         // next stage input (stages 1-3)
@@ -145,8 +144,6 @@ __device__ __forceinline__ void mx_rhs(const MxArgs& a, const TIN* cu, const dou
                                        double2 Fpv, double2 Fnx, cx<R> r[5]) {
   constexpr int FIELD_E = MGeom<TJ>::FIELD_E, MT_N = MGeom<TJ>::MT_N;
   const Grid& g = a.g;
-  const Metric& M = a.m;
-  const TIN* gin = reinterpret_cast<const TIN*>(a.in);
   const R al = (R)own[0], be = (R)own[1], dxb = (R)own[2], sg = (R)own[3], rs = (R)own[4], am2 = (R)own[5];
   const R rdx = (R)g.rdx, rdy = (R)g.rdy, rdz = (R)g.rdz;
   const int n = g.NI - 1;
@@ -160,7 +157,6 @@ __device__ __forceinline__ void mx_rhs(const MxArgs& a, const TIN* cu, const dou
     if (sizeof(R) == 4 && sizeof(TIN) == 4) return (R)mtf[o];
     return (R)mt[o];
   };
-  auto G = [&](int v, long long p) -> cx<R> { return ld2<R>(gin + 2 * ((long long)v * g.fs + p)); };
   cx<R> fcu[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) fcu[v] = RF(v, tx, ty);
@@ -191,16 +187,7 @@ __device__ __forceinline__ void mx_rhs(const MxArgs& a, const TIN* cu, const dou
     auto E = [&](int dy) {
       return add(sm(MTV(MT_AL, tx, ty + dy), RF(4, tx, ty + dy)), sm(MTV(MT_BE, tx, ty + dy), RF(1, tx, ty + dy)));
     };
-    auto Eg = [&](int j2, int k2) {
-      const int q2 = off2(g, ii, j2);
-      const long long p2 = off3(g, ii, j2, k2);
-      return add(sm((R)ldm(M.alpha, q2), G(4, p2)), sm((R)ldm(M.beta, q2), G(1, p2)));
-    };
-    cx<R> t;
-    if (jj == 0) t = add(neg(E(1)), Eg(2, ktarget(g, k)));
-    else if (jj == g.NJ - 1) t = b3(E(0), E(-1), (ty >= 1) ? E(-2) : Eg(jj - 2, k));
-    else t = cc(E(-1), E(1));
-    r[2] = sm(rdy, t);
+    r[2] = sm(rdy, cc(E(-1), E(1)));  // no ghost row is computed, so the difference is centred
   }
   // rhs_psi3 (:704-713)
   {
@@ -226,12 +213,7 @@ __device__ __forceinline__ void mx_rhs(const MxArgs& a, const TIN* cu, const dou
     else d = cc(G1(-1), G1(1));
     const cx<R> r1 = dsg(sm(rdx, d), sg, rs);
     auto H = [&](int dy) { return sm(MTV(MT_HT, tx, ty + dy), RF(2, tx, ty + dy)); };
-    auto Hg = [&](int j2, int k2) { return sm((R)ldm(M.asg_gtt, off2(g, ii, j2)), G(2, off3(g, ii, j2, k2))); };
-    cx<R> t;
-    if (jj == 0) t = add(neg(H(1)), Hg(2, ktarget(g, k)));
-    else if (jj == g.NJ - 1) t = b3(H(0), H(-1), (ty >= 1) ? H(-2) : Hg(jj - 2, k));
-    else t = cc(H(-1), H(1));
-    const cx<R> r2 = dsg(sm(rdy, t), sg, rs);
+    const cx<R> r2 = dsg(sm(rdy, cc(H(-1), H(1))), sg, rs);
     const cx<R> fp = CX<R>((R)Fpv.x, (R)Fpv.y), fn = CX<R>((R)Fnx.x, (R)Fnx.y);
     cx<R> z;
     if (k == 0) z = add(neg(fp), fn);
@@ -284,9 +266,13 @@ __device__ __forceinline__ int mx_item(const CUtensorMap* tinp, const CUtensorMa
   const Grid& g = a.g;
   const Metric& M = a.m;
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TI + tx;
-  const int ii0 = bx * TI, jj0 = by * TJ;
+  // every stage is followed by the ghost fill, so what that fill writes is not
+  // computed: the six theta ghost rows and the last phi plane (plane 0 is: the
+  // pole fill may read it)
+  const int nk = g.NK - 1;
+  const int ii0 = bx * TI, jj0 = 3 + by * TJ;
   const int ii = ii0 + tx, jj = jj0 + ty;
-  const bool act = (ii < g.NI) && (jj < g.NJ);
+  const bool act = (ii < g.NI) && (jj < g.NJ - 3);
   // ring slot protocol: full[s] completes when a plane's box has landed (one
   // expect_tx arrival + the bytes); empty[s] when every warp has read the plane
   // for the last time (one arrival per warp), after which thread 0 may load the
@@ -298,8 +284,8 @@ __device__ __forceinline__ int mx_item(const CUtensorMap* tinp, const CUtensorMa
     if (lane == 0) mbar_arrive(&empty[(tb + (uint32_t)t) % NST]);
   };
   const int k0 = bz * a.kchunk;
-  if (k0 >= g.NK) return 0;
-  const int k1 = min(k0 + a.kchunk, g.NK);
+  if (k0 >= nk) return 0;
+  const int k1 = min(k0 + a.kchunk, nk);
   const int nplanes = (k1 - k0) + 2;
   auto plane_of = [&](int t) -> int {
     if (t == 0) return (k0 == 0) ? g.Nz - 2 : k0 - 1;
@@ -523,7 +509,6 @@ __global__ void __launch_bounds__(TI * TJ, MGeom<TJ>::MIN_BLOCKS)
   uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(mt + (size_t)MT_COUNT * MT_N) +
                                                (sizeof(TIN) == 4 ? (size_t)MT_COUNT * MT_N * 4 : 0));
   unsigned char* stg = reinterpret_cast<unsigned char*>(bars + 8);
-  if ((int)blockIdx.z * a.kchunk >= a.g.NK) return;
   init_bars<TJ>(bars);
   (void)mx_item<KIND, MK, TIN, TJ>(&tin, &tp0, &tp1, a, blockIdx.x, blockIdx.y, blockIdx.z, ring, mt, bars, 0u, stg);
 }
@@ -683,10 +668,6 @@ bool enc(CUtensorMap* tm, const Grid& g, const void* base, int esize, bool halo,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-int mx_chunk(const Grid& g) {
-  const int nchunks = (g.NK + 31) / 32;
-  return (g.NK + nchunks - 1) / nchunks;
-}
 
 // maps and arguments of one solve's stage
 int mx_prepare(int kind, const MixedLaunch& L, const double* rsg, int* err, int kchunk, int tj, CUtensorMap* tin,
@@ -703,7 +684,6 @@ int mx_prepare(int kind, const MixedLaunch& L, const double* rsg, int* err, int 
   a->g = L.g;
   a->m = L.m;
   a->rsg = rsg;
-  a->in = first ? (const void*)L.base : (const void*)L.in_f;
   a->base = L.base;
   a->acc = L.acc;
   a->outf = L.out_f;
@@ -716,7 +696,7 @@ int mx_prepare(int kind, const MixedLaunch& L, const double* rsg, int* err, int 
 }
 
 template <int KIND, int MK, class TIN, int TJ>
-int mx_launch_one(const CUtensorMap& tin, const CUtensorMap& tp0, const CUtensorMap& tp1, const MxArgs& a,
+int mx_launch_one(const CUtensorMap& tin, const CUtensorMap& tp0, const CUtensorMap& tp1, MxArgs a,
                   cudaStream_t st) {
   constexpr size_t SMEM = MGeom<TJ>::template smem<TIN>();
   static bool attr = false;
@@ -727,7 +707,10 @@ int mx_launch_one(const CUtensorMap& tin, const CUtensorMap& tp0, const CUtensor
     attr = true;
   }
   const Grid& g = a.g;
-  dim3 grid((g.NI + TI - 1) / TI, (g.NJ + TJ - 1) / TJ, (g.NK + a.kchunk - 1) / a.kchunk);
+  const int planes = g.NK - 1;
+  dim3 grid((g.NI + TI - 1) / TI, (g.NJ - 6 + TJ - 1) / TJ, 1);
+  a.kchunk = phi_chunk(planes, (long long)grid.x * grid.y, 148 * MGeom<TJ>::MIN_BLOCKS, 32);
+  grid.z = (planes + a.kchunk - 1) / a.kchunk;
   mx_stage_kernel<KIND, MK, TIN, TJ><<<grid, dim3(TI, TJ, 1), SMEM, st>>>(tin, tp0, tp1, a);
   return 0;
 }
@@ -755,8 +738,7 @@ int mx_batch_one(const void* items, int n_solves, int n_items, int blocks, cudaS
     attr = true;
   }
   if (n_items <= 0) return 0;
-  mx_batch_kernel<KIND, MK, TIN, TJ><<<blocks, dim3(TI, TJ, 1), SMEM, st>>>(reinterpret_cast<const MxItem*>(items),
-                                                                           n_solves, n_items);
+  mx_batch_kernel<KIND, MK, TIN, TJ><<<blocks, dim3(TI, TJ, 1), SMEM, st>>>(reinterpret_cast<const MxItem*>(items), n_solves, n_items);
   return 0;
 }
 
@@ -777,7 +759,7 @@ int launch_stage_mixed(int kind, const MixedLaunch& L, const double* rsg, int* e
   if (tj != 4) tj = 8;
   CUtensorMap tin, tp0, tp1;
   MxArgs a;
-  if (mx_prepare(kind, L, rsg, err, mx_chunk(L.g), tj, &tin, &tp0, &tp1, &a)) return -1;
+  if (mx_prepare(kind, L, rsg, err, 0 /* set at the launch */, tj, &tin, &tp0, &tp1, &a)) return -1;
   if (tj == 4)
     return L.metric_kind == MK_KS ? mx_launch_mk<MK_KS, 4>(kind, tin, tp0, tp1, a, st)
                                   : mx_launch_mk<MK_SCHW, 4>(kind, tin, tp0, tp1, a, st);
@@ -790,16 +772,16 @@ size_t mixed_item_bytes() { return sizeof(MxItem); }
 int build_mixed_item(void* dst, int kind, const MixedLaunch& L, const double* rsg, int* err, int kchunk, int item0,
                      int tj) {
   {  // equal chunks of at most the requested length (as in the FP64 batch)
-    const int nch = (L.g.NK + kchunk - 1) / kchunk;
-    kchunk = (L.g.NK + nch - 1) / nch;
+    const int nch = (L.g.NK - 1 + kchunk - 1) / kchunk;
+    kchunk = (L.g.NK - 1 + nch - 1) / nch;
   }
   MxItem* B = reinterpret_cast<MxItem*>(dst);
   memset(B, 0, sizeof(MxItem));
   if (mx_prepare(kind, L, rsg, err, kchunk, tj, &B->tin, &B->tp0, &B->tp1, &B->a)) return -1;
   B->tiles_x = (L.g.NI + TI - 1) / TI;
-  B->tiles_y = (L.g.NJ + tj - 1) / tj;
+  B->tiles_y = (L.g.NJ - 6 + tj - 1) / tj;
   B->item0 = item0;
-  B->n_items = B->tiles_x * B->tiles_y * ((L.g.NK + kchunk - 1) / kchunk);
+  B->n_items = B->tiles_x * B->tiles_y * ((L.g.NK - 1 + kchunk - 1) / kchunk);
   return B->n_items;
 }
 

@@ -73,6 +73,26 @@ __device__ __forceinline__ double2 cdivm(double2 a, double b, double rb) {
 // (2e8 random operands over all exponents)
 constexpr double kThird = 1.0 / 3.0, kSixth = 1.0 / 6.0;
 
+// the stages that advance all five variables are each followed by the ghost
+// fill, which overwrites stored rows 0..2 and NJ-3..NJ-1 and phi plane Nz
+template <int KIND>
+constexpr __host__ __device__ bool filled_kind() {
+  return KIND != ST_P2_S1A && KIND != ST_P3_S2A && KIND != ST_P2_S1B && KIND != ST_P3_S2B;
+}
+// theta rows [row_first, row_end) and phi planes [0, plane_end) that a stage computes
+template <int KIND>
+constexpr __host__ __device__ int row_first() {
+  return filled_kind<KIND>() ? 3 : 0;
+}
+template <int KIND>
+__host__ __device__ __forceinline__ int row_end(const Grid& g) {
+  return filled_kind<KIND>() ? g.NJ - 3 : g.NJ;
+}
+template <int KIND>
+__host__ __device__ __forceinline__ int plane_end(const Grid& g) {
+  return filled_kind<KIND>() ? g.NK - 1 : g.NK;
+}
+
 struct TmaArgs {
   Grid g;
   Metric m;
@@ -111,12 +131,15 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
   constexpr int FIELD_D = GT::FIELD_D, STAGE_D = GT::STAGE_D, STAGE_B = GT::STAGE_B, MT_N = GT::MT_N;
   constexpr bool PSI = (KIND != ST_P2_S1B && KIND != ST_P3_S2B);
   constexpr bool PI_ = (KIND != ST_P2_S1A && KIND != ST_P3_S2A);
+  // what the ghost fill behind this stage writes is not computed: the six theta
+  // ghost rows and the last phi plane (plane 0 is: the pole fill may read it)
+  constexpr bool FILLED = filled_kind<KIND>();
   const Grid& g = a.g;
   const Metric& M = a.m;
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TI + tx;
-  const int ii0 = bx * TI, jj0 = by * TJ;
+  const int ii0 = bx * TI, jj0 = row_first<KIND>() + by * TJ;
   const int ii = ii0 + tx, jj = jj0 + ty;
-  const bool act = (ii < g.NI) && (jj < g.NJ);
+  const bool act = (ii < g.NI) && (jj < row_end<KIND>(g));
   // ring slot protocol: full[s] (bars[s]) completes when a plane's boxes have
   // landed; empty[s] when all eight warps have read the plane for the last
   // time, after which thread 0 may load the next plane into the slot, so the
@@ -124,8 +147,8 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
   uint64_t* empty = bars + NST;
   const int lane = tid & 31;
   const int k0 = bz * a.kchunk;
-  if (k0 >= g.NK) return 0;
-  const int k1 = min(k0 + a.kchunk, g.NK);
+  if (k0 >= plane_end<KIND>(g)) return 0;
+  const int k1 = min(k0 + a.kchunk, plane_end<KIND>(g));
   const int nplanes = (k1 - k0) + 2;  // previous, the chunk, next
   auto plane_of = [&](int t) -> int {
     if (t == 0) return (k0 == 0) ? g.Nz - 2 : k0 - 1;
@@ -297,7 +320,8 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
             return cadd(rmul(ldm(M.alpha, q2), ldf(a.in[4], p2)), rmul(ldm(M.beta, q2), ldf(a.in[1], p2)));
           };
           double2 t;
-          if (jj == 0) t = cadd(cneg(E(1)), Eg(2, ktarget(g, k)));
+          if (FILLED) t = ctr(E(-1), E(1));
+          else if (jj == 0) t = cadd(cneg(E(1)), Eg(2, ktarget(g, k)));
           else if (jj == g.NJ - 1) t = bwd3(E(0), E(-1), (ty >= 1) ? E(-2) : Eg(jj - 2, k));
           else t = ctr(E(-1), E(1));
           r[2] = rmul(g.rdy, t);
@@ -325,7 +349,8 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
             return rmul(ldm(M.asg_gtt, off2(g, ii, j2)), ldf(a.in[2], off3(g, ii, j2, k2)));
           };
           double2 t;
-          if (jj == 0) t = cadd(cneg(H(1)), Hg(2, ktarget(g, k)));
+          if (FILLED) t = ctr(H(-1), H(1));
+          else if (jj == 0) t = cadd(cneg(H(1)), Hg(2, ktarget(g, k)));
           else if (jj == g.NJ - 1) t = bwd3(H(0), H(-1), (ty >= 1) ? H(-2) : Hg(jj - 2, k));
           else t = ctr(H(-1), H(1));
           const double2 r2 = cdivm(rmul(g.rdy, t), sg, rs);
@@ -454,7 +479,6 @@ __global__ void __launch_bounds__(TI * TJ, Geom<TJ>::MIN_BLOCKS)
   double* ring = reinterpret_cast<double*>(align128(smem_raw));
   double* mt = ring + (size_t)NST * Geom<TJ>::STAGE_D;
   uint64_t* bars = reinterpret_cast<uint64_t*>(mt + (size_t)MT_COUNT * Geom<TJ>::MT_N);
-  if ((int)blockIdx.z * a.kchunk >= a.g.NK) return;
   init_ring_barriers<TJ>(bars);
   (void)stage_item<KIND, MK, TJ>(&tm4, &tm1, &tp0, &tp1, a, blockIdx.x, blockIdx.y, blockIdx.z, ring, mt, bars, 0u);
 }
@@ -535,17 +559,13 @@ bool encode(CUtensorMap* tm, const Grid& g, const double2* base, int nvars, bool
   return r == CUDA_SUCCESS;
 }
 
-int tma_chunk(const Grid& g) {
-  const int nchunks = (g.NK + 31) / 32;
-  return (g.NK + nchunks - 1) / nchunks;
-}
 
 struct Maps {
   CUtensorMap tm4, tm1, tp0, tp1;
 };
 
 template <int KIND, int MK, int TJ>
-int launch_one(const Maps& m, const TmaArgs& a, cudaStream_t st) {
+int launch_one(const Maps& m, TmaArgs a, cudaStream_t st) {
   constexpr size_t SMEM = Geom<TJ>::SMEM_BYTES;
   static bool attr_set = false;
   if (!attr_set) {
@@ -556,7 +576,10 @@ int launch_one(const Maps& m, const TmaArgs& a, cudaStream_t st) {
   }
   const Grid& g = a.g;
   dim3 block(TI, TJ, 1);
-  dim3 grid((g.NI + TI - 1) / TI, (g.NJ + TJ - 1) / TJ, (g.NK + a.kchunk - 1) / a.kchunk);
+  const int planes = plane_end<KIND>(g), rows = row_end<KIND>(g) - row_first<KIND>();
+  dim3 grid((g.NI + TI - 1) / TI, (rows + TJ - 1) / TJ, 1);
+  a.kchunk = phi_chunk(planes, (long long)grid.x * grid.y, 148 * Geom<TJ>::MIN_BLOCKS, 32);
+  grid.z = (planes + a.kchunk - 1) / a.kchunk;
   tma_stage_kernel<KIND, MK, TJ><<<grid, block, SMEM, st>>>(m.tm4, m.tm1, m.tp0, m.tp1, a);
   return 0;
 }
@@ -584,9 +607,10 @@ int build_batch_item(void* dst, int kind, const StageLaunch& L, const double* rs
   // the requested chunk length is an upper bound: the solve's planes are split
   // into equal chunks, so no chunk is a short remainder that pays a whole
   // pipeline prologue for a few planes
+  const int planes = L.g.NK - 1, rows = L.g.NJ - 6;  // the batched kinds are all followed by the ghost fill
   {
-    const int nch = (L.g.NK + kchunk - 1) / kchunk;
-    kchunk = (L.g.NK + nch - 1) / nch;
+    const int nch = (planes + kchunk - 1) / kchunk;
+    kchunk = (planes + nch - 1) / nch;
   }
   BatchItem* B = reinterpret_cast<BatchItem*>(dst);
   memset(B, 0, sizeof(BatchItem));
@@ -627,8 +651,8 @@ int build_batch_item(void* dst, int kind, const StageLaunch& L, const double* rs
   a.npf = npf;
   a.base_in = base_in;
   B->tiles_x = (L.g.NI + TI - 1) / TI;
-  B->tiles_y = (L.g.NJ + tj - 1) / tj;
-  const int chunks = (L.g.NK + kchunk - 1) / kchunk;
+  B->tiles_y = (rows + tj - 1) / tj;
+  const int chunks = (planes + kchunk - 1) / kchunk;
   B->item0 = item0;
   B->n_items = B->tiles_x * B->tiles_y * chunks;
   return B->n_items;
@@ -646,8 +670,7 @@ int batch_one(const void* items, int n_solves, int n_items, int blocks, cudaStre
     attr_set = true;
   }
   if (n_items <= 0) return 0;
-  tma_batch_kernel<KIND, MK, TJ><<<blocks, dim3(TI, TJ, 1), SMEM, st>>>(reinterpret_cast<const BatchItem*>(items),
-                                                                       n_solves, n_items);
+  tma_batch_kernel<KIND, MK, TJ><<<blocks, dim3(TI, TJ, 1), SMEM, st>>>(reinterpret_cast<const BatchItem*>(items), n_solves, n_items);
   return 0;
 }
 template <int KIND>
@@ -666,9 +689,6 @@ int batch_kind(const void* items, int n_solves, int n_items, int blocks, int mk,
 int launch_batch_tma(int kind, int mk, const void* d_items, int n_solves, int n_items, int blocks, int tj,
                      cudaStream_t st) {
   switch (kind) {
-    case ST_P2_S1A: return batch_kind<ST_P2_S1A>(d_items, n_solves, n_items, blocks, mk, tj, st);
-    case ST_P2_S1B: return batch_kind<ST_P2_S1B>(d_items, n_solves, n_items, blocks, mk, tj, st);
-    case ST_P2_S2: return batch_kind<ST_P2_S2>(d_items, n_solves, n_items, blocks, mk, tj, st);
     case ST_RK4_1: return batch_kind<ST_RK4_1>(d_items, n_solves, n_items, blocks, mk, tj, st);
     case ST_RK4_2: return batch_kind<ST_RK4_2>(d_items, n_solves, n_items, blocks, mk, tj, st);
     case ST_RK4_3: return batch_kind<ST_RK4_3>(d_items, n_solves, n_items, blocks, mk, tj, st);
@@ -737,7 +757,7 @@ int launch_stage_tma(int kind, const StageLaunch& L, const double* rsg, int* err
   a.out4 = L.out4;
   a.acc = L.acc;
   a.skip_last_i = L.skip_last_i;
-  a.kchunk = tma_chunk(L.g);
+  a.kchunk = 0;  // set at the launch, from the tiles of the grid
   a.err = err;
   a.npf = npf;
   a.base_in = base_in && (kind == ST_P2_S1A || kind == ST_RK3_1 || kind == ST_RK4_1);
