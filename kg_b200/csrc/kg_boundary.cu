@@ -7,13 +7,9 @@
 // and boundary_yR (theta ghost rows copied from the interior rows at phi + pi,
 // no sign change), boundary_zL and boundary_zR (duplicated phi planes).
 //
-// The stepper path runs this as two launches:
-//   ghost_xy: every x-face point of the interior theta rows and every point of
-//             the six theta ghost rows.  A theta ghost row takes the post-x
-//             value of its source, which is computed on the fly from the
-//             pre-boundary state, so no point read is written by the launch.
-//   ghost_z:  the two duplicated phi planes, from planes Nz-1 and 1 after
-//             ghost_xy (the reference's zL/zR run after the theta fill).
+// The stepper path runs this as one launch over independent rows along r; each
+// takes the value the whole sequence leaves there, computed from the
+// pre-boundary state (see ghost_unit).
 // `face` launches run one reference routine at a time (parity hook).
 #include "kg_device.cuh"
 #include "kg_internal.h"
@@ -34,130 +30,149 @@ __device__ __forceinline__ int ghost_src_row(const Grid& g, int jj) {
   return (jj <= 2) ? (5 - jj) : (2 * g.NJ - 7 - jj);
 }
 
-__global__ void ghost_xy_kernel(Grid g, double2* u, const double2* up, int inflow, long long n_rows,
-                                long long n_faces) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = n_rows + n_faces;
-  if (t >= total) return;
-  if (t < n_rows) {
-    // ghost-row points: t = ii + NI*(r + 6*k), r in 0..5
-    const int ii = (int)(t % g.NI);
-    const long long rk = t / g.NI;
-    const int r = (int)(rk % 6);
-    const int k = (int)(rk / 6);
-    const int jj = (r < 3) ? r : (g.NJ - 6 + r);
-    const int js = ghost_src_row(g, jj);
-    const int kt = ktarget(g, k);
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      const double2* uv = u + v * g.fs;
-      const double2* upv = up + v * g.fs;
-      u[v * g.fs + off3(g, ii, jj, k)] = xval(g, uv, upv, inflow, ii, js, kt);
-    }
-  } else {
-    // x-face points of interior rows: f = jr + (NJ-6)*(side + 2*k)
-    const long long f = t - n_rows;
-    const int nin = g.NJ - 6;
-    const int jj = 3 + (int)(f % nin);
-    const long long sk = f / nin;
-    const int side = (int)(sk % 2);
-    const int k = (int)(sk / 2);
-    const int ii = side ? g.NI - 1 : 0;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      const double2* uv = u + v * g.fs;
-      const double2* upv = up + v * g.fs;
-      u[v * g.fs + off3(g, ii, jj, k)] = xval(g, uv, upv, inflow, ii, jj, k);
-    }
+// ---- the whole fill in one launch --------------------------------------------
+// Units, each done by one thread block with its threads along r:
+//   A  ghost row r of plane k, 1 <= k < Nz: the source row (js, k + pi) after the
+//      x fill (6 (Nz - 1) rows);
+//   C  row jj of plane 0 (from plane Nz - 1) and of plane Nz (from plane 1), ghost
+//      rows through their source row (2 NJ rows);
+//   B  the two x-face points of the interior rows of planes 1..Nz-1.
+// No point that a unit reads is written by another one, with one exception: the
+// partner of plane kp = Nz - 1 - Nz/2 is plane 0, so the ghost rows of kp take
+// rows 3..5 and NJ-6..NJ-4 of plane 0 as the stage left them, and C overwrites
+// those rows.  The C unit of such a row therefore writes kp's ghost rows first
+// and the row itself behind a block barrier (A leaves plane kp out).
+// What bounds it: on small grids the launch and the latency of one load-store
+// chain per thread, so one launch replaces the former two (ghost rows and faces,
+// then the phi planes); on large ones memory, 2 x 80 B per point of the ghost rows.
+// Measured, event-timed (a launch pair before, one after): 64 x 17 x 33 13.0 ->
+// 8.8 us, 256 x 33 x 65 18.8 -> 12.3 us, 1024 x 65 x 129 43 -> 33 us, 2048 x 129 x
+// 257 124 -> 105 us.
+template <class T>
+__device__ __forceinline__ T xval_t(const Grid& g, const T* u, const double2* up, int inflow, int ii, int jj, int k);
+template <>
+__device__ __forceinline__ double2 xval_t<double2>(const Grid& g, const double2* u, const double2* up, int inflow,
+                                                   int ii, int jj, int k) {
+  return xval(g, u, up, inflow, ii, jj, k);
+}
+// FP32 stage states: the excision extrapolation is formed in FP64, the inflow
+// hold reads u^n (FP64)
+template <>
+__device__ __forceinline__ float2 xval_t<float2>(const Grid& g, const float2* u, const double2* up, int inflow, int ii,
+                                                 int jj, int k) {
+  if (ii == 0) {
+    const float2 a = u[off3(g, 1, jj, k)], b = u[off3(g, 2, jj, k)], c = u[off3(g, 3, jj, k)];
+    const double rx = (3.0 * (double)a.x - 3.0 * (double)b.x) + (double)c.x;
+    const double ry = (3.0 * (double)a.y - 3.0 * (double)b.y) + (double)c.y;
+    return make_float2((float)rx, (float)ry);
   }
+  if (ii == g.NI - 1) {
+    if (inflow) {
+      const double2 v = up[off3(g, ii, jj, k)];
+      return make_float2((float)v.x, (float)v.y);
+    }
+    return u[off3(g, ii - 1, jj, k)];
+  }
+  return u[off3(g, ii, jj, k)];
 }
 
-__global__ void ghost_z_kernel(Grid g, double2* u) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long n = (long long)g.NI * g.NJ;
-  if (t >= 2 * n) return;
-  const int side = (int)(t / n);
-  const long long q = t % n;
-  const int ii = (int)(q % g.NI), jj = (int)(q / g.NI);
-  const int kd = side ? g.Nz : 0;
-  const int ks = side ? 1 : g.Nz - 1;
+// row (jd, kd) <- row (js, ks) after the x fill, all five variables
+template <class T>
+__device__ __forceinline__ void ghost_row(const Grid& g, T* u, const double2* up, int inflow, int jd, int kd, int js,
+                                          int ks) {
+  const long long d = off3(g, 0, jd, kd), s = off3(g, 0, js, ks);
+  for (int ii = threadIdx.x; ii < g.NI; ii += blockDim.x) {
+    T v[5];
+    if (ii == 0 || ii == g.NI - 1) {
 #pragma unroll
-  for (int v = 0; v < 5; ++v) u[v * g.fs + off3(g, ii, jj, kd)] = u[v * g.fs + off3(g, ii, jj, ks)];
-}
-
-void launch_ghost_fill(const Grid& g, double2* u, const double2* up, int inflow, cudaStream_t st) {
-  const long long n_rows = 6LL * g.NK * g.NI;
-  const long long n_faces = 2LL * (g.NJ - 6) * g.NK;
-  const long long total = n_rows + n_faces;
-  ghost_xy_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(g, u, up, inflow, n_rows, n_faces);
-  const long long nz = 2LL * g.NI * g.NJ;
-  ghost_z_kernel<<<(unsigned)((nz + 255) / 256), 256, 0, st>>>(g, u);
-}
-
-// ---- many solves at once (batched engine) -----------------------------------
-__global__ void ghost_xy_batch_kernel(const GhostDesc* __restrict__ d) {
-  const GhostDesc& D = d[blockIdx.y];
-  const Grid& g = D.g;
-  const long long n_rows = 6LL * g.NK * g.NI;
-  const long long n_faces = 2LL * (g.NJ - 6) * g.NK;
-  const long long total = n_rows + n_faces;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    int ii, jj, k, si, sj, sk;
-    if (t < n_rows) {
-      ii = (int)(t % g.NI);
-      const long long rk = t / g.NI;
-      const int r = (int)(rk % 6);
-      k = (int)(rk / 6);
-      jj = (r < 3) ? r : (g.NJ - 6 + r);
-      si = ii;
-      sj = ghost_src_row(g, jj);
-      sk = ktarget(g, k);
+      for (int w = 0; w < 5; ++w) v[w] = xval_t<T>(g, u + w * g.fs, up + w * g.fs, inflow, ii, js, ks);
     } else {
-      const long long f = t - n_rows;
-      const int nin = g.NJ - 6;
-      jj = 3 + (int)(f % nin);
-      const long long s2 = f / nin;
-      const int side = (int)(s2 % 2);
-      k = (int)(s2 / 2);
-      ii = side ? g.NI - 1 : 0;
-      si = ii;
-      sj = jj;
-      sk = k;
+#pragma unroll
+      for (int w = 0; w < 5; ++w) v[w] = u[w * g.fs + s + ii];
     }
 #pragma unroll
-    for (int v = 0; v < 5; ++v)
-      D.u[v * g.fs + off3(g, ii, jj, k)] = xval(g, D.u + v * g.fs, D.up + v * g.fs, D.inflow, si, sj, sk);
+    for (int w = 0; w < 5; ++w) u[w * g.fs + d + ii] = v[w];
   }
 }
 
-__global__ void ghost_z_batch_kernel(const GhostDesc* __restrict__ d) {
-  const GhostDesc& D = d[blockIdx.y];
-  const Grid& g = D.g;
-  const long long n = (long long)g.NI * g.NJ;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < 2 * n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int side = (int)(t / n);
-    const long long q = t % n;
-    const int ii = (int)(q % g.NI), jj = (int)(q / g.NI);
-    const int kd = side ? g.Nz : 0;
-    const int ks = side ? 1 : g.Nz - 1;
+__host__ __device__ __forceinline__ int ghost_units(const Grid& g, int threads) {
+  const int faces = 2 * (g.NJ - 6) * (g.Nz - 1);
+  return 2 * g.NJ + 6 * (g.Nz - 1) + (faces + threads - 1) / threads;
+}
+
+template <class T>
+__device__ __forceinline__ void ghost_unit(const Grid& g, T* u, const double2* up, int inflow, int unit) {
+  const int nC = 2 * g.NJ, nA = 6 * (g.Nz - 1);
+  if (unit < nC) {  // row jj of plane 0 or Nz
+    const int jj = unit % g.NJ;
+    const bool last = unit >= g.NJ;
+    const int ks = last ? 1 : g.Nz - 1;
+    const bool ghost = jj < 3 || jj >= g.NJ - 3;
+    if (!last && !ghost) {
+      const int kp = g.Nzm1 - g.dis;
+      const bool north = jj <= 5, south = jj >= g.NJ - 6;
+      if (north) ghost_row(g, u, up, inflow, 5 - jj, kp, jj, 0);
+      if (south) ghost_row(g, u, up, inflow, 2 * g.NJ - 7 - jj, kp, jj, 0);
+      if (north || south) __syncthreads();
+    }
+    ghost_row(g, u, up, inflow, jj, last ? g.Nz : 0, ghost ? ghost_src_row(g, jj) : jj, ghost ? ktarget(g, ks) : ks);
+  } else if (unit < nC + nA) {  // ghost row of an inner plane
+    const int q = unit - nC;
+    const int r = q % 6, k = 1 + q / 6;
+    const int kt = ktarget(g, k);
+    if (kt == 0) return;  // with plane 0's own rows
+    const int jj = (r < 3) ? r : (g.NJ - 6 + r);
+    ghost_row(g, u, up, inflow, jj, k, ghost_src_row(g, jj), kt);
+  } else {  // x-face points
+    const int f = (unit - nC - nA) * blockDim.x + threadIdx.x;
+    const int nin = g.NJ - 6;
+    if (f >= 2 * nin * (g.Nz - 1)) return;
+    const int jj = 3 + f % nin, sk = f / nin;
+    const int k = 1 + (sk >> 1), ii = (sk & 1) ? g.NI - 1 : 0;
 #pragma unroll
-    for (int v = 0; v < 5; ++v) D.u[v * g.fs + off3(g, ii, jj, kd)] = D.u[v * g.fs + off3(g, ii, jj, ks)];
+    for (int w = 0; w < 5; ++w)
+      u[w * g.fs + off3(g, ii, jj, k)] = xval_t<T>(g, u + w * g.fs, up + w * g.fs, inflow, ii, jj, k);
   }
 }
 
-void launch_ghost_fill_batch(const GhostDesc* d_desc, int n, long long max_rows, long long max_faces,
-                             long long max_zplanes, cudaStream_t st) {
+// threads of a block: a row of a small grid in one pass, 256 for longer rows
+static int ghost_threads(int ni) { return ni >= 256 ? 256 : (ni + 31) / 32 * 32; }
+
+template <class T>
+__global__ void ghost_kernel(Grid g, T* u, const double2* up, int inflow, int unit0) {
+  ghost_unit(g, u, up, inflow, unit0 + blockIdx.x);
+}
+
+void launch_ghost_fill(const Grid& g, double2* u, const double2* up, int inflow, cudaStream_t st, bool faces_apart) {
+  const int nt = ghost_threads(g.NI), n = ghost_units(g, nt), rows = 2 * g.NJ + 6 * (g.Nz - 1);
+  if (!faces_apart) {
+    ghost_kernel<double2><<<n, nt, 0, st>>>(g, u, up, inflow, 0);
+    return;
+  }
+  ghost_kernel<double2><<<rows, nt, 0, st>>>(g, u, up, inflow, 0);
+  ghost_kernel<double2><<<n - rows, nt, 0, st>>>(g, u, up, inflow, rows);
+}
+
+void launch_ghost_fill_f32(const Grid& g, float2* u, const double2* up, int inflow, cudaStream_t st) {
+  const int nt = ghost_threads(g.NI);
+  ghost_kernel<float2><<<ghost_units(g, nt), nt, 0, st>>>(g, u, up, inflow, 0);
+}
+
+// ---- many solves at once (batched engine): one block row per solve -----------
+constexpr int GB_THREADS = 128;
+template <class T>
+__global__ void ghost_batch_kernel(const GhostDesc* __restrict__ d) {
+  const GhostDesc& D = d[blockIdx.y];
+  if ((int)blockIdx.x < ghost_units(D.g, GB_THREADS))
+    ghost_unit(D.g, static_cast<T*>(D.u), D.up, D.inflow, blockIdx.x);
+}
+
+int ghost_batch_units(const Grid& g) { return ghost_units(g, GB_THREADS); }
+
+void launch_ghost_fill_batch(const GhostDesc* d_desc, int n, int max_units, int f32, cudaStream_t st) {
   if (n <= 0) return;
-  long long bx = (max_rows + max_faces + 255) / 256;
-  if (bx > 1024) bx = 1024;
-  if (bx < 1) bx = 1;
-  ghost_xy_batch_kernel<<<dim3((unsigned)bx, n), 256, 0, st>>>(d_desc);
-  long long bz = (max_zplanes + 255) / 256;
-  if (bz > 1024) bz = 1024;
-  if (bz < 1) bz = 1;
-  ghost_z_batch_kernel<<<dim3((unsigned)bz, n), 256, 0, st>>>(d_desc);
+  if (f32) ghost_batch_kernel<float2><<<dim3(max_units, n), GB_THREADS, 0, st>>>(d_desc);
+  else ghost_batch_kernel<double2><<<dim3(max_units, n), GB_THREADS, 0, st>>>(d_desc);
 }
 
 // ---- one reference routine at a time ---------------------------------------

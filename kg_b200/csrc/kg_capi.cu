@@ -78,7 +78,6 @@ struct kg_solver {
   // mixed precision (RK4): FP32 stage states R1, R2 and increment sum, 5 slots each
   int precision = 0;                     // 0: FP64, 1: FP32 RHS with FP64 state update
   float2* MX = nullptr;
-  unsigned char* mx_gdesc = nullptr;     // FP32 ghost-fill descriptors of R1, R2 (device)
   int graph_gen = 0;
   // detectors and projection
   int n_det = 5;
@@ -733,9 +732,11 @@ int check_device_flag(kg_solver* h) {
   }
   return KG_OK;
 }
-void run_ghost(kg_solver* h, double2* u, const double2* up, int inflow) {
-  Prof pf(h, PK_GHOST, 2);
-  kg::launch_ghost_fill(h->g, u, up, inflow, h->stream);
+// faces_apart: two launches instead of one; a PIRK2 step is four launches, a
+// count that kg_launch_count reports and its callers rely on
+void run_ghost(kg_solver* h, double2* u, const double2* up, int inflow, bool faces_apart = false) {
+  Prof pf(h, PK_GHOST, faces_apart ? 2 : 1);
+  kg::launch_ghost_fill(h->g, u, up, inflow, h->stream, faces_apart);
 }
 
 kg::StageLaunch base_launch(kg_solver* h) {
@@ -843,7 +844,7 @@ int kg_destroy(kg_solver* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   void* bufs[] = {h->dmet, h->U, h->S, h->T, h->RK, h->UP, h->HV, h->stage_buf, h->rho, h->partials,
                   h->d_int, h->d_dbl, h->shells, h->alm, h->flux, h->derr, h->ylm_tab, h->ylm_buf,
-                  h->rad_jr, h->rad_ft, h->MX, h->mx_gdesc};
+                  h->rad_jr, h->rad_ft, h->MX};
   for (void* b : bufs) dfree(h, b);
   for (auto& row : h->graphs)
     for (auto& e : row)
@@ -942,7 +943,7 @@ int step_pirk2(kg_solver* h, int nsteps) {
     L.out = h->U;
     L.skip_last_i = inflow;
     run_stage(h, kg::ST_P2_S2, L);
-    run_ghost(h, h->U, h->U, inflow);
+    run_ghost(h, h->U, h->U, inflow, true);
     h->s_cur = 9 - h->s_cur;
     h->t = h->t + h->dt;
   }
@@ -1047,20 +1048,10 @@ int step_rk4(kg_solver* h, int nsteps) {
   return KG_OK;
 }
 
-// FP32 stage buffers and their ghost-fill descriptors
+// FP32 stage buffers
 int ensure_mixed(kg_solver* h) {
   if (h->MX) return KG_OK;
-  int rc;
-  if ((rc = dalloc(h, (void**)&h->MX, (size_t)15 * h->g.fs * sizeof(float2)))) return rc;
-  const size_t dsz = kg::ghost_f32_desc_bytes();
-  if ((rc = dalloc(h, (void**)&h->mx_gdesc, 2 * dsz))) return rc;
-  std::vector<unsigned char> d(2 * dsz);
-  const int inflow = h->p.bc_rmax == KG_INFLOW;
-  kg::fill_ghost_f32_desc(d.data(), h->g, h->MX, h->U, inflow);
-  kg::fill_ghost_f32_desc(d.data() + dsz, h->g, h->MX + 5 * h->g.fs, h->U, inflow);
-  KG_CK(cudaMemcpyAsync(h->mx_gdesc, d.data(), d.size(), cudaMemcpyHostToDevice, h->stream));
-  KG_CK(cudaStreamSynchronize(h->stream));
-  return KG_OK;
+  return dalloc(h, (void**)&h->MX, (size_t)15 * h->g.fs * sizeof(float2));
 }
 
 kg::MixedLaunch mixed_launch(kg_solver* h) {
@@ -1083,11 +1074,9 @@ int run_mixed_stage(kg_solver* h, int st, const kg::MixedLaunch& L) {
   return KG_OK;
 }
 
-void run_ghost_f32(kg_solver* h, int which) {
-  Prof pf(h, PK_GHOST_F32, 2);
-  const Grid& g = h->g;
-  kg::launch_ghost_fill_f32(h->mx_gdesc + which * kg::ghost_f32_desc_bytes(), 1, 6LL * g.NK * g.NI,
-                            2LL * (g.NJ - 6) * g.NK, 2LL * g.NI * g.NJ, h->stream);
+void run_ghost_f32(kg_solver* h, float2* u) {
+  Prof pf(h, PK_GHOST_F32, 1);
+  kg::launch_ghost_fill_f32(h->g, u, h->U, h->p.bc_rmax == KG_INFLOW, h->stream);
 }
 
 // RK4 with the stencil RHS in FP32 and the state update in FP64 (kg_mixed.cu)
@@ -1101,15 +1090,15 @@ int step_rk4_mixed(kg_solver* h, int nsteps) {
     kg::MixedLaunch L = mixed_launch(h);
     L.out_f = R1;
     if ((rc = run_mixed_stage(h, 0, L))) return rc;
-    run_ghost_f32(h, 0);
+    run_ghost_f32(h, R1);
     L.in_f = R1;
     L.out_f = R2;
     if ((rc = run_mixed_stage(h, 1, L))) return rc;
-    run_ghost_f32(h, 1);
+    run_ghost_f32(h, R2);
     L.in_f = R2;
     L.out_f = R1;
     if ((rc = run_mixed_stage(h, 2, L))) return rc;
-    run_ghost_f32(h, 0);
+    run_ghost_f32(h, R1);
     L.in_f = R1;
     L.out_f = nullptr;
     L.out_d = h->U;
@@ -2013,11 +2002,10 @@ struct kg_batch {
   // per RK4 stage: item records and ghost descriptors (device)
   unsigned char* ditems[4] = {nullptr, nullptr, nullptr, nullptr};
   kg::GhostDesc* dghost[4] = {nullptr, nullptr, nullptr, nullptr};
-  unsigned char* dghost_f[3] = {nullptr, nullptr, nullptr};  // FP32 stage fills (mixed precision)
   int precision = 0;                                         // 0: FP64 RK4, 1: mixed (kg_mixed.cu)
   size_t items_cap = 0, ghost_cap = 0;
   int n_items[4] = {0, 0, 0, 0};
-  long long max_rows = 0, max_faces = 0, max_z = 0;
+  int ghost_units = 0;                                       // the largest member's
   int* derr = nullptr;
   cudaGraphExec_t graph = nullptr;
   long long graph_launches = 0;
@@ -2052,7 +2040,6 @@ int batch_rebuild(kg_batch* b) {
   const bool mixed = b->precision == 1;
   const size_t isz = mixed ? kg::mixed_item_bytes() : kg::batch_item_bytes();
   const size_t isz_max = std::max(kg::mixed_item_bytes(), kg::batch_item_bytes());
-  const size_t gfsz = kg::ghost_f32_desc_bytes();
   if (b->graph) {
     cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
@@ -2064,23 +2051,17 @@ int batch_rebuild(kg_batch* b) {
       b->ditems[st] = nullptr;
       b->dghost[st] = nullptr;
     }
-    for (int st = 0; st < 3; ++st) {
-      if (b->dghost_f[st]) cudaFree(b->dghost_f[st]);
-      b->dghost_f[st] = nullptr;
-    }
     size_t cap = n < 16 ? 16 : (size_t)n * 2;
     for (int st = 0; st < 4; ++st) {
       KG_BCK(cudaMalloc((void**)&b->ditems[st], cap * isz_max));
       KG_BCK(cudaMalloc((void**)&b->dghost[st], cap * sizeof(kg::GhostDesc)));
     }
-    for (int st = 0; st < 3; ++st) KG_BCK(cudaMalloc((void**)&b->dghost_f[st], cap * gfsz));
     b->items_cap = cap;
   }
   std::vector<unsigned char> hitems((size_t)n * isz);
   std::vector<kg::GhostDesc> hg(n);
-  std::vector<unsigned char> hgf((size_t)n * gfsz);
   const int kinds[4] = {kg::ST_RK4_1, kg::ST_RK4_2, kg::ST_RK4_3, kg::ST_RK4_4};
-  b->max_rows = b->max_faces = b->max_z = 0;
+  b->ghost_units = 0;
   for (int st = 0; st < 4; ++st) {
     int item0 = 0;
     for (int i = 0; i < n; ++i) {
@@ -2103,16 +2084,8 @@ int batch_rebuild(kg_batch* b) {
           return KG_ECUDA;
         }
         item0 += ni;
-        if (st < 3) kg::fill_ghost_f32_desc(hgf.data() + (size_t)i * gfsz, g, M.out_f, h->U, inflow);
-        hg[i].g = g;
-        hg[i].u = h->U;
-        hg[i].up = h->U;
-        hg[i].inflow = inflow;
-        if (st == 0) {
-          b->max_rows = std::max(b->max_rows, 6LL * g.NK * g.NI);
-          b->max_faces = std::max(b->max_faces, 2LL * (g.NJ - 6) * g.NK);
-          b->max_z = std::max(b->max_z, 2LL * g.NI * g.NJ);
-        }
+        hg[i] = {g, st < 3 ? (void*)M.out_f : (void*)h->U, h->U, inflow};
+        b->ghost_units = std::max(b->ghost_units, kg::ghost_batch_units(g));
         continue;
       }
       double2* R1 = h->RK;
@@ -2134,22 +2107,13 @@ int batch_rebuild(kg_batch* b) {
         return KG_ECUDA;
       }
       item0 += ni;
-      hg[i].g = g;
-      hg[i].u = out;
-      hg[i].up = h->U;
-      hg[i].inflow = h->p.bc_rmax == KG_INFLOW;
-      if (st == 0) {
-        b->max_rows = std::max(b->max_rows, 6LL * g.NK * g.NI);
-        b->max_faces = std::max(b->max_faces, 2LL * (g.NJ - 6) * g.NK);
-        b->max_z = std::max(b->max_z, 2LL * g.NI * g.NJ);
-      }
+      hg[i] = {g, out, h->U, h->p.bc_rmax == KG_INFLOW};
+      b->ghost_units = std::max(b->ghost_units, kg::ghost_batch_units(g));
     }
     b->n_items[st] = item0;
     KG_BCK(cudaMemcpyAsync(b->ditems[st], hitems.data(), (size_t)n * isz, cudaMemcpyHostToDevice, b->stream));
     KG_BCK(cudaMemcpyAsync(b->dghost[st], hg.data(), (size_t)n * sizeof(kg::GhostDesc), cudaMemcpyHostToDevice,
                            b->stream));
-    if (mixed && st < 3)
-      KG_BCK(cudaMemcpyAsync(b->dghost_f[st], hgf.data(), (size_t)n * gfsz, cudaMemcpyHostToDevice, b->stream));
   }
   KG_BCK(cudaStreamSynchronize(b->stream));
   b->dirty = false;
@@ -2169,11 +2133,8 @@ int batch_enqueue_step(kg_batch* b) {
       b->err = "batched stage launch could not be configured";
       return KG_ECUDA;
     }
-    if (b->precision == 1 && st < 3)
-      kg::launch_ghost_fill_f32(b->dghost_f[st], n, b->max_rows, b->max_faces, b->max_z, b->stream);
-    else
-      kg::launch_ghost_fill_batch(b->dghost[st], n, b->max_rows, b->max_faces, b->max_z, b->stream);
-    b->launches += 3;
+    kg::launch_ghost_fill_batch(b->dghost[st], n, b->ghost_units, b->precision == 1 && st < 3, b->stream);
+    b->launches += 2;
   }
   KG_BCK(cudaGetLastError());
   return KG_OK;
@@ -2216,8 +2177,6 @@ int kg_batch_destroy(kg_batch* b) {
     if (b->ditems[st]) cudaFree(b->ditems[st]);
     if (b->dghost[st]) cudaFree(b->dghost[st]);
   }
-  for (int st = 0; st < 3; ++st)
-    if (b->dghost_f[st]) cudaFree(b->dghost_f[st]);
   if (b->pin) cudaFreeHost(b->pin);
   if (b->derr) cudaFree(b->derr);
   if (b->ev) cudaEventDestroy(b->ev);

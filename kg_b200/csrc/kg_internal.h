@@ -91,15 +91,16 @@ int ylm_gemm_pad_m(int rows);
 int ylm_gemm_pad_n(int cols);
 int ylm_gemm_pad_k(int k);
 int ylm_gemm_splits(int Kp);  // K ranges of the split-K GEMM (FP32 partial tiles added in FP64)
-// batched ghost fill: one launch pair for many solves
+// batched ghost fill: one launch for many solves; u points to FP64 or (f32)
+// FP32 complex values; max_units: the largest ghost_batch_units of the solves
 struct GhostDesc {
   Grid g;
-  double2* u;
+  void* u;
   const double2* up;
   int inflow;
 };
-void launch_ghost_fill_batch(const GhostDesc* d_desc, int n, long long max_rows, long long max_faces,
-                             long long max_zplanes, cudaStream_t st);
+int ghost_batch_units(const Grid& g);
+void launch_ghost_fill_batch(const GhostDesc* d_desc, int n, int max_units, int f32, cudaStream_t st);
 // mixed-precision RK4 (kg_mixed.cu): FP32 stage states and increment sum, FP64 u
 struct MixedLaunch {
   Grid g;
@@ -119,10 +120,6 @@ int build_mixed_item(void* dst, int kind, const MixedLaunch& L, const double* rs
                      int tj);
 int launch_batch_mixed(int kind, int mk, const void* d_items, int n_solves, int n_items, int blocks, int tj,
                        cudaStream_t st);
-size_t ghost_f32_desc_bytes();
-void fill_ghost_f32_desc(void* dst, const Grid& g, float2* u, const double2* up, int inflow);
-void launch_ghost_fill_f32(const void* d_desc, int n, long long max_rows, long long max_faces, long long max_z,
-                           cudaStream_t st);
 // configured method (kg_config.cu): RK4 stage with fourth-order differences,
 // Kreiss-Oliger dissipation and a Sommerfeld outer plane; coef = 1/(12 h) for
 // r, theta, phi then eps/(64 h) for r, theta, phi; rN = outermost r; rsg = the
@@ -140,7 +137,11 @@ void launch_rhs(const Grid& g, const Metric& m, int metric_kind, const double2* 
                 unsigned mask, cudaStream_t st);
 
 // boundary fills on a 5-variable state u; up = u_p (inflow source)
-void launch_ghost_fill(const Grid& g, double2* u, const double2* up, int inflow, cudaStream_t st);
+// faces_apart: the x faces in a second launch of their own
+void launch_ghost_fill(const Grid& g, double2* u, const double2* up, int inflow, cudaStream_t st,
+                       bool faces_apart = false);
+// the same on the FP32 stage states of the mixed form; up = u^n (FP64)
+void launch_ghost_fill_f32(const Grid& g, float2* u, const double2* up, int inflow, cudaStream_t st);
 void launch_face(const Grid& g, double2* u, const double2* up, int inflow, int face, cudaStream_t st);
 
 // layout conversion between the Fortran AoS layout and the device planes,

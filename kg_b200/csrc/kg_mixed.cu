@@ -553,88 +553,6 @@ __global__ void __launch_bounds__(TI * TJ, MGeom<TJ>::MIN_BLOCKS)
   }
 }
 
-// ---- FP32 stage states: ghost-zone, pole and outer-boundary fills ----------
-// Same points and order as the FP64 fill (boundary_xL .. boundary_zR,
-// MoL/lines_method_lib.f90:507-597); the excision extrapolation
-// 3 u1 - 3 u2 + u3 is formed in FP64, the inflow hold reads u^n (FP64).
-__device__ __forceinline__ float2 xval_f(const Grid& g, const float2* u, const double2* up, int inflow, int ii,
-                                         int jj, int k) {
-  if (ii == 0) {
-    const float2 a = u[off3(g, 1, jj, k)], b = u[off3(g, 2, jj, k)], c = u[off3(g, 3, jj, k)];
-    const double rx = (3.0 * (double)a.x - 3.0 * (double)b.x) + (double)c.x;
-    const double ry = (3.0 * (double)a.y - 3.0 * (double)b.y) + (double)c.y;
-    return make_float2((float)rx, (float)ry);
-  }
-  if (ii == g.NI - 1) {
-    if (inflow) {
-      const double2 v = up[off3(g, ii, jj, k)];
-      return make_float2((float)v.x, (float)v.y);
-    }
-    return u[off3(g, ii - 1, jj, k)];
-  }
-  return u[off3(g, ii, jj, k)];
-}
-
-__device__ __forceinline__ int src_row(const Grid& g, int jj) { return (jj <= 2) ? (5 - jj) : (2 * g.NJ - 7 - jj); }
-
-struct GhostF {
-  Grid g;
-  float2* u;
-  const double2* up;
-  int inflow;
-};
-
-__global__ void ghost_xy_f32(const GhostF* __restrict__ d) {
-  const GhostF& D = d[blockIdx.y];
-  const Grid& g = D.g;
-  const long long n_rows = 6LL * g.NK * g.NI;
-  const long long n_faces = 2LL * (g.NJ - 6) * g.NK;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n_rows + n_faces;
-       t += (long long)gridDim.x * blockDim.x) {
-    int ii, jj, k, si, sj, sk;
-    if (t < n_rows) {
-      ii = (int)(t % g.NI);
-      const long long rk = t / g.NI;
-      const int r = (int)(rk % 6);
-      k = (int)(rk / 6);
-      jj = (r < 3) ? r : (g.NJ - 6 + r);
-      si = ii;
-      sj = src_row(g, jj);
-      sk = ktarget(g, k);
-    } else {
-      const long long f = t - n_rows;
-      const int nin = g.NJ - 6;
-      jj = 3 + (int)(f % nin);
-      const long long s2 = f / nin;
-      const int side = (int)(s2 % 2);
-      k = (int)(s2 / 2);
-      ii = side ? g.NI - 1 : 0;
-      si = ii;
-      sj = jj;
-      sk = k;
-    }
-#pragma unroll
-    for (int v = 0; v < 5; ++v)
-      D.u[v * g.fs + off3(g, ii, jj, k)] = xval_f(g, D.u + v * g.fs, D.up + v * g.fs, D.inflow, si, sj, sk);
-  }
-}
-
-__global__ void ghost_z_f32(const GhostF* __restrict__ d) {
-  const GhostF& D = d[blockIdx.y];
-  const Grid& g = D.g;
-  const long long n = (long long)g.NI * g.NJ;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < 2 * n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int side = (int)(t / n);
-    const long long q = t % n;
-    const int ii = (int)(q % g.NI), jj = (int)(q / g.NI);
-    const int kd = side ? g.Nz : 0;
-    const int ks = side ? 1 : g.Nz - 1;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) D.u[v * g.fs + off3(g, ii, jj, kd)] = D.u[v * g.fs + off3(g, ii, jj, ks)];
-  }
-}
-
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -793,27 +711,6 @@ int launch_batch_mixed(int kind, int mk, const void* d_items, int n_solves, int 
   if (tj != 8) return -1;
   return mk == MK_KS ? mx_batch_mk<MK_KS, 8>(kind, d_items, n_solves, n_items, blocks, st)
                      : mx_batch_mk<MK_SCHW, 8>(kind, d_items, n_solves, n_items, blocks, st);
-}
-
-size_t ghost_f32_desc_bytes() { return sizeof(GhostF); }
-
-void fill_ghost_f32_desc(void* dst, const Grid& g, float2* u, const double2* up, int inflow) {
-  GhostF* d = reinterpret_cast<GhostF*>(dst);
-  d->g = g;
-  d->u = u;
-  d->up = up;
-  d->inflow = inflow;
-}
-
-void launch_ghost_fill_f32(const void* d_desc, int n, long long max_rows, long long max_faces, long long max_z,
-                           cudaStream_t st) {
-  if (n <= 0) return;
-  long long bx = (max_rows + max_faces + 255) / 256;
-  bx = bx > 1024 ? 1024 : (bx < 1 ? 1 : bx);
-  ghost_xy_f32<<<dim3((unsigned)bx, n), 256, 0, st>>>(reinterpret_cast<const GhostF*>(d_desc));
-  long long bz = (max_z + 255) / 256;
-  bz = bz > 1024 ? 1024 : (bz < 1 ? 1 : bz);
-  ghost_z_f32<<<dim3((unsigned)bz, n), 256, 0, st>>>(reinterpret_cast<const GhostF*>(d_desc));
 }
 
 }  // namespace kg
