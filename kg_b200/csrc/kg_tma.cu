@@ -376,24 +376,33 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
           r[4] = csub(cadd(cadd(cadd(cadd(r1, r2), r3), r4), r5), r6);
         }
         const double dt = g.dt;
-        auto B = [&](int v) { return a.base_in ? fcu[v] : ldf(a.base + v * g.fs, p); };
+        // the point-wise operands of the plane, all requested before the first
+        // store: behind a store each load would wait for its turn (20 RK4 steps on
+        // 301 x 46 x 90 9.36 -> 8.56 ms, no spills)
+        double2 bv[5], sv[5];
+        constexpr bool ACC = KIND == ST_RK4_2 || KIND == ST_RK4_3 || KIND == ST_RK4_4;
+#pragma unroll
+        for (int v = 0; v < 5; ++v)
+          if (v < 4 ? PSI : PI_) {
+            if (ACC) sv[v] = ldf(a.acc, v * g.fs + p);
+            bv[v] = a.base_in ? fcu[v] : ldf(a.base, v * g.fs + p);
+          }
         if (KIND == ST_P2_S1A) {
 #pragma unroll
-          for (int v = 0; v < 4; ++v) a.out[v * g.fs + p] = cadd(B(v), rmul(dt, r[v]));
+          for (int v = 0; v < 4; ++v) a.out[v * g.fs + p] = cadd(bv[v], rmul(dt, r[v]));
         } else if (KIND == ST_P3_S2A) {
 #pragma unroll
           for (int v = 0; v < 4; ++v)
-            a.out[v * g.fs + p] =
-                cadd(rmul(0.75, ldf(a.base + v * g.fs, p)), rmul(0.25, cadd(fcu[v], rmul(dt, r[v]))));
+            a.out[v * g.fs + p] = cadd(rmul(0.75, bv[v]), rmul(0.25, cadd(fcu[v], rmul(dt, r[v]))));
         } else if (KIND == ST_P2_S1B) {
-          a.out4[p] = cadd(ldf(a.base + 4 * g.fs, p), rmul(dt, r[4]));
+          a.out4[p] = cadd(bv[4], rmul(dt, r[4]));
         } else if (KIND == ST_P3_S2B) {
-          a.out4[p] = cadd(rmul(0.75, ldf(a.base + 4 * g.fs, p)), rmul(0.25, cadd(ldf(a.aux4, p), rmul(dt, r[4]))));
+          a.out4[p] = cadd(rmul(0.75, bv[4]), rmul(0.25, cadd(ldf(a.aux4, p), rmul(dt, r[4]))));
         } else if (!(a.skip_last_i && ii == n)) {
 #pragma unroll
           for (int v = 0; v < 5; ++v) {
             const long long o = v * g.fs + p;
-            const double2 b = B(v);
+            const double2 b = bv[v];
             double2 res;
             if (KIND == ST_P2_S2) {
               res = rmul(0.5, cadd(cadd(b, fcu[v]), rmul(dt, r[v])));
@@ -411,15 +420,15 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
               res = cadd(b, rmul(0.50, kk));
             } else if (KIND == ST_RK4_2) {
               const double2 kk = rmul(dt, r[v]);
-              a.acc[o] = cadd(a.acc[o], rmul(2.0, kk));
+              a.acc[o] = cadd(sv[v], rmul(2.0, kk));
               res = cadd(b, rmul(0.50, kk));
             } else if (KIND == ST_RK4_3) {
               const double2 kk = rmul(dt, r[v]);
-              a.acc[o] = cadd(a.acc[o], rmul(2.0, kk));
+              a.acc[o] = cadd(sv[v], rmul(2.0, kk));
               res = cadd(b, kk);
             } else {
               const double2 kk = rmul(dt, r[v]);
-              res = cadd(b, cdivm(cadd(a.acc[o], kk), 6.0, kSixth));
+              res = cadd(b, cdivm(cadd(sv[v], kk), 6.0, kSixth));
             }
             a.out[o] = res;
           }
