@@ -45,9 +45,9 @@ __device__ __forceinline__ int ghost_src_row(const Grid& g, int jj) {
 // What bounds it: on small grids the launch and the latency of one load-store
 // chain per thread, so one launch replaces the former two (ghost rows and faces,
 // then the phi planes); on large ones memory, 2 x 80 B per point of the ghost rows.
-// Measured, event-timed (a launch pair before, one after): 64 x 17 x 33 13.0 ->
-// 8.8 us, 256 x 33 x 65 18.8 -> 12.3 us, 1024 x 65 x 129 43 -> 33 us, 2048 x 129 x
-// 257 124 -> 105 us.
+// Event-timed, two launches before and one after: 301 x 46 x 90 21.5 -> 17.1 us,
+// 1024 x 65 x 129 43.1 -> 33.9 us (FP32 states 37.4 -> 22.1 us).  With the x faces
+// apart (PIRK2) 64 x 17 x 33 13.0 -> 12.1 us, 2048 x 129 x 257 123.8 -> 119.9 us.
 template <class T>
 __device__ __forceinline__ T xval_t(const Grid& g, const T* u, const double2* up, int inflow, int ii, int jj, int k);
 template <>
@@ -140,28 +140,30 @@ static int ghost_threads(int ni) { return ni >= 256 ? 256 : (ni + 31) / 32 * 32;
 
 template <class T>
 __global__ void ghost_kernel(Grid g, T* u, const double2* up, int inflow, int unit0) {
+  pdl_wait();
   ghost_unit(g, u, up, inflow, unit0 + blockIdx.x);
 }
 
 void launch_ghost_fill(const Grid& g, double2* u, const double2* up, int inflow, cudaStream_t st, bool faces_apart) {
   const int nt = ghost_threads(g.NI), n = ghost_units(g, nt), rows = 2 * g.NJ + 6 * (g.Nz - 1);
   if (!faces_apart) {
-    ghost_kernel<double2><<<n, nt, 0, st>>>(g, u, up, inflow, 0);
+    launch_pdl(ghost_kernel<double2>, n, nt, 0, st, g, u, up, inflow, 0);
     return;
   }
-  ghost_kernel<double2><<<rows, nt, 0, st>>>(g, u, up, inflow, 0);
-  ghost_kernel<double2><<<n - rows, nt, 0, st>>>(g, u, up, inflow, rows);
+  launch_pdl(ghost_kernel<double2>, rows, nt, 0, st, g, u, up, inflow, 0);
+  launch_pdl(ghost_kernel<double2>, n - rows, nt, 0, st, g, u, up, inflow, rows);
 }
 
 void launch_ghost_fill_f32(const Grid& g, float2* u, const double2* up, int inflow, cudaStream_t st) {
   const int nt = ghost_threads(g.NI);
-  ghost_kernel<float2><<<ghost_units(g, nt), nt, 0, st>>>(g, u, up, inflow, 0);
+  launch_pdl(ghost_kernel<float2>, ghost_units(g, nt), nt, 0, st, g, u, up, inflow, 0);
 }
 
 // ---- many solves at once (batched engine): one block row per solve -----------
 constexpr int GB_THREADS = 128;
 template <class T>
 __global__ void ghost_batch_kernel(const GhostDesc* __restrict__ d) {
+  pdl_wait();
   const GhostDesc& D = d[blockIdx.y];
   if ((int)blockIdx.x < ghost_units(D.g, GB_THREADS))
     ghost_unit(D.g, static_cast<T*>(D.u), D.up, D.inflow, blockIdx.x);
@@ -171,8 +173,8 @@ int ghost_batch_units(const Grid& g) { return ghost_units(g, GB_THREADS); }
 
 void launch_ghost_fill_batch(const GhostDesc* d_desc, int n, int max_units, int f32, cudaStream_t st) {
   if (n <= 0) return;
-  if (f32) ghost_batch_kernel<float2><<<dim3(max_units, n), GB_THREADS, 0, st>>>(d_desc);
-  else ghost_batch_kernel<double2><<<dim3(max_units, n), GB_THREADS, 0, st>>>(d_desc);
+  launch_pdl(f32 ? ghost_batch_kernel<float2> : ghost_batch_kernel<double2>, dim3(max_units, n), GB_THREADS, 0, st,
+             d_desc);
 }
 
 // ---- one reference routine at a time ---------------------------------------

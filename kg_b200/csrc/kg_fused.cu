@@ -195,6 +195,7 @@ __global__ void __launch_bounds__(NTH, 2)
   };
   int nissued = 0;
   if (tid == 0) {
+    pdl_wait();
     for (int t = 0; t < NSTF && t < NP; ++t) {
       issue(t);
       nissued = t + 1;
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(NTH, 2)
   auto Eglob = [&](int r, int p) {
     const int q = off2(g, c, r);
     const long long o = off3(g, c, r, p);
-    return cadd(rmul(ldm(M.alpha, q), ldf(U + 4 * fs, o)), rmul(ldm(M.beta, q), ldf(U + fs, o)));
+    return cadd(rmul(ldm(M.alpha, q), lds(U + 4 * fs, o)), rmul(ldm(M.beta, q), lds(U + fs, o)));
   };
   // phi-direction difference at plane k from the values at prev(k), next(k)
   // (the seam planes as the reference writes them)
@@ -301,8 +302,9 @@ __global__ void __launch_bounds__(NTH, 2)
   // planes just outside the sequence whose E the psi3 stage at P[0] / P[NP-1] needs
   const int X1 = (plane_of(0) == 0) ? g.Nz - 2 : plane_of(0) - 1;        // prev(P[0])
   const int X4 = (plane_of(NP - 1) == g.Nz) ? 2 : plane_of(NP - 1) + 1;  // next(P[NP-1])
+  pdl_wait();                // ahead of this thread's own reads and writes of the state
   double2 phinx = c2(0, 0);  // phi of the own point at the next inner plane, loaded a step ahead
-  if (own) phinx = ldf(U, pcol + (long long)plane_of(1) * g.plane);
+  if (own) phinx = lds(U, pcol + (long long)plane_of(1) * g.plane);
   __syncthreads();  // metric tables
   const bool ends = (i0 == 0) || (n < i0 + FO);  // the tile holds an array end (block-uniform)
   const bool fast = __all_sync(0xffffffffu, c >= 2 && c <= n - 2 && MAB(mBE, 0, 0) > 0.0);
@@ -374,10 +376,10 @@ __global__ void __launch_bounds__(NTH, 2)
             // (row 2 is an interior row: a centred difference of E)
             const int pk = ktarget(g, p);
             const double2 tt = ctr(Eglob(1, pk), Eglob(3, pk));
-            const double2 s2 = cadd(ldf(U + 2 * fs, off3(g, c, 2, pk)), rmul(g.dt, rmul(g.rdy, tt)));
+            const double2 s2 = cadd(lds(U + 2 * fs, off3(g, c, 2, pk)), rmul(g.dt, rmul(g.rdy, tt)));
             Hpn = rmul(ldm(M.asg_gtt, off2(g, c, 2)), s2);
           }
-          if (t + 1 <= NP - 2) phinx = ldf(U, pcol + (long long)plane_of(t + 1) * g.plane);
+          if (t + 1 <= NP - 2) phinx = lds(U, pcol + (long long)plane_of(t + 1) * g.plane);
         }
       }
       // ---- Pi stage of P[t-1]
@@ -520,8 +522,10 @@ int fused_launch(const CUtensorMap* tms, FusedArgs a, cudaStream_t st) {
   dim3 grid(tiles_x, (g.NJ + FJ - 1) / FJ, 1);
   a.kchunk = phi_chunk(g.NK, (long long)grid.x * grid.y, 148 * 2, 64);
   grid.z = (g.NK + a.kchunk - 1) / a.kchunk;
-  pirk_s1_fused_kernel<MK><<<grid, dim3(FL, FJ, 1), SMEM, st>>>(tms[0], tms[1], tms[2], tms[3], a);
-  return 0;
+  return launch_pdl(pirk_s1_fused_kernel<MK>, grid, dim3(FL, FJ, 1), SMEM, st, tms[0], tms[1], tms[2], tms[3], a) ==
+                 cudaSuccess
+             ? 0
+             : -1;
 }
 
 }  // namespace

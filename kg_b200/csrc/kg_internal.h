@@ -51,6 +51,34 @@ inline int phi_chunk(int planes, long long tiles, int slots, int longest) {
   return best;
 }
 
+// Launches a kernel whose blocks may be set up while the last blocks of the
+// kernel before it on the stream finish (programmatic dependent launch), so that
+// the launch, the barrier set-up and the load of the metric tile, which no kernel
+// writes, do not wait for the full drain.  Such a kernel calls pdl_wait() before
+// it touches anything that earlier work on the stream writes or reads, in every
+// block.  No kernel releases its successor early: with a release at the start
+// the waiting blocks took the slots unevenly and everything got slower (256 x 33
+// x 65 PIRK2 94 -> 104 us a step).  us a pass, without -> with: 40 evolve steps on
+// 64 x 17 x 33 4070 -> 3960, 60 PIRK2 steps on 256 x 33 x 65 5520 -> 5440, three
+// levels of RK4 on 512 x 33 x 65 9640 -> 9290; nothing on the largest grids.
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+// until the kernel before this one has finished and its writes are visible
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 struct StageLaunch {
   Grid g;
   Metric m;

@@ -310,6 +310,7 @@ __device__ __forceinline__ int mx_item(const CUtensorMap* tinp, const CUtensorMa
   };
   int nissued = 0;
   if (tid == 0) {
+    pdl_wait();
     for (int t = 0; t < NST && t < nplanes; ++t) {
       issue(t);
       nissued = t + 1;
@@ -333,6 +334,7 @@ __device__ __forceinline__ int mx_item(const CUtensorMap* tinp, const CUtensorMa
       for (int w = 0; w < MT_COUNT; ++w) mtf[w * MT_N + t] = (float)mt[w * MT_N + t];
   }
   __syncthreads();
+  pdl_wait();  // ahead of this thread's own reads and writes of the state
   // own-point metric: alpha, beta, d_r beta, sqrt(gamma), 1/sqrt(gamma), alpha m^2, phi-flux factors
   double own[9] = {0, 0, 0, 1, 1, 0, 0, 0, 0};
   if (act) {
@@ -435,7 +437,7 @@ __device__ __forceinline__ int mx_item(const CUtensorMap* tinp, const CUtensorMa
         } else if (STG) {
           b = base_s[v * TI * TJ + tid];
         } else {
-          b = ldf(a.base, o);
+          b = lds(a.base, o);
         }
         if (KIND == ST_RK4_1) {
           a.acc[o] = make_float2((float)kk.x, (float)kk.y);
@@ -629,8 +631,10 @@ int mx_launch_one(const CUtensorMap& tin, const CUtensorMap& tp0, const CUtensor
   dim3 grid((g.NI + TI - 1) / TI, (g.NJ - 6 + TJ - 1) / TJ, 1);
   a.kchunk = phi_chunk(planes, (long long)grid.x * grid.y, 148 * MGeom<TJ>::MIN_BLOCKS, 32);
   grid.z = (planes + a.kchunk - 1) / a.kchunk;
-  mx_stage_kernel<KIND, MK, TIN, TJ><<<grid, dim3(TI, TJ, 1), SMEM, st>>>(tin, tp0, tp1, a);
-  return 0;
+  return launch_pdl(mx_stage_kernel<KIND, MK, TIN, TJ>, grid, dim3(TI, TJ, 1), SMEM, st, tin, tp0, tp1, a) ==
+                 cudaSuccess
+             ? 0
+             : -1;
 }
 
 template <int MK, int TJ>
@@ -656,8 +660,10 @@ int mx_batch_one(const void* items, int n_solves, int n_items, int blocks, cudaS
     attr = true;
   }
   if (n_items <= 0) return 0;
-  mx_batch_kernel<KIND, MK, TIN, TJ><<<blocks, dim3(TI, TJ, 1), SMEM, st>>>(reinterpret_cast<const MxItem*>(items), n_solves, n_items);
-  return 0;
+  return launch_pdl(mx_batch_kernel<KIND, MK, TIN, TJ>, blocks, dim3(TI, TJ, 1), SMEM, st,
+                    reinterpret_cast<const MxItem*>(items), n_solves, n_items) == cudaSuccess
+             ? 0
+             : -1;
 }
 
 template <int MK, int TJ>

@@ -184,6 +184,7 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
   };
   int nissued = 0;  // meaningful in thread 0 only
   if (tid == 0) {
+    pdl_wait();
     for (int t = 0; t < NST && t < nplanes; ++t) {
       issue(t);
       nissued = t + 1;
@@ -206,6 +207,7 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
     mt[MT_HT * MT_N + t] = in ? ldm(M.asg_gtt, q) : 0.0;
   }
   __syncthreads();
+  pdl_wait();  // ahead of this thread's own reads and writes of the state
   // own-point metric
   const int q = act ? off2(g, ii, jj) : 0;
   double al = 0, be = 0, dxb = 0, sg = 1, rs = 1, am2 = 0, fa = 0, fgrp = 0, fgpp = 0;
@@ -317,7 +319,7 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
           auto Eg = [&](int j2, int k2) {
             const int q2 = off2(g, ii, j2);
             const long long p2 = off3(g, ii, j2, k2);
-            return cadd(rmul(ldm(M.alpha, q2), ldf(a.in[4], p2)), rmul(ldm(M.beta, q2), ldf(a.in[1], p2)));
+            return cadd(rmul(ldm(M.alpha, q2), lds(a.in[4], p2)), rmul(ldm(M.beta, q2), lds(a.in[1], p2)));
           };
           double2 t;
           if (FILLED) t = ctr(E(-1), E(1));
@@ -346,7 +348,7 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
           const double2 r1 = cdivm(rmul(g.rdx, d), sg, rs);
           auto H = [&](int dy) { return rmul(MTV(MT_HT, tx, ty + dy), RF(cu, 2, tx, ty + dy)); };
           auto Hg = [&](int j2, int k2) {
-            return rmul(ldm(M.asg_gtt, off2(g, ii, j2)), ldf(a.in[2], off3(g, ii, j2, k2)));
+            return rmul(ldm(M.asg_gtt, off2(g, ii, j2)), lds(a.in[2], off3(g, ii, j2, k2)));
           };
           double2 t;
           if (FILLED) t = ctr(H(-1), H(1));
@@ -384,8 +386,8 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
 #pragma unroll
         for (int v = 0; v < 5; ++v)
           if (v < 4 ? PSI : PI_) {
-            if (ACC) sv[v] = ldf(a.acc, v * g.fs + p);
-            bv[v] = a.base_in ? fcu[v] : ldf(a.base, v * g.fs + p);
+            if (ACC) sv[v] = lds(a.acc, v * g.fs + p);
+            bv[v] = a.base_in ? fcu[v] : lds(a.base, v * g.fs + p);
           }
         if (KIND == ST_P2_S1A) {
 #pragma unroll
@@ -397,7 +399,7 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
         } else if (KIND == ST_P2_S1B) {
           a.out4[p] = cadd(bv[4], rmul(dt, r[4]));
         } else if (KIND == ST_P3_S2B) {
-          a.out4[p] = cadd(rmul(0.75, bv[4]), rmul(0.25, cadd(ldf(a.aux4, p), rmul(dt, r[4]))));
+          a.out4[p] = cadd(rmul(0.75, bv[4]), rmul(0.25, cadd(lds(a.aux4, p), rmul(dt, r[4]))));
         } else if (!(a.skip_last_i && ii == n)) {
 #pragma unroll
           for (int v = 0; v < 5; ++v) {
@@ -589,8 +591,9 @@ int launch_one(const Maps& m, TmaArgs a, cudaStream_t st) {
   dim3 grid((g.NI + TI - 1) / TI, (rows + TJ - 1) / TJ, 1);
   a.kchunk = phi_chunk(planes, (long long)grid.x * grid.y, 148 * Geom<TJ>::MIN_BLOCKS, 32);
   grid.z = (planes + a.kchunk - 1) / a.kchunk;
-  tma_stage_kernel<KIND, MK, TJ><<<grid, block, SMEM, st>>>(m.tm4, m.tm1, m.tp0, m.tp1, a);
-  return 0;
+  return launch_pdl(tma_stage_kernel<KIND, MK, TJ>, grid, block, SMEM, st, m.tm4, m.tm1, m.tp0, m.tp1, a) == cudaSuccess
+             ? 0
+             : -1;
 }
 
 // the 4-row tiles are built for the RK4 stages (the batched forms' stepper) only
@@ -679,8 +682,10 @@ int batch_one(const void* items, int n_solves, int n_items, int blocks, cudaStre
     attr_set = true;
   }
   if (n_items <= 0) return 0;
-  tma_batch_kernel<KIND, MK, TJ><<<blocks, dim3(TI, TJ, 1), SMEM, st>>>(reinterpret_cast<const BatchItem*>(items), n_solves, n_items);
-  return 0;
+  return launch_pdl(tma_batch_kernel<KIND, MK, TJ>, blocks, dim3(TI, TJ, 1), SMEM, st,
+                    reinterpret_cast<const BatchItem*>(items), n_solves, n_items) == cudaSuccess
+             ? 0
+             : -1;
 }
 template <int KIND>
 int batch_kind(const void* items, int n_solves, int n_items, int blocks, int mk, int tj, cudaStream_t st) {
