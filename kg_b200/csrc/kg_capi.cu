@@ -2006,7 +2006,8 @@ struct kg_batch {
   size_t items_cap = 0, ghost_cap = 0;
   int n_items[4] = {0, 0, 0, 0};
   int ghost_units = 0;                                       // the largest member's
-  int* derr = nullptr;
+  int* derr = nullptr;  // error flag, then (at 16 bytes) the stages' work-list counters
+  kg::BatchCounter* counters() const { return reinterpret_cast<kg::BatchCounter*>(derr + 4); }
   cudaGraphExec_t graph = nullptr;
   long long graph_launches = 0;
   long long launches = 0;
@@ -2035,8 +2036,36 @@ struct kg_batch {
 
 namespace {
 
+constexpr size_t BATCH_FLAGS = 16 + 4 * sizeof(kg::BatchCounter);
+
+// Phi planes per work item, at most the tuned kchunk: kg::phi_chunk's rule on the
+// whole list.  Long items leave the last wave of a list of a few items per CTA
+// nearly empty.  (Ten mixed steps of 16 solves, Nr 128..512, Ntheta 16 or 32, kchunk
+// 32: 23.76 -> 22.43 ms a pass, with the items taken from a counter.)
+int batch_chunk(const kg_batch* b) {
+  int best = b->kchunk;
+  double cost = 1e300;
+  int longest = 1;
+  for (const kg_solver* h : b->members) longest = std::max(longest, h->NK - 1);
+  for (int c = 1; c <= std::min(b->kchunk, longest); ++c) {
+    double items = 0.0;
+    for (const kg_solver* h : b->members) {
+      const double tiles = (double)((h->NI + 31) / 32) * ((h->NJ - 6 + b->tile_rows - 1) / b->tile_rows);
+      items += tiles * ((h->NK - 1 + c - 1) / c);
+    }
+    const double waves = items / b->blocks + 0.25;
+    const double t = (waves > 1.0 ? waves : 1.0) * (c + 1);
+    if (t < cost) {
+      cost = t;
+      best = c;
+    }
+  }
+  return best;
+}
+
 int batch_rebuild(kg_batch* b) {
   const int n = (int)b->members.size();
+  const int kchunk = batch_chunk(b);
   const bool mixed = b->precision == 1;
   const size_t isz = mixed ? kg::mixed_item_bytes() : kg::batch_item_bytes();
   const size_t isz_max = std::max(kg::mixed_item_bytes(), kg::batch_item_bytes());
@@ -2077,7 +2106,7 @@ int batch_rebuild(kg_batch* b) {
         M.out_d = st == 3 ? h->U : nullptr;
         M.skip_last_i = st == 3 ? inflow : 0;
         const double* rsg = h->dmet + (size_t)T_RSG * h->NJ * h->PI;
-        const int ni = kg::build_mixed_item(hitems.data() + (size_t)i * isz, kinds[st], M, rsg, b->derr, b->kchunk,
+        const int ni = kg::build_mixed_item(hitems.data() + (size_t)i * isz, kinds[st], M, rsg, b->derr, kchunk,
                                             item0, b->tile_rows);
         if (ni < 0) {
           b->err = "tensor-map encoding failed for a batch member";
@@ -2100,7 +2129,7 @@ int batch_rebuild(kg_batch* b) {
       L.out = out;
       L.skip_last_i = (st == 3) ? (h->p.bc_rmax == KG_INFLOW) : 0;
       const double* rsg = h->dmet + (size_t)T_RSG * h->NJ * h->PI;
-      const int ni = kg::build_batch_item(hitems.data() + (size_t)i * isz, kinds[st], L, rsg, b->derr, b->kchunk,
+      const int ni = kg::build_batch_item(hitems.data() + (size_t)i * isz, kinds[st], L, rsg, b->derr, kchunk,
                                           item0, b->tile_rows);
       if (ni < 0) {
         b->err = "tensor-map encoding failed for a batch member";
@@ -2126,9 +2155,9 @@ int batch_enqueue_step(kg_batch* b) {
   for (int st = 0; st < 4; ++st) {
     const int bad = b->precision == 1
                         ? kg::launch_batch_mixed(kinds[st], b->metric_kind, b->ditems[st], n, b->n_items[st],
-                                                 b->blocks, b->tile_rows, b->stream)
+                                                 b->blocks, b->tile_rows, b->counters() + st, b->stream)
                         : kg::launch_batch_tma(kinds[st], b->metric_kind, b->ditems[st], n, b->n_items[st],
-                                               b->blocks, b->tile_rows, b->stream);
+                                               b->blocks, b->tile_rows, b->counters() + st, b->stream);
     if (bad) {
       b->err = "batched stage launch could not be configured";
       return KG_ECUDA;
@@ -2160,7 +2189,8 @@ int kg_batch_create(int device, kg_batch** out) {
   b->blocks = 2 * sms;
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&b->ev, cudaEventDisableTiming) != cudaSuccess ||
-      cudaMalloc((void**)&b->derr, 16) != cudaSuccess || cudaMemsetAsync(b->derr, 0, 16, b->stream) != cudaSuccess ||
+      cudaMalloc((void**)&b->derr, BATCH_FLAGS) != cudaSuccess ||
+      cudaMemsetAsync(b->derr, 0, BATCH_FLAGS, b->stream) != cudaSuccess ||
       cudaStreamSynchronize(b->stream) != cudaSuccess) {
     kg_batch_destroy(b);
     return KG_ECUDA;

@@ -109,11 +109,22 @@ int launch_wait_check(int* err, long long polls, cudaStream_t st);
 // true when the driver can encode the tensor maps the TMA form needs for this grid
 bool tma_available(const Grid& g, const double2* some_state);
 // batched (multi-solve) persistent launches of the TMA stage kernel
+// the work list's position, one per stage kind of a batch: zero before and after a
+// launch (the last CTA to leave clears it)
+struct BatchCounter {
+  int next, left;
+};
+__device__ __forceinline__ void batch_done(BatchCounter* c) {
+  if (threadIdx.x == 0 && threadIdx.y == 0 && atomicAdd(&c->left, 1) == (int)gridDim.x - 1) {
+    c->next = 0;
+    c->left = 0;
+  }
+}
 size_t batch_item_bytes();
 int build_batch_item(void* dst, int kind, const StageLaunch& L, const double* rsg, int* err, int kchunk, int item0,
                      int tj);
 int launch_batch_tma(int kind, int mk, const void* d_items, int n_solves, int n_items, int blocks, int tj,
-                     cudaStream_t st);
+                     BatchCounter* ctr, cudaStream_t st);
 // Y_lm projection over all shells (kg_ylm_gemm.cu)
 int ylm_gemm_pad_m(int rows);
 int ylm_gemm_pad_n(int cols);
@@ -147,7 +158,7 @@ size_t mixed_item_bytes();
 int build_mixed_item(void* dst, int kind, const MixedLaunch& L, const double* rsg, int* err, int kchunk, int item0,
                      int tj);
 int launch_batch_mixed(int kind, int mk, const void* d_items, int n_solves, int n_items, int blocks, int tj,
-                       cudaStream_t st);
+                       BatchCounter* ctr, cudaStream_t st);
 // configured method (kg_config.cu): RK4 stage with fourth-order differences,
 // Kreiss-Oliger dissipation and a Sommerfeld outer plane; coef = 1/(12 h) for
 // r, theta, phi then eps/(64 h) for r, theta, phi; rN = outermost r; rsg = the

@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(TI * TJ, MGeom<TJ>::MIN_BLOCKS)
 
 template <int KIND, int MK, class TIN, int TJ>
 __global__ void __launch_bounds__(TI * TJ, MGeom<TJ>::MIN_BLOCKS)
-    mx_batch_kernel(const MxItem* __restrict__ solves, int n_solves, int n_items) {
+    mx_batch_kernel(const MxItem* __restrict__ solves, int n_solves, int n_items, BatchCounter* ctr) {
   using GT = MGeom<TJ>;
   constexpr int MT_N = GT::MT_N;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -527,11 +527,13 @@ __global__ void __launch_bounds__(TI * TJ, MGeom<TJ>::MIN_BLOCKS)
                                                (sizeof(TIN) == 4 ? (size_t)MT_COUNT * MT_N * 4 : 0));
   unsigned char* stg = reinterpret_cast<unsigned char*>(bars + 8);
   __shared__ MxArgs sa;
-  __shared__ int s_bx, s_by, s_bz, s_solve;
+  __shared__ int s_bx, s_by, s_bz, s_solve, s_next;
   init_bars<TJ>(bars);
   uint32_t tb = 0;
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+  pdl_wait();
+  for (int item = blockIdx.x, next; item < n_items; item = next) {
     if (threadIdx.x == 0 && threadIdx.y == 0) {
+      s_next = gridDim.x + atomicAdd(&ctr->next, 1);  // under this item's work
       int lo = 0, hi = n_solves - 1;
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -547,12 +549,14 @@ __global__ void __launch_bounds__(TI * TJ, MGeom<TJ>::MIN_BLOCKS)
       sa = B.a;
     }
     __syncthreads();
+    next = s_next;
     const MxItem& B = solves[s_solve];
     const int used = mx_item<KIND, MK, TIN, TJ>(&B.tin, &B.tp0, &B.tp1, sa, s_bx, s_by, s_bz, ring, mt, bars, tb, stg);
     if (used < 0) break;
     tb += (uint32_t)used;
     __syncthreads();
   }
+  batch_done(ctr);
 }
 
 // ---------------------------------------------------------------------------
@@ -650,7 +654,7 @@ int mx_launch_mk(int kind, const CUtensorMap& tin, const CUtensorMap& tp0, const
 }
 
 template <int KIND, int MK, class TIN, int TJ>
-int mx_batch_one(const void* items, int n_solves, int n_items, int blocks, cudaStream_t st) {
+int mx_batch_one(const void* items, int n_solves, int n_items, int blocks, BatchCounter* ctr, cudaStream_t st) {
   constexpr size_t SMEM = MGeom<TJ>::template smem<TIN>();
   static bool attr = false;
   if (!attr) {
@@ -661,18 +665,19 @@ int mx_batch_one(const void* items, int n_solves, int n_items, int blocks, cudaS
   }
   if (n_items <= 0) return 0;
   return launch_pdl(mx_batch_kernel<KIND, MK, TIN, TJ>, blocks, dim3(TI, TJ, 1), SMEM, st,
-                    reinterpret_cast<const MxItem*>(items), n_solves, n_items) == cudaSuccess
+                    reinterpret_cast<const MxItem*>(items), n_solves, n_items, ctr) == cudaSuccess
              ? 0
              : -1;
 }
 
 template <int MK, int TJ>
-int mx_batch_mk(int kind, const void* items, int n_solves, int n_items, int blocks, cudaStream_t st) {
+int mx_batch_mk(int kind, const void* items, int n_solves, int n_items, int blocks, BatchCounter* ctr,
+                cudaStream_t st) {
   switch (kind) {
-    case ST_RK4_1: return mx_batch_one<ST_RK4_1, MK, double, TJ>(items, n_solves, n_items, blocks, st);
-    case ST_RK4_2: return mx_batch_one<ST_RK4_2, MK, float, TJ>(items, n_solves, n_items, blocks, st);
-    case ST_RK4_3: return mx_batch_one<ST_RK4_3, MK, float, TJ>(items, n_solves, n_items, blocks, st);
-    case ST_RK4_4: return mx_batch_one<ST_RK4_4, MK, float, TJ>(items, n_solves, n_items, blocks, st);
+    case ST_RK4_1: return mx_batch_one<ST_RK4_1, MK, double, TJ>(items, n_solves, n_items, blocks, ctr, st);
+    case ST_RK4_2: return mx_batch_one<ST_RK4_2, MK, float, TJ>(items, n_solves, n_items, blocks, ctr, st);
+    case ST_RK4_3: return mx_batch_one<ST_RK4_3, MK, float, TJ>(items, n_solves, n_items, blocks, ctr, st);
+    case ST_RK4_4: return mx_batch_one<ST_RK4_4, MK, float, TJ>(items, n_solves, n_items, blocks, ctr, st);
     default: return -1;
   }
 }
@@ -710,13 +715,13 @@ int build_mixed_item(void* dst, int kind, const MixedLaunch& L, const double* rs
 }
 
 int launch_batch_mixed(int kind, int mk, const void* d_items, int n_solves, int n_items, int blocks, int tj,
-                       cudaStream_t st) {
+                       BatchCounter* ctr, cudaStream_t st) {
   if (tj == 4)
-    return mk == MK_KS ? mx_batch_mk<MK_KS, 4>(kind, d_items, n_solves, n_items, blocks, st)
-                       : mx_batch_mk<MK_SCHW, 4>(kind, d_items, n_solves, n_items, blocks, st);
+    return mk == MK_KS ? mx_batch_mk<MK_KS, 4>(kind, d_items, n_solves, n_items, blocks, ctr, st)
+                       : mx_batch_mk<MK_SCHW, 4>(kind, d_items, n_solves, n_items, blocks, ctr, st);
   if (tj != 8) return -1;
-  return mk == MK_KS ? mx_batch_mk<MK_KS, 8>(kind, d_items, n_solves, n_items, blocks, st)
-                     : mx_batch_mk<MK_SCHW, 8>(kind, d_items, n_solves, n_items, blocks, st);
+  return mk == MK_KS ? mx_batch_mk<MK_KS, 8>(kind, d_items, n_solves, n_items, blocks, ctr, st)
+                     : mx_batch_mk<MK_SCHW, 8>(kind, d_items, n_solves, n_items, blocks, ctr, st);
 }
 
 }  // namespace kg

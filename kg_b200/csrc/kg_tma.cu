@@ -496,21 +496,24 @@ __global__ void __launch_bounds__(TI * TJ, Geom<TJ>::MIN_BLOCKS)
 
 // ---- persistent kernel over many solves -------------------------------------
 // Every solve of a batch contributes tiles_x * tiles_y * chunks work items; a
-// CTA walks the ragged list item = blockIdx.x, blockIdx.x + gridDim.x, ...
-// and runs each with the solve's own grid, metric, buffers and tensor maps.
+// CTA takes the first by its index and each further one from a counter (items
+// differ in length, and in the mixed form those next to the poles take longer),
+// and runs it with the solve's own grid, metric, buffers and tensor maps.
 template <int KIND, int MK, int TJ>
 __global__ void __launch_bounds__(TI * TJ, Geom<TJ>::MIN_BLOCKS)
-    tma_batch_kernel(const BatchItem* __restrict__ solves, int n_solves, int n_items) {
+    tma_batch_kernel(const BatchItem* __restrict__ solves, int n_solves, int n_items, BatchCounter* ctr) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   double* ring = reinterpret_cast<double*>(align128(smem_raw));
   double* mt = ring + (size_t)NST * Geom<TJ>::STAGE_D;
   uint64_t* bars = reinterpret_cast<uint64_t*>(mt + (size_t)MT_COUNT * Geom<TJ>::MT_N);
   __shared__ TmaArgs sa;
-  __shared__ int s_bx, s_by, s_bz, s_solve;
+  __shared__ int s_bx, s_by, s_bz, s_solve, s_next;
   init_ring_barriers<TJ>(bars);
   uint32_t tb = 0;
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+  pdl_wait();
+  for (int item = blockIdx.x, next; item < n_items; item = next) {
     if (threadIdx.x == 0 && threadIdx.y == 0) {
+      s_next = gridDim.x + atomicAdd(&ctr->next, 1);  // under this item's work
       int lo = 0, hi = n_solves - 1;
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -526,12 +529,14 @@ __global__ void __launch_bounds__(TI * TJ, Geom<TJ>::MIN_BLOCKS)
       sa = B.a;
     }
     __syncthreads();
+    next = s_next;
     const BatchItem& B = solves[s_solve];
     const int used = stage_item<KIND, MK, TJ>(&B.tm4, &B.tm1, &B.tp0, &B.tp1, sa, s_bx, s_by, s_bz, ring, mt, bars, tb);
     if (used < 0) break;
     tb += (uint32_t)used;
     __syncthreads();  // sa and the item indices are rewritten for the next item
   }
+  batch_done(ctr);
 }
 
 // ---------------------------------------------------------------------------
@@ -672,7 +677,7 @@ int build_batch_item(void* dst, int kind, const StageLaunch& L, const double* rs
 
 namespace {
 template <int KIND, int MK, int TJ>
-int batch_one(const void* items, int n_solves, int n_items, int blocks, cudaStream_t st) {
+int batch_one(const void* items, int n_solves, int n_items, int blocks, BatchCounter* ctr, cudaStream_t st) {
   constexpr size_t SMEM = Geom<TJ>::SMEM_BYTES;
   static bool attr_set = false;
   if (!attr_set) {
@@ -683,30 +688,31 @@ int batch_one(const void* items, int n_solves, int n_items, int blocks, cudaStre
   }
   if (n_items <= 0) return 0;
   return launch_pdl(tma_batch_kernel<KIND, MK, TJ>, blocks, dim3(TI, TJ, 1), SMEM, st,
-                    reinterpret_cast<const BatchItem*>(items), n_solves, n_items) == cudaSuccess
+                    reinterpret_cast<const BatchItem*>(items), n_solves, n_items, ctr) == cudaSuccess
              ? 0
              : -1;
 }
 template <int KIND>
-int batch_kind(const void* items, int n_solves, int n_items, int blocks, int mk, int tj, cudaStream_t st) {
+int batch_kind(const void* items, int n_solves, int n_items, int blocks, int mk, int tj, BatchCounter* ctr,
+               cudaStream_t st) {
   if constexpr (has_tj4<KIND>()) {
     if (tj == 4)
-      return mk == MK_KS ? batch_one<KIND, MK_KS, 4>(items, n_solves, n_items, blocks, st)
-                         : batch_one<KIND, MK_SCHW, 4>(items, n_solves, n_items, blocks, st);
+      return mk == MK_KS ? batch_one<KIND, MK_KS, 4>(items, n_solves, n_items, blocks, ctr, st)
+                         : batch_one<KIND, MK_SCHW, 4>(items, n_solves, n_items, blocks, ctr, st);
   }
   if (tj != 8) return -1;
-  return mk == MK_KS ? batch_one<KIND, MK_KS, 8>(items, n_solves, n_items, blocks, st)
-                     : batch_one<KIND, MK_SCHW, 8>(items, n_solves, n_items, blocks, st);
+  return mk == MK_KS ? batch_one<KIND, MK_KS, 8>(items, n_solves, n_items, blocks, ctr, st)
+                     : batch_one<KIND, MK_SCHW, 8>(items, n_solves, n_items, blocks, ctr, st);
 }
 }  // namespace
 
 int launch_batch_tma(int kind, int mk, const void* d_items, int n_solves, int n_items, int blocks, int tj,
-                     cudaStream_t st) {
+                     BatchCounter* ctr, cudaStream_t st) {
   switch (kind) {
-    case ST_RK4_1: return batch_kind<ST_RK4_1>(d_items, n_solves, n_items, blocks, mk, tj, st);
-    case ST_RK4_2: return batch_kind<ST_RK4_2>(d_items, n_solves, n_items, blocks, mk, tj, st);
-    case ST_RK4_3: return batch_kind<ST_RK4_3>(d_items, n_solves, n_items, blocks, mk, tj, st);
-    case ST_RK4_4: return batch_kind<ST_RK4_4>(d_items, n_solves, n_items, blocks, mk, tj, st);
+    case ST_RK4_1: return batch_kind<ST_RK4_1>(d_items, n_solves, n_items, blocks, mk, tj, ctr, st);
+    case ST_RK4_2: return batch_kind<ST_RK4_2>(d_items, n_solves, n_items, blocks, mk, tj, ctr, st);
+    case ST_RK4_3: return batch_kind<ST_RK4_3>(d_items, n_solves, n_items, blocks, mk, tj, ctr, st);
+    case ST_RK4_4: return batch_kind<ST_RK4_4>(d_items, n_solves, n_items, blocks, mk, tj, ctr, st);
     default: return -1;
   }
 }
