@@ -62,7 +62,7 @@ struct kg_solver {
   size_t stage_bytes = 0;
   int stage_planes = 0;
   double* rho = nullptr;
-  double* partials = nullptr;            // mass partial sums + result
+  double* partials = nullptr;            // mass partial sums, result, CTA counter
   int s_cur = 4, t_cur = 4;              // slot holding the current Pi stage value
   int variant = 3;                       // 0: per-point, 1: 2.5-D marching, 2, 3: TMA-pipelined marching
                                          // (3: PIRK stage 1 fused in one kernel; 2: two launches)
@@ -739,6 +739,12 @@ void run_ghost(kg_solver* h, double2* u, const double2* up, int inflow, bool fac
   kg::launch_ghost_fill(h->g, u, up, inflow, h->stream, faces_apart);
 }
 
+// a_lm and fluxes of the detector shells
+void shell_reduce(kg_solver* h, bool alm, bool flux, cudaStream_t st) {
+  kg::launch_shell_reduce(h->shells, h->si.active, h->n_det, h->L, h->Ny, h->Nz, h->normP, h->cosm, h->sinm, h->sint,
+                          h->dy * h->dz, alm ? h->alm : nullptr, flux ? h->flux : nullptr, st);
+}
+
 kg::StageLaunch base_launch(kg_solver* h) {
   kg::StageLaunch L;
   memset(&L, 0, sizeof(L));
@@ -824,7 +830,7 @@ int kg_create(const kg_params* p, int device, kg_solver** out) {
   int rc = KG_OK;
   if ((rc = dalloc(h, (void**)&h->dmet, (size_t)T_COUNT * h->NJ * h->PI * sizeof(double))) ||
       (rc = upload_tables(h)) || (rc = dalloc(h, (void**)&h->U, 5 * field_bytes(h))) ||
-      (rc = dalloc(h, (void**)&h->partials, (size_t)(kg::mass_blocks(g) + 1) * sizeof(double))) ||
+      (rc = dalloc(h, (void**)&h->partials, (size_t)(kg::mass_blocks(g) + 2) * sizeof(double))) ||
       (rc = dalloc(h, (void**)&h->derr, 16)) ||
       (rc = build_detectors(h))) {
     kg_destroy(h);
@@ -1507,7 +1513,7 @@ int kg_mass_scalar(kg_solver* h, double* out) {
   }
   double* res = h->partials + kg::mass_blocks(h->g);
   {
-    Prof pf(h, PK_MASS, 2);
+    Prof pf(h, PK_MASS, 1);
     kg::launch_mass(h->g, metric_of(h), h->rho, h->dx * h->dy * h->dz, h->partials, res, h->stream);
   }
   KG_CK(cudaGetLastError());
@@ -1519,12 +1525,12 @@ int kg_mass_scalar(kg_solver* h, double* out) {
 int kg_currents_detectors(kg_solver* h, double* mom) {
   if (!h || !mom) return KG_EINVAL;
   {
-    Prof pf(h, PK_SHELL, __builtin_popcount(2 | 4 | 8));
-    kg::launch_shell_interp(h->g, metric_of(h), h->U, h->si, h->n_det, h->Ny, h->Nz, 2 | 4 | 8, h->shells, h->stream);
+    Prof pf(h, PK_SHELL, 1);
+    kg::launch_shell_interp(h->g, metric_of(h), h->U, h->si, h->n_det, h->Ny, h->Nz, 14, h->shells, h->stream);
   }
   {
     Prof pf(h, PK_FLUX, 1);
-    kg::launch_flux(h->shells, h->si.active, h->n_det, h->Ny, h->Nz, h->dy * h->dz, h->flux, h->stream);
+    shell_reduce(h, false, true, h->stream);
   }
   KG_CK(cudaGetLastError());
   std::vector<double> f(3 * (size_t)h->n_det);
@@ -1539,13 +1545,12 @@ int kg_currents_detectors(kg_solver* h, double* mom) {
 int kg_proyector_detectors(kg_solver* h, double* host_alm) {
   if (!h || !host_alm) return KG_EINVAL;
   {
-    Prof pf(h, PK_SHELL, __builtin_popcount(1));
+    Prof pf(h, PK_SHELL, 1);
     kg::launch_shell_interp(h->g, metric_of(h), h->U, h->si, h->n_det, h->Ny, h->Nz, 1, h->shells, h->stream);
   }
   {
     Prof pf(h, PK_PROJECT, 1);
-    kg::launch_project(h->shells, h->si.active, h->n_det, h->L, h->Ny, h->Nz, h->normP, h->cosm, h->sinm, h->sint,
-                     h->dy * h->dz, h->alm, h->stream);
+    shell_reduce(h, true, false, h->stream);
   }
   KG_CK(cudaGetLastError());
   const size_t per = (size_t)(h->L + 1) * (2 * h->L + 1);
@@ -1561,17 +1566,12 @@ int kg_diagnostic(kg_solver* h, int index, double* mass_out) {
   if (!h) return KG_EINVAL;
   if (index % h->save == 0) {
     {
-      Prof pf(h, PK_SHELL, __builtin_popcount(15));
+      Prof pf(h, PK_SHELL, 1);
       kg::launch_shell_interp(h->g, metric_of(h), h->U, h->si, h->n_det, h->Ny, h->Nz, 15, h->shells, h->stream);
     }
     {
-      Prof pf(h, PK_FLUX, 1);
-      kg::launch_flux(h->shells, h->si.active, h->n_det, h->Ny, h->Nz, h->dy * h->dz, h->flux, h->stream);
-    }
-    {
-      Prof pf(h, PK_PROJECT, 1);
-      kg::launch_project(h->shells, h->si.active, h->n_det, h->L, h->Ny, h->Nz, h->normP, h->cosm, h->sinm, h->sint,
-                       h->dy * h->dz, h->alm, h->stream);
+      Prof pf(h, PK_PROJECT, 1);  // the fluxes with it
+      shell_reduce(h, true, true, h->stream);
     }
     KG_CK(cudaGetLastError());
   }
@@ -2361,8 +2361,7 @@ int kg_batch_proyector_detectors(kg_batch* b, double* host_alm) {
   for (kg_solver* h : b->members) {
     const size_t n = (size_t)(h->L + 1) * (2 * h->L + 1) * h->n_det;
     kg::launch_shell_interp(h->g, metric_of(h), h->U, h->si, h->n_det, h->Ny, h->Nz, 1, h->shells, b->stream);
-    kg::launch_project(h->shells, h->si.active, h->n_det, h->L, h->Ny, h->Nz, h->normP, h->cosm, h->sinm, h->sint,
-                       h->dy * h->dz, h->alm, b->stream);
+    shell_reduce(h, true, false, b->stream);
     KG_BCK(cudaMemcpyAsync(b->pin + off, h->alm, n * sizeof(double2), cudaMemcpyDeviceToHost, b->stream));
     off += n;
   }

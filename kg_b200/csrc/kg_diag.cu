@@ -91,8 +91,16 @@ int mass_blocks(const Grid& g) { return 148 * 4; }  // one wave at 4 CTAs (64 re
 // loads are coalesced and no per-point index division is needed; the block
 // count is fixed, so the partial sums (and the result) do not depend on the
 // device.
-__global__ void mass_partial_kernel(Grid g, const double* __restrict__ sqrtg, const double* __restrict__ rho,
-                                    double* partials) {
+// One launch: the CTA that finishes last (a counter behind a fence, cleared for
+// the next call) adds the partials, in the same fixed order as a second launch
+// would.  A grid with fewer rows than 8 per CTA leaves the surplus CTAs out; their
+// partials were zero.
+struct MassSum {
+  double value;
+  unsigned int left;
+};
+__global__ void mass_kernel(Grid g, const double* __restrict__ sqrtg, const double* __restrict__ rho,
+                            double* partials, MassSum* sum, double scale) {
   const int ni = g.NI - 4, nj = g.NJ - 4, nk = g.NK;
   const int rows = nj * nk;
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -122,21 +130,45 @@ __global__ void mass_partial_kernel(Grid g, const double* __restrict__ sqrtg, co
     }
   }
   acc = block_sum(acc);
-  if (threadIdx.x == 0) partials[blockIdx.x] = acc;
-}
-
-__global__ void sum_partials_kernel(const double* partials, int n, double scale, double* out) {
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) acc += partials[i];
-  acc = block_sum(acc);
-  if (threadIdx.x == 0) *out = acc * scale;
+  __shared__ int last;
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = acc;
+    __threadfence();
+    last = atomicAdd(&sum->left, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // 1024 strided sums and their tree, by 256 threads of four sums each
+  double t4[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    t4[q] = 0.0;
+    for (int i = threadIdx.x + MASS_THREADS * q; i < (int)gridDim.x; i += 4 * MASS_THREADS) t4[q] += __ldcg(partials + i);
+  }
+  // warp w of 32 held threads 32 w .. 32 w + 31: here warps 0..7 hold eight of them per q
+  __shared__ double ws[32];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const double v = warp_sum(t4[q]);
+    if (lane == 0) ws[(threadIdx.x >> 5) + 8 * q] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const double v = warp_sum(ws[threadIdx.x]);
+    if (threadIdx.x == 0) {
+      sum->value = v * scale;
+      sum->left = 0u;
+    }
+  }
 }
 
 void launch_mass(const Grid& g, const Metric& m, const double* rho, double dxdydz, double* partials, double* out,
                  cudaStream_t st) {
-  const int nb = mass_blocks(g);
-  mass_partial_kernel<<<nb, MASS_THREADS, 0, st>>>(g, m.sqrtg, rho, partials);
-  sum_partials_kernel<<<1, 1024, 0, st>>>(partials, nb, dxdydz, out);
+  const long long rows = (long long)(g.NJ - 4) * g.NK;
+  const int nw = MASS_THREADS / 32;
+  const int nb = (int)(rows < (long long)nw * mass_blocks(g) ? (rows + nw - 1) / nw : mass_blocks(g));
+  mass_kernel<<<nb, MASS_THREADS, 0, st>>>(g, m.sqrtg, rho, partials, reinterpret_cast<MassSum*>(out), dxdydz);
 }
 
 // ---- detector shells ---------------------------------------------------------
@@ -145,58 +177,70 @@ void launch_mass(const Grid& g, const Metric& m, const double* rho, double dxdyd
 // the weights depend only on the vertex index in each direction; they are
 // computed once on the host with the reference's arithmetic and passed in.
 //   src: 0 = phi, 1..3 = j_i * sqrtg (currents_ADM, diagnostic_lib.f90:219-229)
-template <int SRC>
-__device__ __forceinline__ double2 shell_src(const Grid& g, const Metric& m, const double2* u, int ii, int jj,
-                                             int k) {
-  const long long p = off3(g, ii, jj, k);
-  if (SRC == 0) return u[p];
-  const int q = off2(g, ii, jj);
-  const double2 u2 = u[g.fs + p], u3 = u[2 * g.fs + p], u4 = u[3 * g.fs + p], u5 = u[4 * g.fs + p];
-  const double2 n5 = cneg(u5);
-  double2 a;
-  if (SRC == 1) a = cadd(rmul(m.grr[q], u2), rmul(m.grp[q], u4));
-  else if (SRC == 2) a = rmul(m.gtt[q], u3);
-  else a = cadd(rmul(m.grp[q], u2), rmul(m.gpp[q], u4));
-  const double2 j = c2(n5.x * a.x - n5.y * a.y, n5.x * a.y + n5.y * a.x);
-  const double sg = m.sqrtg[q];
-  return c2(j.x * sg, j.y * sg);
-}
-
-template <int SRC>
+// One thread forms every field asked for (bit 0: phi, bits 1..3: the currents)
+// at its vertex: the eight corners' values are loaded once, as independent loads,
+// where a launch per field read them again behind a launch each.  The kernel is
+// bound by that one latency on the grids that are sampled every few steps: four
+// fields on 64 x 17 x 33, five detectors, 31 -> 8.7 us event-timed.
+template <int MASK>
 __global__ void shell_interp_kernel(Grid g, Metric m, const double2* __restrict__ u, ShellInterp si, int Ny, int Nz,
                                     double2* __restrict__ out) {
+  constexpr int NF = MASK == 1 ? 1 : (MASK & 1) ? 4 : 3, F0 = (MASK & 1) ? 0 : 1;  // fields F0 .. F0 + NF - 1
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int d = blockIdx.y;
   if (t >= Ny * Nz || !si.active[d]) return;
   const int jv = t % Ny, kv = t / Ny;
   const int ir = si.i_r[d], ith = si.i_th[jv], iph = si.i_ph[kv];
-  double2* o = out + ((long long)d * 4 + SRC) * Ny * Nz + t;
+  double2* o = out + (long long)d * 4 * Ny * Nz + t;
+  // the fields at one stored point (currents_ADM, diagnostic_lib.f90:219-229)
+  auto src = [&](int ii, int jj, int k, double2 (&f)[NF]) {
+    const long long p = off3(g, ii, jj, k);
+    if (MASK & 1) f[0] = u[p];
+    if (MASK & 14) {
+      const int q = off2(g, ii, jj);
+      const double2 u2 = u[g.fs + p], u3 = u[2 * g.fs + p], u4 = u[3 * g.fs + p], u5 = u[4 * g.fs + p];
+      const double2 n5 = cneg(u5);
+      const double sg = m.sqrtg[q], grp = m.grp[q];
+      const double2 a[3] = {cadd(rmul(m.grr[q], u2), rmul(grp, u4)), rmul(m.gtt[q], u3),
+                            cadd(rmul(grp, u2), rmul(m.gpp[q], u4))};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double2 j = c2(n5.x * a[c].x - n5.y * a[c].y, n5.x * a[c].y + n5.y * a[c].x);
+        f[NF - 3 + c] = c2(j.x * sg, j.y * sg);
+      }
+    }
+  };
   const int fl = si.th_flag[jv];
-  if (fl == 1) { *o = shell_src<SRC>(g, m, u, ir, 0, iph); return; }
-  if (fl == 2) { *o = shell_src<SRC>(g, m, u, ir, g.NJ - 1, iph); return; }
-  const int ip1 = iph + 1;
+  if (fl) {
+    double2 f[NF];
+    src(ir, fl == 1 ? 0 : g.NJ - 1, iph, f);
+#pragma unroll
+    for (int v = 0; v < NF; ++v) o[(long long)(F0 + v) * Ny * Nz] = f[v];
+    return;
+  }
   const double wr = si.w_r[d], wt = si.w_th[jv], wp = si.w_ph[kv];
-  const double2 f000 = shell_src<SRC>(g, m, u, ir, ith, iph), f001 = shell_src<SRC>(g, m, u, ir, ith, ip1);
-  const double2 f010 = shell_src<SRC>(g, m, u, ir, ith + 1, iph), f011 = shell_src<SRC>(g, m, u, ir, ith + 1, ip1);
-  const double2 f100 = shell_src<SRC>(g, m, u, ir + 1, ith, iph), f101 = shell_src<SRC>(g, m, u, ir + 1, ith, ip1);
-  const double2 f110 = shell_src<SRC>(g, m, u, ir + 1, ith + 1, iph),
-                f111 = shell_src<SRC>(g, m, u, ir + 1, ith + 1, ip1);
-  const double2 f00 = cadd(rmul(1.0 - wp, f000), rmul(wp, f001));
-  const double2 f01 = cadd(rmul(1.0 - wp, f010), rmul(wp, f011));
-  const double2 f10 = cadd(rmul(1.0 - wp, f100), rmul(wp, f101));
-  const double2 f11 = cadd(rmul(1.0 - wp, f110), rmul(wp, f111));
-  const double2 f0 = cadd(rmul(1.0 - wt, f00), rmul(wt, f01));
-  const double2 f1 = cadd(rmul(1.0 - wt, f10), rmul(wt, f11));
-  *o = cadd(rmul(1.0 - wr, f0), rmul(wr, f1));
+  double2 c[8][NF];  // corners, bits: r, theta, phi
+#pragma unroll
+  for (int q = 0; q < 8; ++q) src(ir + (q >> 2), ith + ((q >> 1) & 1), iph + (q & 1), c[q]);
+#pragma unroll
+  for (int v = 0; v < NF; ++v) {
+    const double2 f00 = cadd(rmul(1.0 - wp, c[0][v]), rmul(wp, c[1][v]));
+    const double2 f01 = cadd(rmul(1.0 - wp, c[2][v]), rmul(wp, c[3][v]));
+    const double2 f10 = cadd(rmul(1.0 - wp, c[4][v]), rmul(wp, c[5][v]));
+    const double2 f11 = cadd(rmul(1.0 - wp, c[6][v]), rmul(wp, c[7][v]));
+    const double2 f0 = cadd(rmul(1.0 - wt, f00), rmul(wt, f01));
+    const double2 f1 = cadd(rmul(1.0 - wt, f10), rmul(wt, f11));
+    o[(long long)(F0 + v) * Ny * Nz] = cadd(rmul(1.0 - wr, f0), rmul(wr, f1));
+  }
 }
 
 void launch_shell_interp(const Grid& g, const Metric& m, const double2* u, const ShellInterp& si, int n_det, int Ny,
                          int Nz, int which_mask, double2* out, cudaStream_t st) {
-  dim3 gr((Ny * Nz + 255) / 256, n_det);
-  if (which_mask & 1) shell_interp_kernel<0><<<gr, 256, 0, st>>>(g, m, u, si, Ny, Nz, out);
-  if (which_mask & 2) shell_interp_kernel<1><<<gr, 256, 0, st>>>(g, m, u, si, Ny, Nz, out);
-  if (which_mask & 4) shell_interp_kernel<2><<<gr, 256, 0, st>>>(g, m, u, si, Ny, Nz, out);
-  if (which_mask & 8) shell_interp_kernel<3><<<gr, 256, 0, st>>>(g, m, u, si, Ny, Nz, out);
+  const int nt = 64;  // a vertex sphere of a small grid still spreads over the SMs
+  dim3 gr((Ny * Nz + nt - 1) / nt, n_det);
+  if (which_mask == 1) shell_interp_kernel<1><<<gr, nt, 0, st>>>(g, m, u, si, Ny, Nz, out);
+  else if (which_mask == 14) shell_interp_kernel<14><<<gr, nt, 0, st>>>(g, m, u, si, Ny, Nz, out);
+  else shell_interp_kernel<15><<<gr, nt, 0, st>>>(g, m, u, si, Ny, Nz, out);
 }
 
 // trapezium_2D_complex selector weight (tools/integral.f90:330-362)
@@ -206,10 +250,8 @@ __device__ __forceinline__ double trap_w(int jv, int kv, int Ny, int Nz) {
 }
 
 // momentum(c, d) = Re trapezium_2D(shell of j_c sqrtg): one block per (c, d)
-__global__ void flux_kernel(const double2* __restrict__ shells, const int* active, int Ny, int Nz, double dydz,
-                            double* out) {
-  const int c = blockIdx.x, d = blockIdx.y;
-  if (!active[d]) return;
+__device__ __forceinline__ void flux_block(const double2* shells, int c, int d, int Ny, int Nz, double dydz,
+                                           double* out) {
   const double2* f = shells + ((long long)d * 4 + 1 + c) * Ny * Nz;
   double2 acc = c2(0.0, 0.0);
   for (int t = threadIdx.x; t < Ny * Nz; t += blockDim.x) {
@@ -220,21 +262,31 @@ __global__ void flux_kernel(const double2* __restrict__ shells, const int* activ
   if (threadIdx.x == 0) out[c + 3 * d] = dydz * acc.x;
 }
 
-void launch_flux(const double2* shells, const int* active, int n_det, int Ny, int Nz, double dydz, double* out,
-                 cudaStream_t st) {
-  flux_kernel<<<dim3(3, n_det), 256, 0, st>>>(shells, active, Ny, Nz, dydz, out);
-}
-
 // project_sh (tools/FFT_sph.f90:247-279): a_lm = dy dz sum_jk w_jk f conj(Y_lm) sin(theta_j).
 // Y_lm = (norm P_lm)(theta_j) (cos m phi_k, sin m phi_k); Y_l,-m = (-1)^m conj(Y_lm).
-// One block per (l, m, detector).
-__global__ void project_kernel(const double2* __restrict__ shells, const int* active, int L, int Ny, int Nz,
-                               const double* __restrict__ normP, const double* __restrict__ cosm,
-                               const double* __restrict__ sinm, const double* __restrict__ sint, double dydz,
-                               double2* alm) {
-  const int l = blockIdx.x, mi = blockIdx.y, d = blockIdx.z;
-  const int m = mi - L;
-  if (!active[d] || (m < -l) || (m > l)) return;
+// One block per (l, m, detector), m on either side of zero in turn of l: the
+// (L + 1)^2 pairs with |m| <= l, none of them empty; then, when `out` is given,
+// three blocks per detector for the fluxes, which read the same shells.
+__global__ void shell_reduce_kernel(const double2* __restrict__ shells, const int* active, int L, int Ny, int Nz,
+                                    const double* __restrict__ normP, const double* __restrict__ cosm,
+                                    const double* __restrict__ sinm, const double* __restrict__ sint, double dydz,
+                                    double2* alm, double* out) {
+  const int d = blockIdx.y;
+  if (!active[d]) return;
+  int b = blockIdx.x;
+  if (alm) {
+    if (b >= (L + 1) * (L + 1)) {
+      flux_block(shells, b - (L + 1) * (L + 1), d, Ny, Nz, dydz, out);
+      return;
+    }
+  } else {
+    flux_block(shells, b, d, Ny, Nz, dydz, out);
+    return;
+  }
+  int l = (int)sqrtf((float)b);
+  while (l * l > b) --l;
+  while ((l + 1) * (l + 1) <= b) ++l;
+  const int m = b - l * l - l, mi = m + L;
   const int am = m < 0 ? -m : m;
   const double sgn = (am & 1) ? -1.0 : 1.0;
   const double* P = normP + ((long long)l * (L + 1) + am) * Ny;
@@ -258,11 +310,12 @@ __global__ void project_kernel(const double2* __restrict__ shells, const int* ac
   if (threadIdx.x == 0) alm[(long long)l + (L + 1) * ((long long)mi + (2 * L + 1) * d)] = rmul(dydz, acc);
 }
 
-void launch_project(const double2* shells, const int* active, int n_det, int L, int Ny, int Nz, const double* normP,
-                    const double* cosm, const double* sinm, const double* sint, double dydz, double2* alm,
-                    cudaStream_t st) {
-  project_kernel<<<dim3(L + 1, 2 * L + 1, n_det), 256, 0, st>>>(shells, active, L, Ny, Nz, normP, cosm, sinm, sint,
-                                                                 dydz, alm);
+void launch_shell_reduce(const double2* shells, const int* active, int n_det, int L, int Ny, int Nz,
+                         const double* normP, const double* cosm, const double* sinm, const double* sint, double dydz,
+                         double2* alm, double* flux, cudaStream_t st) {
+  const int nb = (alm ? (L + 1) * (L + 1) : 0) + (flux ? 3 : 0);
+  shell_reduce_kernel<<<dim3(nb, n_det), 256, 0, st>>>(shells, active, L, Ny, Nz, normP, cosm, sinm, sint, dydz, alm,
+                                                       flux);
 }
 
 }  // namespace kg

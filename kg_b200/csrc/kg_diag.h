@@ -22,13 +22,13 @@ struct ShellInterp {
   const double* w_ph;  // [Nz]
 };
 
+// which_mask: 1 (phi), 14 (the three currents) or 15 (both)
 void launch_shell_interp(const Grid& g, const Metric& m, const double2* u, const ShellInterp& si, int n_det, int Ny,
                          int Nz, int which_mask, double2* out, cudaStream_t st);
-void launch_flux(const double2* shells, const int* active, int n_det, int Ny, int Nz, double dydz, double* out,
-                 cudaStream_t st);
-void launch_project(const double2* shells, const int* active, int n_det, int L, int Ny, int Nz, const double* normP,
-                    const double* cosm, const double* sinm, const double* sint, double dydz, double2* alm,
-                    cudaStream_t st);
+// the shells' a_lm (alm) and fluxes (flux); either may be null
+void launch_shell_reduce(const double2* shells, const int* active, int n_det, int L, int Ny, int Nz,
+                         const double* normP, const double* cosm, const double* sinm, const double* sint, double dydz,
+                         double2* alm, double* flux, cudaStream_t st);
 
 // all-shell Y_lm projection (kg_ylm_gemm.cu)
 }  // namespace kg
