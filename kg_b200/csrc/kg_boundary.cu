@@ -136,7 +136,7 @@ __device__ __forceinline__ void ghost_unit(const Grid& g, T* u, const double2* u
 }
 
 // threads of a block: a row of a small grid in one pass, 256 for longer rows
-static int ghost_threads(int ni) { return ni >= 256 ? 256 : (ni + 31) / 32 * 32; }
+static int row_threads(int ni) { return ni >= 256 ? 256 : (ni + 31) / 32 * 32; }
 
 template <class T>
 __global__ void ghost_kernel(Grid g, T* u, const double2* up, int inflow, int unit0) {
@@ -145,7 +145,7 @@ __global__ void ghost_kernel(Grid g, T* u, const double2* up, int inflow, int un
 }
 
 void launch_ghost_fill(const Grid& g, double2* u, const double2* up, int inflow, cudaStream_t st, bool faces_apart) {
-  const int nt = ghost_threads(g.NI), n = ghost_units(g, nt), rows = 2 * g.NJ + 6 * (g.Nz - 1);
+  const int nt = row_threads(g.NI), n = ghost_units(g, nt), rows = 2 * g.NJ + 6 * (g.Nz - 1);
   if (!faces_apart) {
     launch_pdl(ghost_kernel<double2>, n, nt, 0, st, g, u, up, inflow, 0);
     return;
@@ -155,7 +155,7 @@ void launch_ghost_fill(const Grid& g, double2* u, const double2* up, int inflow,
 }
 
 void launch_ghost_fill_f32(const Grid& g, float2* u, const double2* up, int inflow, cudaStream_t st) {
-  const int nt = ghost_threads(g.NI);
+  const int nt = row_threads(g.NI);
   launch_pdl(ghost_kernel<float2>, ghost_units(g, nt), nt, 0, st, g, u, up, inflow, 0);
 }
 
@@ -213,43 +213,52 @@ void launch_face(const Grid& g, double2* u, const double2* up, int inflow, int f
 }
 
 // ---- layout conversion -------------------------------------------------------
-// aos: complex u(5, NI, NJ, planes k0..k1-1) (Fortran order, variable fastest)
-__global__ void aos_to_soa_kernel(Grid g, const double2* __restrict__ aos, double2* __restrict__ soa, int k0,
-                                  int k1) {
-  const long long n = (long long)g.NI * g.NJ * (k1 - k0);
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int ii = (int)(t % g.NI);
-  const long long r = t / g.NI;
-  const int jj = (int)(r % g.NJ), k = k0 + (int)(r / g.NJ);
-  const long long o = off3(g, ii, jj, k);
+// aos: complex u(5, NI, NJ, planes k0..k1-1) (Fortran order, variable fastest);
+// soa: variables 0..3 of a state, pi: its Pi variable (the PIRK stage arrays keep
+// it in a slot of its own).  A block works on one (theta row, plane), so the index
+// division is its own and not each thread's; consecutive threads touch
+// consecutive 80-byte records.
+__global__ void aos_to_soa_kernel(Grid g, const double2* __restrict__ aos, double2* __restrict__ soa,
+                                  double2* __restrict__ pi, int k0) {
+  const int ii = blockIdx.y * blockDim.x + threadIdx.x;
+  if (ii >= g.NI) return;
+  const int jj = blockIdx.x % g.NJ, kk = blockIdx.x / g.NJ;
+  const double2* a = aos + 5 * (((long long)kk * g.NJ + jj) * g.NI + ii);
+  const long long o = off3(g, ii, jj, k0 + kk);
+  double2 v[5];
 #pragma unroll
-  for (int v = 0; v < 5; ++v) soa[v * g.fs + o] = aos[5 * t + v];
-}
-
-__global__ void soa_to_aos_kernel(Grid g, const double2* __restrict__ soa, double2* __restrict__ aos, int k0,
-                                  int k1) {
-  const long long n = (long long)g.NI * g.NJ * (k1 - k0);
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int ii = (int)(t % g.NI);
-  const long long r = t / g.NI;
-  const int jj = (int)(r % g.NJ), k = k0 + (int)(r / g.NJ);
-  const long long o = off3(g, ii, jj, k);
+  for (int w = 0; w < 5; ++w) v[w] = a[w];
 #pragma unroll
-  for (int v = 0; v < 5; ++v) aos[5 * t + v] = soa[v * g.fs + o];
+  for (int w = 0; w < 4; ++w) soa[w * g.fs + o] = v[w];
+  pi[o] = v[4];
 }
 
-void launch_aos_to_soa(const Grid& g, const double2* aos, double2* soa, int k0, int k1, cudaStream_t st) {
-  const long long n = (long long)g.NI * g.NJ * (k1 - k0);
-  if (n <= 0) return;
-  aos_to_soa_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, aos, soa, k0, k1);
+__global__ void soa_to_aos_kernel(Grid g, const double2* __restrict__ soa, const double2* __restrict__ pi,
+                                  double2* __restrict__ aos, int k0) {
+  const int ii = blockIdx.y * blockDim.x + threadIdx.x;
+  if (ii >= g.NI) return;
+  const int jj = blockIdx.x % g.NJ, kk = blockIdx.x / g.NJ;
+  double2* a = aos + 5 * (((long long)kk * g.NJ + jj) * g.NI + ii);
+  const long long o = off3(g, ii, jj, k0 + kk);
+  double2 v[5];
+#pragma unroll
+  for (int w = 0; w < 4; ++w) v[w] = soa[w * g.fs + o];
+  v[4] = pi[o];
+#pragma unroll
+  for (int w = 0; w < 5; ++w) a[w] = v[w];
 }
 
-void launch_soa_to_aos(const Grid& g, const double2* soa, double2* aos, int k0, int k1, cudaStream_t st) {
-  const long long n = (long long)g.NI * g.NJ * (k1 - k0);
-  if (n <= 0) return;
-  soa_to_aos_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, soa, aos, k0, k1);
+void launch_aos_to_soa(const Grid& g, const double2* aos, double2* soa, double2* pi, int k0, int k1, cudaStream_t st) {
+  const int nt = row_threads(g.NI);
+  if (k1 > k0)
+    aos_to_soa_kernel<<<dim3(g.NJ * (k1 - k0), (g.NI + nt - 1) / nt), nt, 0, st>>>(g, aos, soa, pi, k0);
+}
+
+void launch_soa_to_aos(const Grid& g, const double2* soa, const double2* pi, double2* aos, int k0, int k1,
+                       cudaStream_t st) {
+  const int nt = row_threads(g.NI);
+  if (k1 > k0)
+    soa_to_aos_kernel<<<dim3(g.NJ * (k1 - k0), (g.NI + nt - 1) / nt), nt, 0, st>>>(g, soa, pi, aos, k0);
 }
 
 }  // namespace kg

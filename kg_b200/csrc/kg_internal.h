@@ -185,8 +185,10 @@ void launch_face(const Grid& g, double2* u, const double2* up, int inflow, int f
 
 // layout conversion between the Fortran AoS layout and the device planes,
 // for planes [k0, k1) of all 5 variables; aos points at plane k0
-void launch_aos_to_soa(const Grid& g, const double2* aos, double2* soa, int k0, int k1, cudaStream_t st);
-void launch_soa_to_aos(const Grid& g, const double2* soa, double2* aos, int k0, int k1, cudaStream_t st);
+// (pi: where the Pi variable lives, soa + 4 g.fs in a plain state)
+void launch_aos_to_soa(const Grid& g, const double2* aos, double2* soa, double2* pi, int k0, int k1, cudaStream_t st);
+void launch_soa_to_aos(const Grid& g, const double2* soa, const double2* pi, double2* aos, int k0, int k1,
+                       cudaStream_t st);
 
 // diagnostics
 struct ShellInterp;  // per-detector interpolation tables (kg_diag.cu)
