@@ -101,14 +101,15 @@ __host__ __device__ __forceinline__ int ghost_units(const Grid& g, int threads) 
 }
 
 template <class T>
-__device__ __forceinline__ void ghost_unit(const Grid& g, T* u, const double2* up, int inflow, int unit) {
+__device__ __forceinline__ void ghost_unit(const Grid& g, T* u, const double2* up, int inflow, int unit,
+                                           int cyclic = 0) {
   const int nC = 2 * g.NJ, nA = 6 * (g.Nz - 1);
   if (unit < nC) {  // row jj of plane 0 or Nz
     const int jj = unit % g.NJ;
     const bool last = unit >= g.NJ;
     const int ks = last ? 1 : g.Nz - 1;
     const bool ghost = jj < 3 || jj >= g.NJ - 3;
-    if (!last && !ghost) {
+    if (!last && !ghost && !cyclic) {
       const int kp = g.Nzm1 - g.dis;
       const bool north = jj <= 5, south = jj >= g.NJ - 6;
       if (north) ghost_row(g, u, up, inflow, 5 - jj, kp, jj, 0);
@@ -119,8 +120,11 @@ __device__ __forceinline__ void ghost_unit(const Grid& g, T* u, const double2* u
   } else if (unit < nC + nA) {  // ghost row of an inner plane
     const int q = unit - nC;
     const int r = q % 6, k = 1 + q / 6;
-    const int kt = ktarget(g, k);
-    if (kt == 0) return;  // with plane 0's own rows
+    int kt = ktarget(g, k);
+    if (kt == 0) {
+      if (!cyclic) return;  // with plane 0's own rows
+      kt = g.Nzm1;          // plane 0 was not computed: it equals plane Nz - 1
+    }
     const int jj = (r < 3) ? r : (g.NJ - 6 + r);
     ghost_row(g, u, up, inflow, jj, k, ghost_src_row(g, jj), kt);
   } else {  // x-face points
@@ -139,24 +143,25 @@ __device__ __forceinline__ void ghost_unit(const Grid& g, T* u, const double2* u
 static int row_threads(int ni) { return ni >= 256 ? 256 : (ni + 31) / 32 * 32; }
 
 template <class T>
-__global__ void ghost_kernel(Grid g, T* u, const double2* up, int inflow, int unit0) {
+__global__ void ghost_kernel(Grid g, T* u, const double2* up, int inflow, int unit0, int cyclic) {
   pdl_wait();
-  ghost_unit(g, u, up, inflow, unit0 + blockIdx.x);
+  ghost_unit(g, u, up, inflow, unit0 + blockIdx.x, cyclic);
 }
 
-void launch_ghost_fill(const Grid& g, double2* u, const double2* up, int inflow, cudaStream_t st, bool faces_apart) {
+void launch_ghost_fill(const Grid& g, double2* u, const double2* up, int inflow, cudaStream_t st, bool faces_apart,
+                       bool cyclic) {
   const int nt = row_threads(g.NI), n = ghost_units(g, nt), rows = 2 * g.NJ + 6 * (g.Nz - 1);
   if (!faces_apart) {
-    launch_pdl(ghost_kernel<double2>, n, nt, 0, st, g, u, up, inflow, 0);
+    launch_pdl(ghost_kernel<double2>, n, nt, 0, st, g, u, up, inflow, 0, (int)cyclic);
     return;
   }
-  launch_pdl(ghost_kernel<double2>, rows, nt, 0, st, g, u, up, inflow, 0);
-  launch_pdl(ghost_kernel<double2>, n - rows, nt, 0, st, g, u, up, inflow, rows);
+  launch_pdl(ghost_kernel<double2>, rows, nt, 0, st, g, u, up, inflow, 0, (int)cyclic);
+  launch_pdl(ghost_kernel<double2>, n - rows, nt, 0, st, g, u, up, inflow, rows, (int)cyclic);
 }
 
 void launch_ghost_fill_f32(const Grid& g, float2* u, const double2* up, int inflow, cudaStream_t st) {
   const int nt = row_threads(g.NI);
-  launch_pdl(ghost_kernel<float2>, ghost_units(g, nt), nt, 0, st, g, u, up, inflow, 0);
+  launch_pdl(ghost_kernel<float2>, ghost_units(g, nt), nt, 0, st, g, u, up, inflow, 0, 0);
 }
 
 // ---- many solves at once (batched engine): one block row per solve -----------

@@ -55,7 +55,14 @@ struct kg_solver {
   double2* U = nullptr;                  // u (5 variables)
   double2* S = nullptr;                  // u_stage (6 slots; slot 4/5 alternate for Pi)
   double2* T = nullptr;                  // u_stage_2 (6 slots)
-  double2* RK = nullptr;                 // RK stage buffers R1, R2 and accumulator (15 slots)
+  // RK stage buffers R1, R2 and accumulator, 5 slots each: blocks of u's size, so
+  // that a solve created after another has gone takes over its blocks one for one
+  double2* RK[3] = {nullptr, nullptr, nullptr};
+  double2* pole = nullptr;               // first-stage rows next to the poles (kg_pair.cu)
+  // u as a ghost fill leaves it: plane 0 = plane Nz-1 and plane Nz = plane 1 in
+  // every row, which the paired stages take for granted.  Cleared by whatever
+  // writes u otherwise.
+  bool seam_filled = false;
   double2* UP = nullptr;                 // u_p for the boundary hook
   double2* HV = nullptr;                 // rhs hook input / output (10 slots)
   double2* stage_buf = nullptr;          // Fortran-layout staging buffer
@@ -67,6 +74,7 @@ struct kg_solver {
   int variant = 3;                       // 0: per-point, 1: 2.5-D marching, 2, 3: TMA-pipelined marching
                                          // (3: PIRK stage 1 fused in one kernel; 2: two launches)
   int tile_rows = 8;                     // theta rows of the TMA tiles of the RK4 stages (8 or 4)
+  int rk4_pairs = 1;                     // RK4 stages in pairs: 0 never, 1 where it pays, 2 always
   int* derr = nullptr;                   // device flag: a bounded wait in a kernel ran out
   // CUDA graphs of two consecutive steps per stepper and Pi-slot state
   int use_graphs = 1;
@@ -203,13 +211,14 @@ double2* fld(double2* base, const Grid& g, int v) { return base + (long long)v *
 // kernel kinds reported by kg_profile_read: the 13 stage kinds, then these
 enum { PK_GHOST = 13, PK_FACE, PK_RHS, PK_CONVERT, PK_DENSITY, PK_MASS, PK_SHELL, PK_FLUX, PK_PROJECT,
        PK_YLM_PREP, PK_YLM_GEMM, PK_YLM_FP64, PK_RADIAL, PK_MX1, PK_MX2, PK_MX3, PK_MX4, PK_GHOST_F32, PK_PROLONG,
-       PK_RESTRICT, PK_S1_FUSED, PK_COUNT };
+       PK_RESTRICT, PK_S1_FUSED, PK_PAIR12, PK_PAIR34, PK_POLE, PK_COUNT };
 const char* const kPkNames[PK_COUNT] = {
     "stage_pirk_s1_psi", "stage_pirk_s1_pi", "stage_pirk2_s2", "stage_pirk3_s2_psi", "stage_pirk3_s2_pi",
     "stage_pirk3_s3", "stage_rk3_1", "stage_rk3_2", "stage_rk3_3", "stage_rk4_1", "stage_rk4_2", "stage_rk4_3",
     "stage_rk4_4", "ghost_fill", "boundary_face", "rhs", "layout_convert", "density", "mass_reduce",
     "shell_interp", "flux_reduce", "ylm_project", "ylm_all_prepare", "ylm_all_gemm_bf16x3", "ylm_all_fp64", "radial_ft", "mixed_rk4_1",
-    "mixed_rk4_2", "mixed_rk4_3", "mixed_rk4_4", "ghost_fill_f32", "bo_prolong", "bo_restrict", "stage_pirk_s1_fused"};
+    "mixed_rk4_2", "mixed_rk4_3", "mixed_rk4_4", "ghost_fill_f32", "bo_prolong", "bo_restrict", "stage_pirk_s1_fused",
+    "stage_rk4_12", "stage_rk4_34", "pole_rows"};
 
 cudaEvent_t take_event(kg_solver* h) {
   if (!h->pool.empty()) {
@@ -615,6 +624,13 @@ int ensure(kg_solver* h, double2** buf, int nslots) {
   return dalloc(h, (void**)buf, (size_t)nslots * field_bytes(h));
 }
 
+// the first n RK buffers
+int ensure_rk(kg_solver* h, int n) {
+  int rc = KG_OK;
+  for (int i = 0; i < n && rc == KG_OK; ++i) rc = ensure(h, &h->RK[i], 5);
+  return rc;
+}
+
 int ensure_staging(kg_solver* h) {
   if (h->stage_buf) return KG_OK;
   const size_t plane_bytes = (size_t)5 * h->NI * h->NJ * sizeof(double2);
@@ -741,9 +757,11 @@ int check_device_flag(kg_solver* h) {
 }
 // faces_apart: two launches instead of one; a PIRK2 step is four launches, a
 // count that kg_launch_count reports and its callers rely on
-void run_ghost(kg_solver* h, double2* u, const double2* up, int inflow, bool faces_apart = false) {
+void run_ghost(kg_solver* h, double2* u, const double2* up, int inflow, bool faces_apart = false,
+               bool cyclic = false) {
   Prof pf(h, PK_GHOST, faces_apart ? 2 : 1);
-  kg::launch_ghost_fill(h->g, u, up, inflow, h->stream, faces_apart);
+  kg::launch_ghost_fill(h->g, u, up, inflow, h->stream, faces_apart, cyclic);
+  if (u == h->U) h->seam_filled = true;
 }
 
 // a_lm and fluxes of the detector shells
@@ -855,7 +873,7 @@ int kg_create(const kg_params* p, int device, kg_solver** out) {
 int kg_destroy(kg_solver* h) {
   if (!h) return KG_EINVAL;
   if (h->stream) cudaStreamSynchronize(h->stream);
-  void* bufs[] = {h->dmet, h->U, h->S, h->T, h->RK, h->UP, h->HV, h->stage_buf, h->rho, h->partials,
+  void* bufs[] = {h->dmet, h->U, h->S, h->T, h->RK[0], h->RK[1], h->RK[2], h->pole, h->UP, h->HV, h->stage_buf, h->rho, h->partials,
                   h->d_int, h->d_dbl, h->shells, h->alm, h->flux, h->derr, h->ylm_tab, h->ylm_buf,
                   h->rad_jr, h->rad_ft, h->MX};
   for (void* b : bufs) dfree(h, b);
@@ -909,6 +927,7 @@ int kg_set_state(kg_solver* h, int which, const double* host_u) {
   View V;
   int rc;
   if ((rc = state_view(h, which, &V))) return rc;
+  if (which == 0) h->seam_filled = false;
   if ((rc = load_view(h, V, host_u, cudaMemcpyHostToDevice))) return rc;
   KG_CK(cudaStreamSynchronize(h->stream));
   return KG_OK;
@@ -929,6 +948,7 @@ int kg_set_state_device(kg_solver* h, int which, const double* dev_u) {
   View V;
   int rc;
   if ((rc = state_view(h, which, &V))) return rc;
+  if (which == 0) h->seam_filled = false;
   return load_view(h, V, dev_u, cudaMemcpyDeviceToDevice);
 }
 
@@ -999,11 +1019,11 @@ int step_pirk3(kg_solver* h, int nsteps) {
 
 int step_rk3(kg_solver* h, int nsteps) {
   int rc;
-  if ((rc = ensure(h, &h->RK, 15))) return rc;
+  if ((rc = ensure_rk(h, 2))) return rc;
   const Grid& g = h->g;
   const int inflow = h->p.bc_rmax == KG_INFLOW;
-  double2* R1 = h->RK;
-  double2* R2 = fld(h->RK, g, 5);
+  double2* R1 = h->RK[0];
+  double2* R2 = h->RK[1];
   for (int s = 0; s < nsteps; ++s) {
     kg::StageLaunch L = base_launch(h);
     L.base = h->U;
@@ -1026,36 +1046,97 @@ int step_rk3(kg_solver* h, int nsteps) {
   return KG_OK;
 }
 
-int step_rk4(kg_solver* h, int nsteps) {
-  int rc;
-  if ((rc = ensure(h, &h->RK, 15))) return rc;
+// one RK4 step of four stage kernels, u -> u
+void rk4_step_single(kg_solver* h) {
   const Grid& g = h->g;
   const int inflow = h->p.bc_rmax == KG_INFLOW;
-  double2* R1 = h->RK;
-  double2* R2 = fld(h->RK, g, 5);
-  double2* A = fld(h->RK, g, 10);
-  for (int s = 0; s < nsteps; ++s) {
-    kg::StageLaunch L = base_launch(h);
-    L.base = h->U;
-    L.acc = A;
-    set_in(L, g, h->U, fld(h->U, g, 4));
-    L.out = R1;
-    run_stage(h, kg::ST_RK4_1, L);
-    run_ghost(h, R1, h->U, inflow);
-    set_in(L, g, R1, fld(R1, g, 4));
-    L.out = R2;
-    run_stage(h, kg::ST_RK4_2, L);
-    run_ghost(h, R2, h->U, inflow);
-    set_in(L, g, R2, fld(R2, g, 4));
-    L.out = R1;
-    run_stage(h, kg::ST_RK4_3, L);
-    run_ghost(h, R1, h->U, inflow);
-    set_in(L, g, R1, fld(R1, g, 4));
-    L.out = h->U;
-    L.skip_last_i = inflow;
-    run_stage(h, kg::ST_RK4_4, L);
-    run_ghost(h, h->U, h->U, inflow);
-    h->t = h->t + h->dt;
+  double2* R1 = h->RK[0];
+  double2* R2 = h->RK[1];
+  double2* A = h->RK[2];
+  kg::StageLaunch L = base_launch(h);
+  L.base = h->U;
+  L.acc = A;
+  set_in(L, g, h->U, fld(h->U, g, 4));
+  L.out = R1;
+  run_stage(h, kg::ST_RK4_1, L);
+  run_ghost(h, R1, h->U, inflow);
+  set_in(L, g, R1, fld(R1, g, 4));
+  L.out = R2;
+  run_stage(h, kg::ST_RK4_2, L);
+  run_ghost(h, R2, h->U, inflow);
+  set_in(L, g, R2, fld(R2, g, 4));
+  L.out = R1;
+  run_stage(h, kg::ST_RK4_3, L);
+  run_ghost(h, R1, h->U, inflow);
+  set_in(L, g, R1, fld(R1, g, 4));
+  L.out = h->U;
+  L.skip_last_i = inflow;
+  run_stage(h, kg::ST_RK4_4, L);
+  run_ghost(h, h->U, h->U, inflow);
+  h->t = h->t + h->dt;
+}
+
+// one RK4 step of two paired kernels (kg_pair.cu), u in `from` -> u in `to`; the
+// other of the two buffers is the first stage buffer R1, which pairs do not use
+int rk4_step_pairs(kg_solver* h, double2* from, double2* to) {
+  const Grid& g = h->g;
+  const int inflow = h->p.bc_rmax == KG_INFLOW;
+  const double* rsg = h->dmet + (size_t)T_RSG * h->NJ * h->PI;
+  double2* R2 = h->RK[1];
+  double2* A = h->RK[2];
+  kg::PairLaunch L;
+  memset(&L, 0, sizeof(L));
+  L.g = g;
+  L.m = metric_of(h);
+  L.metric_kind = h->p.metric == KG_SCHW_EF ? kg::MK_SCHW : kg::MK_KS;
+  L.base = from;
+  L.acc_in = L.acc_out = A;
+  L.pole = h->pole;
+  L.inflow = inflow;
+  for (int pair = 0; pair < 2; ++pair) {
+    L.X = pair ? R2 : from;
+    L.out = pair ? to : R2;
+    {
+      Prof pf(h, PK_POLE, 1);
+      kg::launch_pole_rows(pair, L, rsg, h->pole, h->stream);
+    }
+    {
+      Prof pf(h, pair ? PK_PAIR34 : PK_PAIR12, 1);
+      if (kg::launch_rk4_pair(pair, L, rsg, h->derr, h->stream))
+        return set_err(h, KG_ECUDA, "paired RK4 stages could not be configured (tensor maps)");
+    }
+    run_ghost(h, L.out, from, inflow, false, true);
+  }
+  h->t = h->t + h->dt;
+  return KG_OK;
+}
+
+// the paired form (kg_pair.cu): with the TMA stage forms, where it pays
+bool wants_pairs(const kg_solver* h) {
+  return h->variant >= 2 && (h->rk4_pairs == 2 || (h->rk4_pairs == 1 && kg::rk4_pairs_pay(h->g)));
+}
+
+int step_rk4(kg_solver* h, int nsteps) {
+  int rc;
+  if ((rc = ensure_rk(h, 3))) return rc;
+  // without room for the pole rows the four stage kernels run instead
+  const bool pairs = wants_pairs(h);
+  if (pairs && !h->pole) (void)dalloc(h, (void**)&h->pole, (size_t)10 * h->NK * h->PI * sizeof(double2));
+  for (int s = 0; s < nsteps;) {
+    if (!pairs || !h->pole || !h->seam_filled) {
+      rk4_step_single(h);
+      ++s;
+      continue;
+    }
+    // two steps, u -> R1 -> u; a last odd one is copied back
+    if ((rc = rk4_step_pairs(h, h->U, h->RK[0]))) return rc;
+    ++s;
+    if (s < nsteps) {
+      if ((rc = rk4_step_pairs(h, h->RK[0], h->U))) return rc;
+      ++s;
+    } else {
+      KG_CK(cudaMemcpyAsync(h->U, h->RK[0], 5 * field_bytes(h), cudaMemcpyDeviceToDevice, h->stream));
+    }
   }
   KG_CK(cudaGetLastError());
   return KG_OK;
@@ -1128,15 +1209,16 @@ int step_rk4_mixed(kg_solver* h, int nsteps) {
 // dissipation, Sommerfeld outer plane; kg_config.cu)
 int step_rk4_cfg(kg_solver* h, int nsteps) {
   int rc;
-  if ((rc = ensure(h, &h->RK, 15))) return rc;
+  if ((rc = ensure_rk(h, 3))) return rc;
   const Grid& g = h->g;
-  double2* R1 = h->RK;
-  double2* R2 = fld(h->RK, g, 5);
-  double2* A = fld(h->RK, g, 10);
+  double2* R1 = h->RK[0];
+  double2* R2 = h->RK[1];
+  double2* A = h->RK[2];
   const double* dxb4 = h->dmet + (size_t)T_DXBETA4 * h->NJ * h->PI;
   const double coef[6] = {1.0 / (12.0 * h->dx), 1.0 / (12.0 * h->dy), 1.0 / (12.0 * h->dz),
                           h->ko_eps / (64.0 * h->dx), h->ko_eps / (64.0 * h->dy), h->ko_eps / (64.0 * h->dz)};
   const double rN = h->x1d[h->NI - 1];
+  h->seam_filled = false;
   static const int kinds[4] = {kg::ST_RK4_1, kg::ST_RK4_2, kg::ST_RK4_3, kg::ST_RK4_4};
   for (int s = 0; s < nsteps; ++s) {
     kg::StageLaunch L = base_launch(h);
@@ -1168,13 +1250,14 @@ int step_rk4_cfg(kg_solver* h, int nsteps) {
 // [t_coarse, t_coarse + dt_coarse]; a0 at this step's start, da its length).
 int step_rk4_bo(kg_solver* h, kg_solver* c, const double2* c_old, double a0, double da, int nbuf) {
   int rc;
-  if ((rc = ensure(h, &h->RK, 15))) return rc;
+  if ((rc = ensure_rk(h, 3))) return rc;
   const Grid& g = h->g;
   const int inflow = h->p.bc_rmax == KG_INFLOW;
-  double2* R1 = h->RK;
-  double2* R2 = fld(h->RK, g, 5);
-  double2* A = fld(h->RK, g, 10);
+  double2* R1 = h->RK[0];
+  double2* R2 = h->RK[1];
+  double2* A = h->RK[2];
   auto prolong = [&](double2* u, double alpha) -> int {
+    h->seam_filled = false;
     Prof pf(h, PK_PROLONG, 1);
     if (kg::launch_prolong(g, u, c->g, c_old, c->U, alpha, nbuf, h->stream))
       return set_err(h, KG_EINVAL, "refined level does not fit inside its coarser level");
@@ -1207,12 +1290,13 @@ int step_rk4_bo(kg_solver* h, kg_solver* c, const double2* c_old, double a0, dou
 // coarse values interpolated to those times.
 int step_rk3_bo(kg_solver* h, kg_solver* c, const double2* c_old, double a0, double da, int nbuf) {
   int rc;
-  if ((rc = ensure(h, &h->RK, 15))) return rc;
+  if ((rc = ensure_rk(h, 2))) return rc;
   const Grid& g = h->g;
   const int inflow = h->p.bc_rmax == KG_INFLOW;
-  double2* R1 = h->RK;
-  double2* R2 = fld(h->RK, g, 5);
+  double2* R1 = h->RK[0];
+  double2* R2 = h->RK[1];
   auto prolong = [&](double2* u, double alpha) -> int {
+    h->seam_filled = false;
     Prof pf(h, PK_PROLONG, 1);
     if (kg::launch_prolong(g, u, c->g, c_old, c->U, alpha, nbuf, h->stream))
       return set_err(h, KG_EINVAL, "refined level does not fit inside its coarser level");
@@ -1252,6 +1336,7 @@ int step_pirk_bo(kg_solver* h, kg_solver* c, const double2* c_old, double a0, do
   const Grid& g = h->g;
   const int inflow = h->p.bc_rmax == KG_INFLOW;
   auto prolong = [&](double2* u, double2* upi, double alpha) -> int {
+    h->seam_filled = false;
     Prof pf(h, PK_PROLONG, 1);
     if (kg::launch_prolong(g, u, c->g, c_old, c->U, alpha, nbuf, h->stream, upi))
       return set_err(h, KG_EINVAL, "refined level does not fit inside its coarser level");
@@ -1301,6 +1386,10 @@ int run_steps(kg_solver* h, int which, int nsteps, int (*step)(kg_solver*, int))
   if (!h || nsteps < 0) return KG_EINVAL;
   int rc;
   if (nsteps < 2 || !h->use_graphs || h->prof_on) return step(h, nsteps);
+  if (which == 3 && !h->seam_filled && wants_pairs(h)) {  // the graph holds the paired form
+    if ((rc = step(h, 1))) return rc;
+    if (--nsteps < 2) return nsteps ? step(h, nsteps) : KG_OK;
+  }
   int key = ((h->s_cur == 5) ? 1 : 0) + ((h->t_cur == 5) ? 2 : 0);
   if (!h->graphs[which][key].exec || h->graphs[which][key].gen != h->graph_gen) {
     // one direct step first: buffers, kernel attributes and tensor-map encoders
@@ -1382,6 +1471,7 @@ int kg_get_scheme(const kg_solver* h) { return h ? h->scheme : -1; }
 
 int kg_fill_ghosts_cfg(kg_solver* h) {
   if (!h) return KG_EINVAL;
+  h->seam_filled = false;
   kg::launch_ghost_fill_cfg(h->g, h->U, h->stream);
   KG_CK(cudaGetLastError());
   KG_CK(cudaStreamSynchronize(h->stream));
@@ -1431,6 +1521,7 @@ int kg_boundary(kg_solver* h, unsigned mask) {
   if (!h) return KG_EINVAL;
   const int inflow = h->p.bc_rmax == KG_INFLOW;
   const double2* up = h->UP ? h->UP : h->U;
+  h->seam_filled = false;
   for (int f = 0; f < 6; ++f)
     if (mask & (1u << f)) {
       Prof pf(h, PK_FACE, 1);
@@ -1958,6 +2049,15 @@ int kg_set_tile_rows(kg_solver* h, int rows) {
   return KG_OK;
 }
 
+int kg_set_rk4_pairs(kg_solver* h, int mode) {
+  if (!h || mode < 0 || mode > 2) return KG_EINVAL;
+  if (mode != h->rk4_pairs) {
+    h->rk4_pairs = mode;
+    h->graph_gen++;
+  }
+  return KG_OK;
+}
+
 int kg_get_tile_rows(const kg_solver* h) { return h ? h->tile_rows : KG_EINVAL; }
 
 int kg_profile_enable(kg_solver* h, int on) {
@@ -2124,9 +2224,9 @@ int batch_rebuild(kg_batch* b) {
         b->ghost_units = std::max(b->ghost_units, kg::ghost_batch_units(g));
         continue;
       }
-      double2* R1 = h->RK;
-      double2* R2 = fld(h->RK, g, 5);
-      double2* A = fld(h->RK, g, 10);
+      double2* R1 = h->RK[0];
+      double2* R2 = h->RK[1];
+      double2* A = h->RK[2];
       kg::StageLaunch L = base_launch(h);
       L.base = h->U;
       L.acc = A;
@@ -2235,7 +2335,7 @@ int kg_batch_add(kg_batch* b, kg_solver* h) {
   for (kg_solver* m : b->members)
     if (m == h) return KG_OK;
   int rc;
-  if ((rc = b->precision == 1 ? ensure_mixed(h) : ensure(h, &h->RK, 15))) return rc;
+  if ((rc = b->precision == 1 ? ensure_mixed(h) : ensure_rk(h, 3))) return rc;
   if (!kg::tma_available(h->g, h->U)) {
     b->err = "tensor maps unavailable for this grid";
     return KG_EINVAL;
@@ -2416,7 +2516,7 @@ int kg_batch_set_precision(kg_batch* b, int mode) {
   if (mode == b->precision) return KG_OK;
   KG_BCK(cudaStreamSynchronize(b->stream));
   for (kg_solver* h : b->members) {
-    const int rc = mode == 1 ? ensure_mixed(h) : ensure(h, &h->RK, 15);
+    const int rc = mode == 1 ? ensure_mixed(h) : ensure_rk(h, 3);
     if (rc) {
       b->err = "could not allocate stage buffers of a member: " + h->err;
       return rc;
@@ -2525,6 +2625,7 @@ int hier_step(kg_hier* H, int l, double a0, double da, int method) {
     for (int sub = 0; sub < 2; ++sub)
       if ((rc = hier_step(H, l + 1, 0.5 * sub, 0.5, method))) return rc;
     if ((rc = hier_order(H, f, h, l))) return rc;
+    h->seam_filled = false;
     Prof pf(h, PK_RESTRICT, 1);
     if (kg::launch_restrict(h->g, h->U, f->g, f->U, H->keep_out, h->stream)) {
       H->err = "restriction does not fit";

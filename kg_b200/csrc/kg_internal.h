@@ -35,14 +35,14 @@ enum StageKind {
 // at worst).  Against chunks of about 32 planes on every grid (64 in the fused PIRK stage 1),
 // us per launch: 64 x 17 x 33 PIRK2 stage 2 71 -> 12 and fused stage 1 94 -> 18,
 // 256 x 33 x 65 66 -> 37 and 103 -> 52, RK4 stage 2 98 -> 55.
-inline int phi_chunk(int planes, long long tiles, int slots, int longest) {
+inline int phi_chunk(int planes, long long tiles, int slots, int longest, int extra = 1) {
   int best = planes;
   double cost = 1e300;
   for (int n = (planes + longest - 1) / longest; n <= planes; ++n) {
     const int c = (planes + n - 1) / n;
     const int m = (planes + c - 1) / c;
     const double waves = (double)tiles * m / slots + 0.25;
-    const double t = (waves > 1.0 ? waves : 1.0) * (c + 1);
+    const double t = (waves > 1.0 ? waves : 1.0) * (c + extra);
     if (t < cost) {
       cost = t;
       best = c;
@@ -103,6 +103,26 @@ int launch_stage_tma(int kind, const StageLaunch& L, const double* rsg, int* err
 // dt rhs_pi(S(1:4), Sold).  Returns -1 if the tensor maps cannot be encoded.
 int launch_pirk_s1_fused(const Grid& g, const Metric& m, int mk, const double2* U, const double2* Sold, double2* S,
                          double2* Snew, const double* rsg, int* err, cudaStream_t st);
+// RK4 stages 1 and 2 (pair 0) or 3 and 4 (pair 1) in one kernel (kg_pair.cu); the
+// state's seam planes must hold plane 0 = plane Nz-1, plane Nz = plane 1.
+// Returns -1 if the tensor maps cannot be encoded.
+struct PairLaunch {
+  Grid g;
+  Metric m;
+  int metric_kind;
+  const double2* X;       // stencil input of the first of the two stages
+  const double2* base;    // u^n
+  const double2* acc_in;  // pair 1: k1 + 2 k2
+  double2* acc_out;       // pair 0: k1 + 2 k2
+  double2* out;           // pair 0: u + k2/2; pair 1: u^{n+1} (not u^n's buffer)
+  const double2* pole;    // launch_pole_rows' output for the same X
+  int inflow;
+};
+int launch_rk4_pair(int pair, const PairLaunch& L, const double* rsg, int* err, cudaStream_t st);
+bool rk4_pairs_pay(const Grid& g);  // whether pairs beat the four stage kernels on this grid
+// the first stage's output (after its x fill) on the first and last interior theta
+// row, [side][variable][k][PI], into `pole`: 10 NK PI complex values
+void launch_pole_rows(int pair, const PairLaunch& L, const double* rsg, double2* pole, cudaStream_t st);
 // one warp waits at most `polls` polls on an mbarrier phase that never completes,
 // then sets *err (the failure path of every bounded wait); returns -1 if the launch fails
 int launch_wait_check(int* err, long long polls, cudaStream_t st);
@@ -177,8 +197,9 @@ void launch_rhs(const Grid& g, const Metric& m, int metric_kind, const double2* 
 
 // boundary fills on a 5-variable state u; up = u_p (inflow source)
 // faces_apart: the x faces in a second launch of their own
+// cyclic: plane 0 was not computed and stands for plane Nz-1
 void launch_ghost_fill(const Grid& g, double2* u, const double2* up, int inflow, cudaStream_t st,
-                       bool faces_apart = false);
+                       bool faces_apart = false, bool cyclic = false);
 // the same on the FP32 stage states of the mixed form; up = u^n (FP64)
 void launch_ghost_fill_f32(const Grid& g, float2* u, const double2* up, int inflow, cudaStream_t st);
 void launch_face(const Grid& g, double2* u, const double2* up, int inflow, int face, cudaStream_t st);

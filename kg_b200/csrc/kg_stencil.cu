@@ -47,10 +47,11 @@ __device__ __forceinline__ void rhs_psi(const Grid& g, const Metric& M, const Va
   r[3] = op_dph(g, E, ii, jj, k);
 }
 
-// rhs_pi at one point (lines_method_lib.f90:716-753)
-template <int MK>
-__device__ __forceinline__ double2 rhs_pi(const Grid& g, const Metric& M, const Vars& V,
-                                          int ii, int jj, int k) {
+// rhs_pi at one point (lines_method_lib.f90:716-753); QUOT: divide by sqrt(gamma)
+// as the tiled forms do, from its correctly rounded reciprocal
+template <int MK, bool QUOT = false>
+__device__ __forceinline__ double2 rhs_pi(const Grid& g, const Metric& M, const Vars& V, int ii, int jj, int k,
+                                          const double* rsg = nullptr) {
   const int q = off2(g, ii, jj);
   const long long p = off3(g, ii, jj, k);
   const double sg = ldm(M.sqrtg, q), be = ldm(M.beta, q), dxb = ldm(M.dxbeta, q), am2 = ldm(M.am2, q);
@@ -76,12 +77,17 @@ __device__ __forceinline__ double2 rhs_pi(const Grid& g, const Metric& M, const 
   auto Q = [&](int i2, int j2, int k2) {
     return rmul(ldm(M.sqrtg, off2(g, i2, j2)), ldf(V.v[4], off3(g, i2, j2, k2)));
   };
-  const double2 r1 = cdivr(op_dr(g, G1, ii, jj, k), sg);
-  const double2 r2 = cdivr(op_dth(g, H, ii, jj, k), sg);
+  auto quot1 = [&](double a) {
+    const double rb = ldm(rsg, q), t = a * rb;
+    return __fma_rn(__fma_rn(-t, sg, a), rb, t);
+  };
+  auto quot = [&](double2 a) { return QUOT ? c2(quot1(a.x), quot1(a.y)) : cdivr(a, sg); };
+  const double2 r1 = quot(op_dr(g, G1, ii, jj, k));
+  const double2 r2 = quot(op_dth(g, H, ii, jj, k));
   const double2 d3 = op_dph(g, Fp, ii, jj, k);
-  const double2 r3 = (MK == MK_KS) ? cdivr(d3, sg) : d3;
+  const double2 r3 = (MK == MK_KS) ? quot(d3) : d3;
   const double2 r4 = rmul(dxb, ldf(V.v[4], p));
-  const double2 r5 = cdivr(rmul(be, op_ar(g, Q, be, ii, jj, k)), sg);
+  const double2 r5 = quot(rmul(be, op_ar(g, Q, be, ii, jj, k)));
   const double2 r6 = rmul(am2, ldf(V.v[0], p));
   return csub(cadd(cadd(cadd(cadd(r1, r2), r3), r4), r5), r6);
 }
@@ -238,6 +244,57 @@ void launch_rhs(const Grid& g, const Metric& m, int metric_kind, const double2* 
     rhs_kernel<MK_KS><<<stage_grid(g), stage_block(), 0, st>>>(g, m, V, out, mask);
   else
     rhs_kernel<MK_SCHW><<<stage_grid(g), stage_block(), 0, st>>>(g, m, V, out, mask);
+}
+
+// First stage of a pair of RK4 stages (kg_pair.cu) on the theta rows 3 and NJ-4,
+// planes 1..Nz-1, with its x fill: what the pair's tiles next to a pole take as
+// their ghost row.  Two rows of the grid, so every neighbour comes from the caches.
+constexpr int POLE_T = 128;
+template <int PAIR, int MK>
+__global__ void __launch_bounds__(POLE_T) pole_rows_kernel(Grid g, Metric M, const double* rsg, const double2* X,
+                                                           const double2* base, int inflow, double2* pole) {
+  __shared__ double2 first[4][5];
+  const int ii = blockIdx.x * POLE_T + threadIdx.x;
+  const int side = blockIdx.y, k = 1 + blockIdx.z;
+  const int jj = side ? g.NJ - 4 : 3;
+  const bool hold = ii == g.NI - 1 && inflow;
+  const int ic = ii == g.NI - 1 ? ii - 1 : ii;  // the outer copy forms its source
+  double2 y[5];
+  if (ii < g.NI) {
+    const long long fs = g.fs;
+    if (hold) {
+      for (int v = 1; v < 5; ++v) y[v] = ldf(base + v * fs, off3(g, ii, jj, k));
+    } else {
+      Vars V;
+      for (int v = 0; v < 5; ++v) V.v[v] = X + v * fs;
+      double2 r[5];
+      rhs_psi(g, M, V, ic, jj, k, r);
+      r[4] = rhs_pi<MK, true>(g, M, V, ic, jj, k, rsg);
+      const long long p = off3(g, ic, jj, k);
+#pragma unroll
+      for (int v = 1; v < 5; ++v) {
+        const double2 kk = rmul(g.dt, r[v]);
+        y[v] = cadd(ldf(base + v * fs, p), PAIR == 0 ? rmul(0.50, kk) : kk);
+      }
+    }
+    if (ii >= 1 && ii <= 3)
+      for (int v = 1; v < 5; ++v) first[ii][v] = y[v];
+  }
+  __syncthreads();
+  if (ii >= g.NI) return;
+  if (ii == 0)
+    for (int v = 1; v < 5; ++v)
+      y[v] = cadd(csub(rmul(3.0, first[1][v]), rmul(3.0, first[2][v])), first[3][v]);
+  const long long ps = (long long)g.NK * g.PI;
+#pragma unroll
+  for (int v = 1; v < 5; ++v) pole[(5 * side + v) * ps + (long long)k * g.PI + ii] = y[v];
+}
+
+void launch_pole_rows(int pair, const PairLaunch& L, const double* rsg, double2* pole, cudaStream_t st) {
+  const dim3 grid((L.g.NI + POLE_T - 1) / POLE_T, 2, L.g.Nz - 1);
+  auto kern = pair == 0 ? (L.metric_kind == MK_KS ? pole_rows_kernel<0, MK_KS> : pole_rows_kernel<0, MK_SCHW>)
+                        : (L.metric_kind == MK_KS ? pole_rows_kernel<1, MK_KS> : pole_rows_kernel<1, MK_SCHW>);
+  kern<<<grid, POLE_T, 0, st>>>(L.g, L.m, rsg, L.X, L.base, L.inflow, pole);
 }
 
 }  // namespace kg
