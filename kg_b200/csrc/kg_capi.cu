@@ -15,8 +15,10 @@
 #include <cstring>
 #include <algorithm>
 #include <cstdint>
+#include <atomic>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/kg_capi.h"
@@ -674,6 +676,90 @@ int state_view(kg_solver* h, int which, View* out) {
   }
 }
 
+// Device to host, complete on return.  Into pageable memory the driver's copy runs
+// at one core's rate through its own staging; here four threads each bring pieces
+// through a pinned buffer of their own, the next piece's transfer under the
+// current one's copy (a state of 749 MB: 157 -> 53 ms, one of 52 MB: 11.5 -> 4.2 ms;
+// 17.6 MB of a_lm into a touched array: 1.04 -> 0.73 ms).  The pinned buffers, 8 MB
+// per device, live as long as the process; a second caller on the same device
+// meanwhile, a small copy, and pinned memory take the plain copy.
+constexpr size_t DL_PIECE = 1 << 20, DL_MIN = 4 << 20;
+constexpr int DL_THREADS = 4;
+struct Download {
+  std::mutex busy;
+  unsigned char* buf = nullptr;
+  cudaEvent_t ev[2 * DL_THREADS] = {};
+  bool ready() {  // under `busy`
+    if (buf) return true;
+    if (cudaHostAlloc((void**)&buf, 2 * DL_THREADS * DL_PIECE, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      buf = nullptr;
+      return false;
+    }
+    for (auto& e : ev)
+      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFreeHost(buf);
+        buf = nullptr;
+        return false;
+      }
+    return true;
+  }
+};
+
+bool pageable(const void* p) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return at.type == cudaMemoryTypeUnregistered;
+}
+
+int download(kg_solver* h, void* dst, const void* src, size_t n) {
+  static Download per_device[POOL_DEVICES];
+  Download* d = n >= DL_MIN && h->device < POOL_DEVICES && pageable(dst) ? &per_device[h->device] : nullptr;
+  std::unique_lock<std::mutex> lock;
+  if (d) lock = std::unique_lock<std::mutex>(d->busy, std::try_to_lock);
+  if (!d || !lock.owns_lock() || !d->ready()) {
+    KG_CK(cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, h->stream));
+    KG_CK(cudaStreamSynchronize(h->stream));
+    return KG_OK;
+  }
+  const size_t pieces = (n + DL_PIECE - 1) / DL_PIECE;
+  std::atomic<int> bad{0};
+  auto size = [&](size_t c) { return c + 1 < pieces ? DL_PIECE : n - c * DL_PIECE; };
+  auto work = [&](int w) {
+    if (cudaSetDevice(h->device) != cudaSuccess) bad = 1;
+    auto fetch = [&](size_t c) {
+      const int s = 2 * w + (int)(c / DL_THREADS & 1);
+      if (cudaMemcpyAsync(d->buf + s * DL_PIECE, (const unsigned char*)src + c * DL_PIECE, size(c),
+                          cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
+          cudaEventRecord(d->ev[s], h->stream) != cudaSuccess)
+        bad = 1;
+    };
+    if ((size_t)w < pieces) fetch(w);
+    for (size_t c = w; c < pieces && !bad; c += DL_THREADS) {
+      const int s = 2 * w + (int)(c / DL_THREADS & 1);
+      if (c + DL_THREADS < pieces) fetch(c + DL_THREADS);
+      if (cudaEventSynchronize(d->ev[s]) != cudaSuccess) bad = 1;
+      else memcpy((unsigned char*)dst + c * DL_PIECE, d->buf + s * DL_PIECE, size(c));
+    }
+  };
+  std::thread helper[DL_THREADS];
+  int started = 1;
+  try {
+    for (; started < DL_THREADS; ++started) helper[started] = std::thread(work, started);
+  } catch (...) {  // no more threads: this one does their share
+  }
+  work(0);
+  for (int w = started; w < DL_THREADS; ++w) work(w);
+  for (int w = 1; w < started; ++w) helper[w].join();
+  const cudaError_t e = cudaStreamSynchronize(h->stream);
+  if (e != cudaSuccess || bad) return set_err(h, KG_ECUDA, std::string("copy to the host: ") + cudaGetErrorString(e));
+  return KG_OK;
+}
+
 // a caller's device buffer that the conversion kernels can use in place: memory of
 // this device at the alignment of a complex value
 bool direct_buffer(const kg_solver* h, const void* p) {
@@ -728,8 +814,12 @@ int store_view(kg_solver* h, const View& V, double* dst, cudaMemcpyKind kind) {
     const size_t n = (size_t)(k1 - k0) * plane_elems;
     { Prof pf(h, PK_CONVERT, 1); kg::launch_soa_to_aos(g, V.v[0], V.v[4], h->stage_buf, k0, k1, h->stream); }
     KG_CK(cudaGetLastError());
-    KG_CK(cudaMemcpyAsync((double2*)dst + (size_t)k0 * plane_elems, h->stage_buf, n * sizeof(double2), kind,
-                          h->stream));
+    double2* to = (double2*)dst + (size_t)k0 * plane_elems;
+    if (kind == cudaMemcpyDeviceToHost && pageable(to)) {
+      if ((rc = download(h, to, h->stage_buf, n * sizeof(double2)))) return rc;
+    } else {
+      KG_CK(cudaMemcpyAsync(to, h->stage_buf, n * sizeof(double2), kind, h->stream));
+    }
   }
   return KG_OK;
 }
@@ -1820,8 +1910,7 @@ int kg_project_all_shells(kg_solver* h, int L, int precision, double* host_alm) 
   int rc = project_all(h, L, precision, &dalm);
   if (rc) return rc;
   const size_t szAlm = (size_t)(L + 1) * (2 * L + 1) * h->Nx * sizeof(double2);
-  KG_CK(cudaMemcpyAsync(host_alm, dalm, szAlm, cudaMemcpyDeviceToHost, h->stream));
-  KG_CK(cudaStreamSynchronize(h->stream));
+  if ((rc = download(h, host_alm, dalm, szAlm))) return rc;
   return check_device_flag(h);
 }
 
@@ -1853,9 +1942,7 @@ int kg_sph_ft_radial(kg_solver* h, int L, int Nk, int precision, double* host_ft
     kg::launch_radial_ft(dalm, h->rad_jr, L, Nk, h->Nx, dr, h->rad_ft, h->stream);
   }
   KG_CK(cudaGetLastError());
-  KG_CK(cudaMemcpyAsync(host_ft, h->rad_ft, (size_t)Nk * (L + 1) * (2 * L + 1) * sizeof(double2),
-                        cudaMemcpyDeviceToHost, h->stream));
-  KG_CK(cudaStreamSynchronize(h->stream));
+  if ((rc = download(h, host_ft, h->rad_ft, (size_t)Nk * (L + 1) * (2 * L + 1) * sizeof(double2)))) return rc;
   return check_device_flag(h);
 }
 

@@ -101,7 +101,7 @@ class LinesMethod:
         return (self.NK, self.NJ, self.NI, 5)
 
     def _get(self, which):
-        out = np.zeros(self.state_shape(), np.complex128)
+        out = np.empty(self.state_shape(), np.complex128)
         self._ck(self._lib.kg_get_state(self._h, which, _dp(out.view(np.float64))))
         return out
 
@@ -223,7 +223,7 @@ class LinesMethod:
 
     # -- geometry (MoL/geometry.f90)
     def metric_tables(self):
-        out = np.zeros((8, self.NJ, self.NI))
+        out = np.empty((8, self.NJ, self.NI))
         self._ck(self._lib.kg_get_metric(self._h, _dp(out)))
         return out
 
@@ -251,7 +251,7 @@ class ScalarField(LinesMethod):
 
     @property
     def rho(self):
-        out = np.zeros((self.NK, self.NJ, self.NI))
+        out = np.empty((self.NK, self.NJ, self.NI))
         self._ck(self._lib.kg_get_density(self._h, _dp(out)))
         return out
 
@@ -284,20 +284,20 @@ class ScalarField(LinesMethod):
     def project_all_shells(self, L, precision=1):
         """a_lm (l <= L) of phi on every vertex shell: array (Nx, 2L+1, L+1) complex.
         precision 1: split-BF16 tensor-core GEMM (FP32 accumulation); 0: FP64."""
-        out = np.zeros((self.Nx, 2 * L + 1, L + 1), np.complex128)
+        out = np.empty((self.Nx, 2 * L + 1, L + 1), np.complex128)
         self._ck(self._lib.kg_project_all_shells(self._h, L, precision, _dp(out.view(np.float64))))
         return out
 
     def bessel_basis(self, L, Nk):
         """(k_values (Nk, L+1), j_basis (Nx, Nk, L+1)): generate_full_bessel_basis"""
-        k = np.zeros((Nk, L + 1))
-        jb = np.zeros((self.Nx, Nk, L + 1))
+        k = np.empty((Nk, L + 1))
+        jb = np.empty((self.Nx, Nk, L + 1))
         self._ck(self._lib.kg_bessel_basis(self._h, L, Nk, _dp(k), _dp(jb)))
         return k, jb
 
     def sph_ft_radial(self, L, Nk, precision=0):
         """SphFT_discrete_radial of phi: array (2L+1, L+1, Nk) complex, [m+L, l, n-1]"""
-        out = np.zeros((2 * L + 1, L + 1, Nk), np.complex128)
+        out = np.empty((2 * L + 1, L + 1, Nk), np.complex128)
         self._ck(self._lib.kg_sph_ft_radial(self._h, L, Nk, precision, _dp(out.view(np.float64))))
         return out
 
