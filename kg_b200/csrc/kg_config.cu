@@ -24,6 +24,7 @@
 // Divisions by sqrt(gamma) and RK4's 1/6 use the correctly rounded reciprocal
 // with one Markstein correction (the IEEE quotient for dividends above about
 // 2^-1000 in magnitude).
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include "kg_device.cuh"
 #include "kg_internal.h"
@@ -45,6 +46,7 @@ struct CfgArgs {
   double rr, rt, rp;   // 1 / (12 h) per direction
   double kr, kt, kp;   // eps / (64 h) per direction
   double rN;           // r of the outermost stored plane
+  int* err;            // set when a bounded wait runs out
 };
 
 // plane d steps from plane k (1 <= k <= Nz-1) over the Nz-1 distinct planes 1..Nz-1;
@@ -100,10 +102,10 @@ __device__ __forceinline__ double qdiv(double a, double b, double rb) {
 __device__ __forceinline__ double2 cqdiv(double2 a, double b, double rb) { return c2(qdiv(a.x, b, rb), qdiv(a.y, b, rb)); }
 constexpr double kSixth = 1.0 / 6.0;
 
-// RHS and RK4 combination at one stored point (ii, jj, k).  S(v, i, j) returns
+// RHS and RK4 combination at one interior point (ii, jj, k): rows 3..NJ-4, planes
+// 1..Nz-1 (the ghost fill behind every stage writes the others).  S(v, i, j) returns
 // variable v of the stage input at (i, j) on plane k, P(v, d) at the point's
-// own (ii, jj) on the plane d steps away in phi (d = -3..3, d != 0; only asked
-// for 1 <= k <= Nz-1); the two kernels below differ only in where S and P read
+// own (ii, jj) on the plane d steps away in phi (d = -3..3, d != 0); the two kernels below differ only in where S and P read
 // from, so they produce the same bits.
 template <int KIND, class SF, class PF>
 __device__ __forceinline__ void cfg_point(const CfgArgs& a, int ii, int jj, int k, const SF& S, const PF& P) {
@@ -113,10 +115,7 @@ __device__ __forceinline__ void cfg_point(const CfgArgs& a, int ii, int jj, int 
   const int q = off2(g, ii, jj);
   double2 r[5];
   const int n = g.NI - 1;
-  if (jj <= 2 || jj >= g.NJ - 3 || k == 0 || k == g.Nz) {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) r[v] = c2(0.0, 0.0);
-  } else if (ii == n) {
+  if (ii == n) {
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
       auto f = [&](int i2) { return S(v, i2, jj); };
@@ -181,23 +180,30 @@ __device__ __forceinline__ void cfg_point(const CfgArgs& a, int ii, int jj, int 
   }
   // RK4 combination, as the reference's k1..k4 form (MoL/lines_method_lib.f90:411-474)
   const double dt = g.dt;
+  // the operands of all variables are requested ahead of the first store
+  double2 bv[5], sv[5];
+#pragma unroll
+  for (int v = 0; v < 5; ++v) {
+    bv[v] = lds(a.base, (long long)v * g.fs + p);
+    if (KIND != ST_RK4_1) sv[v] = lds(a.acc, (long long)v * g.fs + p);
+  }
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
     const long long o = (long long)v * g.fs + p;
-    const double2 b = ldf(a.base, o);
+    const double2 b = bv[v];
     const double2 kk = c2(r[v].x * dt, r[v].y * dt);
     double2 res;
     if (KIND == ST_RK4_1) {
       a.acc[o] = kk;
       res = cadd(b, rmul(0.50, kk));
     } else if (KIND == ST_RK4_2) {
-      a.acc[o] = cadd(a.acc[o], rmul(2.0, kk));
+      a.acc[o] = cadd(sv[v], rmul(2.0, kk));
       res = cadd(b, rmul(0.50, kk));
     } else if (KIND == ST_RK4_3) {
-      a.acc[o] = cadd(a.acc[o], rmul(2.0, kk));
+      a.acc[o] = cadd(sv[v], rmul(2.0, kk));
       res = cadd(b, kk);
     } else {
-      res = cadd(b, cqdiv(cadd(a.acc[o], kk), 6.0, kSixth));
+      res = cadd(b, cqdiv(cadd(sv[v], kk), 6.0, kSixth));
     }
     a.out[o] = res;
   }
@@ -208,8 +214,8 @@ template <int KIND>
 __global__ void __launch_bounds__(128) cfg_stage_kernel(CfgArgs a) {
   const Grid& g = a.g;
   const int ii = blockIdx.x * blockDim.x + threadIdx.x;
-  const int jj = blockIdx.y;
-  const int k = blockIdx.z;
+  const int jj = 3 + blockIdx.y;
+  const int k = 1 + blockIdx.z;
   if (ii >= g.NI) return;
   const double2* U = a.in;
   auto S = [&](int v, int i2, int j2) { return ldf(U + (long long)v * g.fs, off3(g, i2, j2, k)); };
@@ -217,13 +223,17 @@ __global__ void __launch_bounds__(128) cfg_stage_kernel(CfgArgs a) {
   cfg_point<KIND>(a, ii, jj, k, S, P);
 }
 
-// Tiled form: a CTA owns a 32 x 8 tile of (r, theta) columns and marches through
-// a chunk of phi planes.  The plane being updated arrives in shared memory with
-// a +-4 r and +-3 theta halo (every same-plane neighbour the fourth-order
-// differences, the r closures and the sixth-order dissipation touch), double
-// buffered: the next plane's tile is copied by cp.async while this plane is
-// computed.  The phi neighbours of the thread's own column (planes k+-1..3)
-// are read through the read-only cache; the same values serve seven
+// Tiled form: a CTA owns a 32 x 8 tile of (r, theta) columns of the interior rows
+// and marches through a chunk of the planes 1..Nz-1.  The plane being updated
+// arrives in shared memory with a +-4 r and +-3 theta halo (every same-plane
+// neighbour the fourth-order differences, the r closures and the sixth-order
+// dissipation touch), double buffered: one TMA box of all five variables brings
+// the next plane's tile while this plane is computed (eleven cp.async per thread
+// and plane, each with its index arithmetic, did before).  With that, only the
+// interior rows and planes, the point-wise operands requested together and the fill
+// in one launch, 20 RK4 steps on 256 x 33 x 65 went from 13.3 to 9.7 ms (a stage 164
+// -> 125 us); the phi neighbours' latency from L2 bounds it.  Those (planes k+-1..3
+// of the thread's own column) are plain loads; the same values serve seven
 // consecutive planes of the march.  (Holding them in a rolling register window
 // instead needs 255 registers per thread and one CTA per SM, and ran the C0
 // grid at half the speed.)
@@ -232,114 +242,146 @@ constexpr int CW = CTI + 2 * CRH, CH = CTJ + 2 * CTH, CT_N = CW * CH;
 constexpr size_t CFG_TILE_BYTES = (size_t)5 * CT_N * sizeof(double2);
 
 template <int KIND>
-__global__ void __launch_bounds__(CTI * CTJ, 2) cfg_march_kernel(CfgArgs a, int kchunk) {
-  extern __shared__ __align__(16) unsigned char cfg_smem[];
-  double2* tiles = reinterpret_cast<double2*>(cfg_smem);
+__global__ void __launch_bounds__(CTI * CTJ, 2)
+    cfg_march_kernel(const __grid_constant__ CUtensorMap tm, CfgArgs a, int kchunk) {
+  extern __shared__ __align__(128) unsigned char cfg_smem[];
+  double2* tiles;
+  {
+    const uint32_t b = saddr(cfg_smem);
+    tiles = reinterpret_cast<double2*>(cfg_smem + ((128u - (b & 127u)) & 127u));
+  }
+  __shared__ uint64_t bars[2];
   const Grid& g = a.g;
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * CTI + tx;
-  const int ii0 = blockIdx.x * CTI, jj0 = blockIdx.y * CTJ;
+  const int ii0 = blockIdx.x * CTI, jj0 = 3 + blockIdx.y * CTJ;
   const int ii = ii0 + tx, jj = jj0 + ty;
-  const bool act = ii < g.NI && jj < g.NJ;
-  const int k0 = blockIdx.z * kchunk;
-  if (k0 >= g.NK) return;  // uniform over the block
-  const int k1 = min(k0 + kchunk, g.NK);
+  const bool act = ii < g.NI && jj < g.NJ - 3;
+  const int k0 = 1 + blockIdx.z * kchunk, k1 = min(k0 + kchunk, g.Nz);
   const double2* col = a.in + (act ? off3(g, ii, jj, 0) : 0);
-  // points of the halo tile outside the array are not copied; no stencil reads them
-  auto load = [&](int k, int buf) {
-    double2* dst = tiles + (size_t)buf * 5 * CT_N;
-    for (int t = tid; t < 5 * CT_N; t += CTI * CTJ) {
-      const int v = t / CT_N, r = t - v * CT_N, ly = r / CW, lx = r - ly * CW;
-      const int gi = ii0 - CRH + lx, gj = jj0 - CTH + ly;
-      if (gi >= 0 && gi < g.NI && gj >= 0 && gj < g.NJ)
-        cp_async16(dst + t, a.in + (long long)v * g.fs + off3(g, gi, gj, k));
-    }
-    cp_async_commit();
+  if (tid == 0) {
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  pdl_wait();
+  auto load = [&](int k, int buf) {  // the box starts at most 4 columns before the array, where it reads zeros
+    mbar_expect_tx(&bars[buf], (uint32_t)CFG_TILE_BYTES);
+    tma_load_4d(tiles + (size_t)buf * 5 * CT_N, &tm, 2 * (ii0 - CRH), jj0 - CTH, k, 0, &bars[buf]);
   };
-  load(k0, 0);
-  for (int k = k0; k < k1; ++k) {
+  if (tid == 0) load(k0, 0);
+  int timed_out = 0;
+  bool failed = false;
+  int last = k0;  // the plane of the newest copy
+  for (int k = k0; k < k1 && !failed; ++k) {
     const int buf = (k - k0) & 1;
     if (k + 1 < k1) {
-      load(k + 1, buf ^ 1);  // that buffer was last read before the previous block barrier
-      cp_async_wait_prior();
-    } else {
-      cp_async_wait_all();
+      if (tid == 0) load(k + 1, buf ^ 1);  // that buffer was last read before the barrier of the plane before
+      last = k + 1;
     }
-    __syncthreads();
-    if (act) {
+    if (!mbar_wait_bounded(&bars[buf], (uint32_t)((k - k0) >> 1) & 1u)) timed_out = 1;
+    if (act && !timed_out) {
       // every same-plane neighbour lies inside the halo tile
       const double2* T = tiles + (size_t)buf * 5 * CT_N + (ty + CTH) * CW + (tx + CRH);
       auto S = [&](int v, int i2, int j2) { return T[v * CT_N + (j2 - jj) * CW + (i2 - ii)]; };
-      auto P = [&](int v, int d) { return ldf(col + (long long)v * g.fs, (long long)kper(g, k, d) * g.plane); };
+      auto P = [&](int v, int d) { return lds(col + (long long)v * g.fs, (long long)kper(g, k, d) * g.plane); };
       cfg_point<KIND>(a, ii, jj, k, S, P);
+    }
+    failed = __syncthreads_or(timed_out) != 0;
+  }
+  if (failed) {
+    if (tid == 0) {
+      atomicExch(a.err, 1);
+      // the newest copy into either buffer lands before the CTA's shared memory is released (bounded)
+      for (int q = last; q >= k0 && q > last - 2; --q)
+        (void)mbar_wait_bounded(&bars[(q - k0) & 1], (uint32_t)((q - k0) >> 1) & 1u);
     }
     __syncthreads();
   }
 }
 
-// duplicated phi planes: k = 0 <- Nz-1, k = Nz <- 1
-__global__ void cfg_ghost_z(Grid g, double2* u) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long n = (long long)g.NI * g.NJ;
-  if (t >= n) return;
-  const int ii = (int)(t % g.NI), jj = (int)(t / g.NI);
+// The method's fill: phi planes 0 <- Nz-1 and Nz <- 1, then the theta ghost rows
+// from the interior rows at phi + pi, psi_2 negated.  One launch, a block per row:
+// a ghost row whose partner is plane 0 reads plane Nz-1, its source, so no row that
+// is read is written (event-timed on 256 x 33 x 65, two launches before: 19.0 ->
+// 8.9 us).
+__global__ void cfg_ghost_kernel(Grid g, double2* u) {
+  pdl_wait();
+  const int nz = 2 * (g.NJ - 6);  // interior rows of the two planes
+  int jd, kd, js, ks;
+  bool ghost = false;
+  if ((int)blockIdx.x < nz) {
+    jd = js = 3 + blockIdx.x % (g.NJ - 6);
+    const bool last = (int)blockIdx.x >= g.NJ - 6;
+    kd = last ? g.Nz : 0;
+    ks = last ? 1 : g.Nz - 1;
+  } else {
+    const int q = blockIdx.x - nz, r = q % 6;
+    ghost = true;
+    kd = q / 6;
+    jd = r < 3 ? r : g.NJ - 6 + r;
+    js = jd <= 2 ? 5 - jd : 2 * g.NJ - 7 - jd;
+    ks = ktarget(g, kd);
+    if (ks == 0) ks = g.Nz - 1;
+  }
+  for (int ii = threadIdx.x; ii < g.NI; ii += blockDim.x) {
+    double2 s[5];
 #pragma unroll
-  for (int v = 0; v < 5; ++v) {
-    double2* w = u + (long long)v * g.fs;
-    w[off3(g, ii, jj, 0)] = w[off3(g, ii, jj, g.Nz - 1)];
-    w[off3(g, ii, jj, g.Nz)] = w[off3(g, ii, jj, 1)];
+    for (int v = 0; v < 5; ++v) s[v] = u[(long long)v * g.fs + off3(g, ii, js, ks)];
+    if (ghost) s[2] = rmul(-1.0, s[2]);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) u[(long long)v * g.fs + off3(g, ii, jd, kd)] = s[v];
   }
 }
 
-// theta ghost rows from the interior rows at phi + pi, psi_2 negated
-__global__ void cfg_ghost_rows(Grid g, double2* u) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long n = 6LL * g.NI * g.NK;
-  if (t >= n) return;
-  const int ii = (int)(t % g.NI);
-  const long long rk = t / g.NI;
-  const int r = (int)(rk % 6);
-  const int k = (int)(rk / 6);
-  const int jj = (r < 3) ? r : (g.NJ - 6 + r);
-  const int js = (jj <= 2) ? (5 - jj) : (2 * g.NJ - 7 - jj);
-  const int kt = ktarget(g, k);
-#pragma unroll
-  for (int v = 0; v < 5; ++v) {
-    double2* w = u + (long long)v * g.fs;
-    const double2 s = w[off3(g, ii, js, kt)];
-    w[off3(g, ii, jj, k)] = (v == 2) ? rmul(-1.0, s) : s;
+typedef CUresult (*EncodeTiledFnC)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// the stage input as (doubles along r, theta rows, phi planes, variables), boxes of
+// one plane's halo tile
+bool cfg_encode(CUtensorMap* tm, const Grid& g, const double2* base) {
+  static EncodeTiledFnC fn = nullptr;
+  if (!fn) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = (EncodeTiledFnC)p;
+    if (!fn) return false;
   }
+  cuuint64_t dims[4] = {(cuuint64_t)(2 * g.PI), (cuuint64_t)g.NJ, (cuuint64_t)g.NK, 5};
+  cuuint64_t strides[3] = {(cuuint64_t)g.PI * 16, (cuuint64_t)g.plane * 16, (cuuint64_t)g.fs * 16};
+  cuuint32_t box[4] = {2 * CW, CH, 1, 5};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return fn(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, (void*)base, dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <int KIND>
 int cfg_march_launch(const CfgArgs& a, cudaStream_t st) {
   static bool attr = false;  // dynamic shared memory above 48 KB, set once per stage kind
+  constexpr int SMEM = 2 * (int)CFG_TILE_BYTES + 128;
   if (!attr) {
-    if (cudaFuncSetAttribute(cfg_march_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(2 * CFG_TILE_BYTES)) != cudaSuccess)
+    if (cudaFuncSetAttribute(cfg_march_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
       return -1;
     attr = true;
   }
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
-  }
   const Grid& g = a.g;
-  const int tx = (g.NI + CTI - 1) / CTI, ty = (g.NJ + CTJ - 1) / CTJ;
-  // about two waves of two CTAs per SM: small grids are cut into phi chunks
-  int nch = (4 * sms + tx * ty - 1) / (tx * ty);
-  nch = nch < 1 ? 1 : (nch > g.NK ? g.NK : nch);
-  const int kchunk = (g.NK + nch - 1) / nch;
-  nch = (g.NK + kchunk - 1) / kchunk;
-  cfg_march_kernel<KIND><<<dim3(tx, ty, nch), dim3(CTI, CTJ, 1), 2 * CFG_TILE_BYTES, st>>>(a, kchunk);
-  return 0;
+  CUtensorMap tm;
+  if (!cfg_encode(&tm, g, a.in)) return -1;
+  const int tx = (g.NI + CTI - 1) / CTI, ty = (g.NJ - 6 + CTJ - 1) / CTJ, planes = g.Nz - 1;
+  const int kchunk = phi_chunk(planes, (long long)tx * ty, 148 * 2, 32);
+  return launch_pdl(cfg_march_kernel<KIND>, dim3(tx, ty, (planes + kchunk - 1) / kchunk), dim3(CTI, CTJ, 1), SMEM, st,
+                    tm, a, kchunk) == cudaSuccess
+             ? 0
+             : -1;
 }
 
 }  // namespace
 
 int launch_stage_cfg(int kind, const StageLaunch& L, const double* dxbeta4, const double* rsg, const double coef[6],
-                     double rN, int tiled, cudaStream_t st) {
+                     double rN, int tiled, int* err, cudaStream_t st) {
   CfgArgs a;
   a.g = L.g;
   a.m = L.m;
@@ -356,16 +398,17 @@ int launch_stage_cfg(int kind, const StageLaunch& L, const double* dxbeta4, cons
   a.kt = coef[4];
   a.kp = coef[5];
   a.rN = rN;
-  if (tiled) {
+  a.err = err;
+  if (tiled) {  // without tensor maps: one thread per point
     switch (kind) {
-      case ST_RK4_1: return cfg_march_launch<ST_RK4_1>(a, st);
-      case ST_RK4_2: return cfg_march_launch<ST_RK4_2>(a, st);
-      case ST_RK4_3: return cfg_march_launch<ST_RK4_3>(a, st);
-      case ST_RK4_4: return cfg_march_launch<ST_RK4_4>(a, st);
+      case ST_RK4_1: if (cfg_march_launch<ST_RK4_1>(a, st) == 0) return 0; break;
+      case ST_RK4_2: if (cfg_march_launch<ST_RK4_2>(a, st) == 0) return 0; break;
+      case ST_RK4_3: if (cfg_march_launch<ST_RK4_3>(a, st) == 0) return 0; break;
+      case ST_RK4_4: if (cfg_march_launch<ST_RK4_4>(a, st) == 0) return 0; break;
       default: return -1;
     }
   }
-  dim3 grid((L.g.NI + 127) / 128, L.g.NJ, L.g.NK);
+  dim3 grid((L.g.NI + 127) / 128, L.g.NJ - 6, L.g.Nz - 1);
   switch (kind) {
     case ST_RK4_1: cfg_stage_kernel<ST_RK4_1><<<grid, 128, 0, st>>>(a); return 0;
     case ST_RK4_2: cfg_stage_kernel<ST_RK4_2><<<grid, 128, 0, st>>>(a); return 0;
@@ -376,10 +419,8 @@ int launch_stage_cfg(int kind, const StageLaunch& L, const double* dxbeta4, cons
 }
 
 void launch_ghost_fill_cfg(const Grid& g, double2* u, cudaStream_t st) {
-  const long long nz = (long long)g.NI * g.NJ;
-  cfg_ghost_z<<<(unsigned)((nz + 255) / 256), 256, 0, st>>>(g, u);
-  const long long nr = 6LL * g.NI * g.NK;
-  cfg_ghost_rows<<<(unsigned)((nr + 255) / 256), 256, 0, st>>>(g, u);
+  const int nt = g.NI >= 256 ? 256 : (g.NI + 31) / 32 * 32;
+  launch_pdl(cfg_ghost_kernel, 2 * (g.NJ - 6) + 6 * g.NK, nt, 0, st, g, u);
 }
 
 }  // namespace kg

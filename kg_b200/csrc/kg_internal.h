@@ -185,7 +185,7 @@ int launch_batch_mixed(int kind, int mk, const void* d_items, int n_solves, int 
 // 1/sqrt(gamma) table; tiled = 1 for the shared-memory tiled marching form, 0 for
 // one thread per point (same bits)
 int launch_stage_cfg(int kind, const StageLaunch& L, const double* dxbeta4, const double* rsg, const double coef[6],
-                     double rN, int tiled, cudaStream_t st);
+                     double rN, int tiled, int* err, cudaStream_t st);
 void launch_ghost_fill_cfg(const Grid& g, double2* u, cudaStream_t st);
 // Berger-Oliger transfers between radially nested 2:1 levels (kg_refine.cu)
 // uf_pi: where the fine Pi variable lives (nullptr: uf + 4 fs, the 5-variable layout)
