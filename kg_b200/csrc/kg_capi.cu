@@ -71,6 +71,7 @@ struct kg_solver {
   size_t stage_bytes = 0;
   int stage_planes = 0;
   double* rho = nullptr;
+  double* mass_host = nullptr;           // mapped host slot of the mass integral (host_slot)
   double* partials = nullptr;            // mass partial sums, result, CTA counter
   int s_cur = 4, t_cur = 4;              // slot holding the current Pi stage value
   int variant = 3;                       // 0: per-point, 1: 2.5-D marching, 2, 3: TMA-pipelined marching
@@ -168,6 +169,43 @@ cudaMemPool_t solver_pool(int dev) {
     pools[dev] = pool;
   }
   return pools[dev];
+}
+
+// One double of mapped host memory for a handle's mass integral: the kernel stores
+// it there, so that a caller who reads it every step waits for the kernel alone and
+// not for a copy behind it.  512 slots in one page-locked block per process; a
+// handle beyond them copies.
+struct HostSlots {
+  std::mutex mu;
+  double* base = nullptr;
+  bool tried = false;
+  std::vector<int> free_;
+};
+HostSlots& host_slots() {
+  static HostSlots* s = new HostSlots();  // outlives every handle
+  return *s;
+}
+double* host_slot() {
+  HostSlots& s = host_slots();
+  std::lock_guard<std::mutex> lock(s.mu);
+  if (!s.tried) {
+    s.tried = true;
+    if (cudaHostAlloc((void**)&s.base, 512 * sizeof(double), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      s.base = nullptr;
+    }
+    for (int i = 0; s.base && i < 512; ++i) s.free_.push_back(i);
+  }
+  if (s.free_.empty()) return nullptr;
+  const int i = s.free_.back();
+  s.free_.pop_back();
+  return s.base + i;
+}
+void free_host_slot(double* p) {
+  if (!p) return;
+  HostSlots& s = host_slots();
+  std::lock_guard<std::mutex> lock(s.mu);
+  s.free_.push_back((int)(p - s.base));
 }
 
 int dalloc(kg_solver* h, void** p, size_t n) {
@@ -963,6 +1001,7 @@ int kg_create(const kg_params* p, int device, kg_solver** out) {
 int kg_destroy(kg_solver* h) {
   if (!h) return KG_EINVAL;
   if (h->stream) cudaStreamSynchronize(h->stream);
+  free_host_slot(h->mass_host);
   void* bufs[] = {h->dmet, h->U, h->S, h->T, h->RK[0], h->RK[1], h->RK[2], h->pole, h->UP, h->HV, h->stage_buf, h->rho, h->partials,
                   h->d_int, h->d_dbl, h->shells, h->alm, h->flux, h->derr, h->ylm_tab, h->ylm_buf,
                   h->rad_jr, h->rad_ft, h->MX};
@@ -1699,14 +1738,16 @@ int kg_mass_scalar(kg_solver* h, double* out) {
     int rc = dalloc(h, (void**)&h->rho, (size_t)h->g.fs * sizeof(double));
     if (rc) return rc;
   }
+  if (!h->mass_host) h->mass_host = host_slot();
   double* res = h->partials + kg::mass_blocks(h->g);
   {
     Prof pf(h, PK_MASS, 1);
-    kg::launch_mass(h->g, metric_of(h), h->rho, h->dx * h->dy * h->dz, h->partials, res, h->stream);
+    kg::launch_mass(h->g, metric_of(h), h->rho, h->dx * h->dy * h->dz, h->partials, res, h->mass_host, h->stream);
   }
   KG_CK(cudaGetLastError());
-  KG_CK(cudaMemcpyAsync(out, res, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  if (!h->mass_host) KG_CK(cudaMemcpyAsync(out, res, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   KG_CK(cudaStreamSynchronize(h->stream));
+  if (h->mass_host) *out = *(volatile double*)h->mass_host;
   return KG_OK;
 }
 

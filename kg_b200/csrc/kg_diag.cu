@@ -52,8 +52,8 @@ __device__ double2 block_sum2(double2 v) {
 
 // density (diagnostic_lib.f90:277-289); the complex term 2 g^rphi |psi1| psi3
 // makes the sum complex and rho keeps its real part.
-__global__ void density_kernel(Grid g, Metric m, const double2* __restrict__ u, double mass2,
-                               double* __restrict__ rho) {
+__global__ void density_kernel(Grid g, Metric m, const double2* u, double mass2, double* rho) {
+  pdl_wait();
   const int ii = blockIdx.x * blockDim.x + threadIdx.x;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
@@ -78,7 +78,7 @@ __global__ void density_kernel(Grid g, Metric m, const double2* __restrict__ u, 
 
 void launch_density(const Grid& g, const Metric& m, const double2* u, double mass2, double* rho, cudaStream_t st) {
   dim3 b(64, 4, 1), gr((g.NI + 63) / 64, (g.NJ + 3) / 4, g.NK);
-  density_kernel<<<gr, b, 0, st>>>(g, m, u, mass2, rho);
+  launch_pdl(density_kernel, gr, b, 0, st, g, m, u, mass2, rho);
 }
 
 // trapezium over i in [0,Nx] (ii in [2, NI-3]), j in [0,Ny], k in [0,Nz] of
@@ -99,8 +99,9 @@ struct MassSum {
   double value;
   unsigned int left;
 };
-__global__ void mass_kernel(Grid g, const double* __restrict__ sqrtg, const double* __restrict__ rho,
-                            double* partials, MassSum* sum, double scale) {
+__global__ void mass_kernel(Grid g, const double* sqrtg, const double* rho, double* partials, MassSum* sum,
+                            double scale, double* host) {
+  pdl_wait();
   const int ni = g.NI - 4, nj = g.NJ - 4, nk = g.NK;
   const int rows = nj * nk;
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -118,7 +119,7 @@ __global__ void mass_kernel(Grid g, const double* __restrict__ sqrtg, const doub
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const int a = a0 + 32 * u;
-        rv[u] = a < ni ? __ldg(rr + a) : 0.0;
+        rv[u] = a < ni ? rr[a] : 0.0;
         sv[u] = a < ni ? __ldg(sr + a) : 0.0;
       }
 #pragma unroll
@@ -158,17 +159,19 @@ __global__ void mass_kernel(Grid g, const double* __restrict__ sqrtg, const doub
     const double v = warp_sum(ws[threadIdx.x]);
     if (threadIdx.x == 0) {
       sum->value = v * scale;
+      if (host) *host = v * scale;
       sum->left = 0u;
     }
   }
 }
 
 void launch_mass(const Grid& g, const Metric& m, const double* rho, double dxdydz, double* partials, double* out,
-                 cudaStream_t st) {
+                 double* host, cudaStream_t st) {
   const long long rows = (long long)(g.NJ - 4) * g.NK;
   const int nw = MASS_THREADS / 32;
   const int nb = (int)(rows < (long long)nw * mass_blocks(g) ? (rows + nw - 1) / nw : mass_blocks(g));
-  mass_kernel<<<nb, MASS_THREADS, 0, st>>>(g, m.sqrtg, rho, partials, reinterpret_cast<MassSum*>(out), dxdydz);
+  launch_pdl(mass_kernel, nb, MASS_THREADS, 0, st, g, m.sqrtg, rho, partials, reinterpret_cast<MassSum*>(out), dxdydz,
+             host);
 }
 
 // ---- detector shells ---------------------------------------------------------
@@ -183,8 +186,9 @@ void launch_mass(const Grid& g, const Metric& m, const double* rho, double dxdyd
 // bound by that one latency on the grids that are sampled every few steps: four
 // fields on 64 x 17 x 33, five detectors, 31 -> 8.7 us event-timed.
 template <int MASK>
-__global__ void shell_interp_kernel(Grid g, Metric m, const double2* __restrict__ u, ShellInterp si, int Ny, int Nz,
-                                    double2* __restrict__ out) {
+__global__ void shell_interp_kernel(Grid g, Metric m, const double2* u, ShellInterp si, int Ny, int Nz,
+                                    double2* out) {
+  pdl_wait();
   constexpr int NF = MASK == 1 ? 1 : (MASK & 1) ? 4 : 3, F0 = (MASK & 1) ? 0 : 1;  // fields F0 .. F0 + NF - 1
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int d = blockIdx.y;
@@ -238,9 +242,8 @@ void launch_shell_interp(const Grid& g, const Metric& m, const double2* u, const
                          int Nz, int which_mask, double2* out, cudaStream_t st) {
   const int nt = 64;  // a vertex sphere of a small grid still spreads over the SMs
   dim3 gr((Ny * Nz + nt - 1) / nt, n_det);
-  if (which_mask == 1) shell_interp_kernel<1><<<gr, nt, 0, st>>>(g, m, u, si, Ny, Nz, out);
-  else if (which_mask == 14) shell_interp_kernel<14><<<gr, nt, 0, st>>>(g, m, u, si, Ny, Nz, out);
-  else shell_interp_kernel<15><<<gr, nt, 0, st>>>(g, m, u, si, Ny, Nz, out);
+  launch_pdl(which_mask == 1 ? shell_interp_kernel<1> : which_mask == 14 ? shell_interp_kernel<14> : shell_interp_kernel<15>,
+             gr, nt, 0, st, g, m, u, si, Ny, Nz, out);
 }
 
 // trapezium_2D_complex selector weight (tools/integral.f90:330-362)
@@ -267,10 +270,11 @@ __device__ __forceinline__ void flux_block(const double2* shells, int c, int d, 
 // One block per (l, m, detector), m on either side of zero in turn of l: the
 // (L + 1)^2 pairs with |m| <= l, none of them empty; then, when `out` is given,
 // three blocks per detector for the fluxes, which read the same shells.
-__global__ void shell_reduce_kernel(const double2* __restrict__ shells, const int* active, int L, int Ny, int Nz,
+__global__ void shell_reduce_kernel(const double2* shells, const int* active, int L, int Ny, int Nz,
                                     const double* __restrict__ normP, const double* __restrict__ cosm,
                                     const double* __restrict__ sinm, const double* __restrict__ sint, double dydz,
                                     double2* alm, double* out) {
+  pdl_wait();
   const int d = blockIdx.y;
   if (!active[d]) return;
   int b = blockIdx.x;
@@ -314,8 +318,8 @@ void launch_shell_reduce(const double2* shells, const int* active, int n_det, in
                          const double* normP, const double* cosm, const double* sinm, const double* sint, double dydz,
                          double2* alm, double* flux, cudaStream_t st) {
   const int nb = (alm ? (L + 1) * (L + 1) : 0) + (flux ? 3 : 0);
-  shell_reduce_kernel<<<dim3(nb, n_det), 256, 0, st>>>(shells, active, L, Ny, Nz, normP, cosm, sinm, sint, dydz, alm,
-                                                       flux);
+  launch_pdl(shell_reduce_kernel, dim3(nb, n_det), 256, 0, st, shells, active, L, Ny, Nz, normP, cosm, sinm, sint, dydz,
+             alm, flux);
 }
 
 }  // namespace kg

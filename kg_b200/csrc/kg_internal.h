@@ -215,9 +215,10 @@ void launch_soa_to_aos(const Grid& g, const double2* soa, const double2* pi, dou
 struct ShellInterp;  // per-detector interpolation tables (kg_diag.cu)
 void launch_density(const Grid& g, const Metric& m, const double2* u, double mass2, double* rho, cudaStream_t st);
 // trapezium integral of rho*sqrtg over i in [0,Nx], j in [0,Ny], k in [0,Nz];
-// partial sums in `partials` (>= nblocks doubles), result in *out (device)
+// partial sums in `partials` (>= nblocks doubles), result in *out (device) and, when
+// given, *host (mapped host memory)
 int mass_blocks(const Grid& g);
-void launch_mass(const Grid& g, const Metric& m, const double* rho, double dxdydz, double* partials,
-                 double* out, cudaStream_t st);
+void launch_mass(const Grid& g, const Metric& m, const double* rho, double dxdydz, double* partials, double* out,
+                 double* host, cudaStream_t st);
 
 }  // namespace kg
