@@ -862,14 +862,29 @@ int store_view(kg_solver* h, const View& V, double* dst, cudaMemcpyKind kind) {
   return KG_OK;
 }
 
-void run_stage(kg_solver* h, int kind, const kg::StageLaunch& L) {
+// whether the stage wrote its ghost values itself
+bool run_stage(kg_solver* h, int kind, const kg::StageLaunch& L) {
   Prof pf(h, kind, 1);
   const double* rsg = h->dmet + (size_t)T_RSG * h->NJ * h->PI;
-  if (h->variant >= 2 && kg::launch_stage_tma(kind, L, rsg, h->derr, h->stream, h->tile_rows) == 0) return;
+  if (h->variant >= 2 && kg::launch_stage_tma(kind, L, rsg, h->derr, h->stream, h->tile_rows) == 0)
+    return L.ghosts != kg::GH_FILL;
   if (h->variant >= 1)
     kg::launch_stage_march(kind, L, rsg, h->stream);
   else
     kg::launch_stage(kind, L, h->stream);
+  return false;
+}
+
+// Who writes the ghost values of the RK stages that start from u as it is now: the
+// stages themselves on a state with filled seam planes and on grids below the pairs'
+// size, where the fill's launch behind each stage counts; on larger ones the
+// scattered stores cost as much as the fill.  us per RK4 step, fills / by the
+// stages: 40 x 9 x 17 37 / 24, 64 x 17 x 33 46 / 33, 256 x 17 x 33 68 / 53, 128 x 33 x 65
+// 111 / 101; in the paired and the mixed kernels, whose registers are full, it was
+// slower at every size (1024 x 65 x 129 1658 / 1938, mixed 1617 / 1663).
+int ghosts_by(const kg_solver* h) {
+  if (h->variant < 2 || !h->seam_filled || kg::rk4_pairs_pay(h->g)) return kg::GH_FILL;
+  return h->p.bc_rmax == KG_INFLOW ? kg::GH_INFLOW : kg::GH_OUTFLOW;
 }
 
 // KG_ETIMEOUT if a kernel reported a bounded wait that ran out (flag is sticky)
@@ -896,6 +911,11 @@ void run_ghost(kg_solver* h, double2* u, const double2* up, int inflow, bool fac
 void shell_reduce(kg_solver* h, bool alm, bool flux, cudaStream_t st) {
   kg::launch_shell_reduce(h->shells, h->si.active, h->n_det, h->L, h->Ny, h->Nz, h->normP, h->cosm, h->sinm, h->sint,
                           h->dy * h->dz, alm ? h->alm : nullptr, flux ? h->flux : nullptr, st);
+}
+
+// an RK stage with the ghost values of its output
+void run_rk_stage(kg_solver* h, int kind, const kg::StageLaunch& L, int inflow) {
+  if (!run_stage(h, kind, L)) run_ghost(h, L.out, h->U, inflow);
 }
 
 kg::StageLaunch base_launch(kg_solver* h) {
@@ -1156,19 +1176,17 @@ int step_rk3(kg_solver* h, int nsteps) {
   for (int s = 0; s < nsteps; ++s) {
     kg::StageLaunch L = base_launch(h);
     L.base = h->U;
+    L.ghosts = ghosts_by(h);
     set_in(L, g, h->U, fld(h->U, g, 4));
     L.out = R1;
-    run_stage(h, kg::ST_RK3_1, L);
-    run_ghost(h, R1, h->U, inflow);
+    run_rk_stage(h, kg::ST_RK3_1, L, inflow);
     set_in(L, g, R1, fld(R1, g, 4));
     L.out = R2;
-    run_stage(h, kg::ST_RK3_2, L);
-    run_ghost(h, R2, h->U, inflow);
+    run_rk_stage(h, kg::ST_RK3_2, L, inflow);
     set_in(L, g, R2, fld(R2, g, 4));
     L.out = h->U;
     L.skip_last_i = inflow;
-    run_stage(h, kg::ST_RK3_3, L);
-    run_ghost(h, h->U, h->U, inflow);
+    run_rk_stage(h, kg::ST_RK3_3, L, inflow);
     h->t = h->t + h->dt;
   }
   KG_CK(cudaGetLastError());
@@ -1184,24 +1202,21 @@ void rk4_step_single(kg_solver* h) {
   double2* A = h->RK[2];
   kg::StageLaunch L = base_launch(h);
   L.base = h->U;
+  L.ghosts = ghosts_by(h);
   L.acc = A;
   set_in(L, g, h->U, fld(h->U, g, 4));
   L.out = R1;
-  run_stage(h, kg::ST_RK4_1, L);
-  run_ghost(h, R1, h->U, inflow);
+  run_rk_stage(h, kg::ST_RK4_1, L, inflow);
   set_in(L, g, R1, fld(R1, g, 4));
   L.out = R2;
-  run_stage(h, kg::ST_RK4_2, L);
-  run_ghost(h, R2, h->U, inflow);
+  run_rk_stage(h, kg::ST_RK4_2, L, inflow);
   set_in(L, g, R2, fld(R2, g, 4));
   L.out = R1;
-  run_stage(h, kg::ST_RK4_3, L);
-  run_ghost(h, R1, h->U, inflow);
+  run_rk_stage(h, kg::ST_RK4_3, L, inflow);
   set_in(L, g, R1, fld(R1, g, 4));
   L.out = h->U;
   L.skip_last_i = inflow;
-  run_stage(h, kg::ST_RK4_4, L);
-  run_ghost(h, h->U, h->U, inflow);
+  run_rk_stage(h, kg::ST_RK4_4, L, inflow);
   h->t = h->t + h->dt;
 }
 
@@ -1515,7 +1530,7 @@ int run_steps(kg_solver* h, int which, int nsteps, int (*step)(kg_solver*, int))
   if (!h || nsteps < 0) return KG_EINVAL;
   int rc;
   if (nsteps < 2 || !h->use_graphs || h->prof_on) return step(h, nsteps);
-  if (which == 3 && !h->seam_filled && wants_pairs(h)) {  // the graph holds the paired form
+  if ((which == 2 || which == 3) && !h->seam_filled) {  // the RK graphs hold stages that rely on filled seam planes
     if ((rc = step(h, 1))) return rc;
     if (--nsteps < 2) return nsteps ? step(h, nsteps) : KG_OK;
   }

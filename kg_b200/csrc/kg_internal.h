@@ -79,6 +79,10 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
 // until the kernel before this one has finished and its writes are visible
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// who writes a stage's ghost values: a fill behind it, or the stage itself
+// (kg_ghost.cuh) with the outer r column copied (outflow) or held (inflow)
+enum GhostBy { GH_FILL = 0, GH_OUTFLOW, GH_INFLOW };
+
 struct StageLaunch {
   Grid g;
   Metric m;
@@ -90,6 +94,7 @@ struct StageLaunch {
   double2* out4;
   double2* acc;
   int skip_last_i;
+  int ghosts;  // GhostBy; the TMA form of the RK stages only
 };
 
 void launch_stage(int kind, const StageLaunch& L, cudaStream_t st);

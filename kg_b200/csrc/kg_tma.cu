@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 #include <cstring>
 #include "kg_device.cuh"
+#include "kg_ghost.cuh"
 #include "kg_internal.h"
 #include "kg_tma_ops.cuh"
 
@@ -79,6 +80,11 @@ template <int KIND>
 constexpr __host__ __device__ bool filled_kind() {
   return KIND != ST_P2_S1A && KIND != ST_P3_S2A && KIND != ST_P2_S1B && KIND != ST_P3_S2B;
 }
+// the RK stages can write the ghost values themselves (kg_ghost.cuh)
+template <int KIND>
+constexpr __host__ __device__ bool copies_kind() {
+  return filled_kind<KIND>() && KIND != ST_P2_S2 && KIND != ST_P3_S3;
+}
 // theta rows [row_first, row_end) and phi planes [0, plane_end) that a stage computes
 template <int KIND>
 constexpr __host__ __device__ int row_first() {
@@ -104,6 +110,7 @@ struct TmaArgs {
   double2* out4;
   double2* acc;
   int skip_last_i;
+  int ghosts;   // GH_FILL, GH_OUTFLOW or GH_INFLOW
   int kchunk;
   int* err;
   int npf;      // number of prefetch maps in use (0..2)
@@ -126,7 +133,7 @@ struct alignas(64) BatchItem {
 template <int KIND, int MK, int TJ>
 __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtensorMap* tm1p, const CUtensorMap* tp0p,
                                           const CUtensorMap* tp1p, const TmaArgs& a, int bx, int by, int bz,
-                                          double* ring, double* mt, uint64_t* bars, uint32_t tb) {
+                                          double* ring, double* mt, uint64_t* bars, uint32_t tb, int ghosts) {
   using GT = Geom<TJ>;
   constexpr int FIELD_D = GT::FIELD_D, STAGE_D = GT::STAGE_D, STAGE_B = GT::STAGE_B, MT_N = GT::MT_N;
   constexpr bool PSI = (KIND != ST_P2_S1B && KIND != ST_P3_S2B);
@@ -139,16 +146,18 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TI + tx;
   const int ii0 = bx * TI, jj0 = row_first<KIND>() + by * TJ;
   const int ii = ii0 + tx, jj = jj0 + ty;
-  const bool act = (ii < g.NI) && (jj < row_end<KIND>(g));
+  // with the ghost values written here, the outer copy is stored by column NI-2
+  const bool copies = copies_kind<KIND>() && ghosts != GH_FILL;
+  const bool act = (ii < g.NI) && (jj < row_end<KIND>(g)) && !(copies && ghosts == GH_OUTFLOW && ii == g.NI - 1);
   // ring slot protocol: full[s] (bars[s]) completes when a plane's boxes have
   // landed; empty[s] when all eight warps have read the plane for the last
   // time, after which thread 0 may load the next plane into the slot, so the
   // warps are not held at a block barrier per plane
   uint64_t* empty = bars + NST;
   const int lane = tid & 31;
-  const int k0 = bz * a.kchunk;
-  if (k0 >= plane_end<KIND>(g)) return 0;
-  const int k1 = min(k0 + a.kchunk, plane_end<KIND>(g));
+  const int k1 = min((bz + 1) * a.kchunk, plane_end<KIND>(g));
+  const int k0 = max(bz * a.kchunk, copies ? 1 : 0);  // plane 0 is a copy then
+  if (k0 >= k1) return 0;
   const int nplanes = (k1 - k0) + 2;  // previous, the chunk, next
   auto plane_of = [&](int t) -> int {
     if (t == 0) return (k0 == 0) ? g.Nz - 2 : k0 - 1;
@@ -276,6 +285,7 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
         const bool okn = okc && mbar_wait_bounded(&bars[slot(tn)], parity(tn));
         if (!okn) timed_out = 1;
       }
+      if (!FAST && copies_kind<KIND>()) timed_out = __any_sync(0xffffffffu, timed_out) ? 1 : 0;  // ahead of shuffles
       if (act && !timed_out) {
         const double* cu = ring + (size_t)slot(tc) * STAGE_D;
         const double* nx = ring + (size_t)slot(tn) * STAGE_D;
@@ -400,7 +410,7 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
           a.out4[p] = cadd(bv[4], rmul(dt, r[4]));
         } else if (KIND == ST_P3_S2B) {
           a.out4[p] = cadd(rmul(0.75, bv[4]), rmul(0.25, cadd(lds(a.aux4, p), rmul(dt, r[4]))));
-        } else if (!(a.skip_last_i && ii == n)) {
+        } else {
 #pragma unroll
           for (int v = 0; v < 5; ++v) {
             const long long o = v * g.fs + p;
@@ -432,7 +442,34 @@ __device__ __forceinline__ int stage_item(const CUtensorMap* tm4p, const CUtenso
               const double2 kk = rmul(dt, r[v]);
               res = cadd(b, cdivm(cadd(sv[v], kk), 6.0, kSixth));
             }
-            a.out[o] = res;
+            if (copies_kind<KIND>()) r[v] = res;
+            if (FAST || (!copies && !(a.skip_last_i && ii == n))) a.out[o] = res;
+          }
+          if (copies_kind<KIND>()) {
+            bool next = false;
+            if (!FAST && copies) {
+              if (ii0 == 0 && tx < 4) {  // the excision column, from its neighbours' results
+#pragma unroll
+                for (int v = 0; v < 5; ++v) {
+                  auto lane_of = [&](int l) {
+                    return c2(__shfl_sync(0xfu, r[v].x, l), __shfl_sync(0xfu, r[v].y, l));
+                  };
+                  const double2 u1 = lane_of(1), u2 = lane_of(2), u3 = lane_of(3);
+                  if (tx == 0) r[v] = cadd(csub(rmul(3.0, u1), rmul(3.0, u2)), u3);
+                }
+              }
+              next = ghosts == GH_OUTFLOW && ii == n - 1;
+              if (ghosts == GH_INFLOW && ii == n) {  // held: u^n (an in-place stage stores what is there)
+#pragma unroll
+                for (int v = 0; v < 5; ++v) r[v] = bv[v];
+              }
+#pragma unroll
+              for (int v = 0; v < 5; ++v) {
+                a.out[v * g.fs + p] = r[v];
+                if (next) a.out[v * g.fs + p + 1] = r[v];
+              }
+            }
+            if (copies && has_copies(g, jj, k)) store_copies(g, a.out, ii, jj, k, r, next);
           }
         }
         Epv = Ecu;
@@ -491,7 +528,8 @@ __global__ void __launch_bounds__(TI * TJ, Geom<TJ>::MIN_BLOCKS)
   double* mt = ring + (size_t)NST * Geom<TJ>::STAGE_D;
   uint64_t* bars = reinterpret_cast<uint64_t*>(mt + (size_t)MT_COUNT * Geom<TJ>::MT_N);
   init_ring_barriers<TJ>(bars);
-  (void)stage_item<KIND, MK, TJ>(&tm4, &tm1, &tp0, &tp1, a, blockIdx.x, blockIdx.y, blockIdx.z, ring, mt, bars, 0u);
+  (void)stage_item<KIND, MK, TJ>(&tm4, &tm1, &tp0, &tp1, a, blockIdx.x, blockIdx.y, blockIdx.z, ring, mt, bars, 0u,
+                                   a.ghosts);
 }
 
 // ---- persistent kernel over many solves -------------------------------------
@@ -531,7 +569,8 @@ __global__ void __launch_bounds__(TI * TJ, Geom<TJ>::MIN_BLOCKS)
     __syncthreads();
     next = s_next;
     const BatchItem& B = solves[s_solve];
-    const int used = stage_item<KIND, MK, TJ>(&B.tm4, &B.tm1, &B.tp0, &B.tp1, sa, s_bx, s_by, s_bz, ring, mt, bars, tb);
+    const int used = stage_item<KIND, MK, TJ>(&B.tm4, &B.tm1, &B.tp0, &B.tp1, sa, s_bx, s_by, s_bz, ring, mt, bars, tb,
+                                                   GH_FILL);  // one fill for the whole batch follows
     if (used < 0) break;
     tb += (uint32_t)used;
     __syncthreads();  // sa and the item indices are rewritten for the next item
@@ -663,6 +702,7 @@ int build_batch_item(void* dst, int kind, const StageLaunch& L, const double* rs
   a.out4 = L.out4;
   a.acc = L.acc;
   a.skip_last_i = L.skip_last_i;
+  a.ghosts = L.ghosts;
   a.kchunk = kchunk;
   a.err = err;
   a.npf = npf;
@@ -777,6 +817,7 @@ int launch_stage_tma(int kind, const StageLaunch& L, const double* rsg, int* err
   a.out4 = L.out4;
   a.acc = L.acc;
   a.skip_last_i = L.skip_last_i;
+  a.ghosts = L.ghosts;
   a.kchunk = 0;  // set at the launch, from the tiles of the grid
   a.err = err;
   a.npf = npf;

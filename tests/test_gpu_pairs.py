@@ -16,13 +16,13 @@ GRIDS = [dict(Nx=16, Ny=9, Nz=17, xmin=1.8, xmax=12.0),     # one tile, partial 
          dict(Nx=92, Ny=26, Nz=9, xmin=1.8, xmax=30.0)]
 
 
-def _pair(g, metric="Kerr_Schild", bc="outflow"):
+def _pair(g, metric="Kerr_Schild", bc="outflow", pairs=2):
     from kg_b200 import ScalarField
     from kg_b200.initial_data import shell_ylm
     from oracle.oracle import Oracle, KERR_SCHILD, SCHW_EF, OUTFLOW, INFLOW
     dev = ScalarField(g["Nx"], g["Ny"], g["Nz"], g["xmin"], g["xmax"], 0.25, m=0.3, metric=metric,
                       boundary_type_rmax=bc)
-    dev._ck(dev._lib.kg_set_rk4_pairs(dev.handle, 2))
+    dev._ck(dev._lib.kg_set_rk4_pairs(dev.handle, pairs))
     ora = Oracle(g["Nx"], g["Ny"], g["Nz"], g["xmin"], g["xmax"], CFL=0.25, m=0.3,
                  metric=KERR_SCHILD if metric == "Kerr_Schild" else SCHW_EF,
                  bc_rmax=OUTFLOW if bc == "outflow" else INFLOW)
@@ -43,10 +43,12 @@ def test_paired_rk4_bitexact(grid, metric, bc):
         assert np.array_equal(dev.u, ora.get_state())
 
 
-def test_paired_rk4_after_other_writers_of_u():
+@pytest.mark.parametrize("pairs", [2, 0])  # 0: the stages that store their own ghost values
+@pytest.mark.parametrize("bc", ["outflow", "inflow"])
+def test_rk4_after_other_writers_of_u(pairs, bc):
     """states whose seam planes no fill has left: set anew, one face filled alone,
     another stepper in between"""
-    dev, ora, u0 = _pair(GRIDS[3])
+    dev, ora, u0 = _pair(GRIDS[3], bc=bc, pairs=pairs)
     rng = np.random.default_rng(5)
     dev.rk4(nsteps=5)
     ora.rk4(5)
@@ -66,6 +68,8 @@ def test_paired_rk4_after_other_writers_of_u():
     ora.set_state(s)
     dev.rk4(nsteps=3)
     ora.rk4(3)
+    dev.rk3(nsteps=2)
+    ora.rk3(2)
     assert np.array_equal(dev.u, ora.get_state())
 
 
