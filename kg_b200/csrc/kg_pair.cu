@@ -43,9 +43,13 @@
 // barrier).  On 1024 x 65 x 129, pair 0 / pair 1 in us: tiles of 4 rows, two CTAs per
 // SM 809 / 1099; 8 rows 787 / 990; with Y's products with the metric formed once by
 // their own point instead of by each neighbour, and the increment sum parked in
-// shared memory, 668 / 828 (this form).  Stage kernels with their fills: 1020 and
-// 1089.  Peeling the march into copies per warp role ran 781 / 993 (instruction
-// fetch), the second right-hand side ahead of the Y stores 736 / 1039.
+// shared memory, 697 / 867; with u parked too (pair 0) or read again where it is
+// used (pair 1), so that little spills, 686 / 864 (301 x 46 x 90: 141 / 186 -> 137 /
+// 175).  Stage kernels with their fills: 1020 and 1089.  Measured and not kept: the
+// march in copies per warp role 781 / 993 (instruction fetch), the second right-hand
+// side ahead of the Y stores 736 / 1039, tiles of 10 rows 712 / 1033, pair 1's u
+// parked 686 / 896 or in registers 686 / 934, ghost values stored by the pairs
+// instead of a fill (a whole step 1658 -> 1938).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include "kg_device.cuh"
@@ -64,16 +68,33 @@ enum { PT_AL = 0, PT_BE, PT_A, PT_GRR, PT_GRP, PT_SG, PT_HT, PT_COUNT };
 // difference, each formed once by its own point
 enum { Y_P1 = 0, Y_AP, Y_E, Y_G, Y_H, Y_Q, Y_COUNT };
 
+// Shared memory of a tile with TJ own rows.  Of the Y planes and the metric tables
+// only E, H and alpha, beta, (alpha sqrtg) gamma^thth are read beyond the own (the
+// region's) rows.
 template <int TJ>
 struct PGeom {
   static constexpr int WARPS = TJ + 2, ROWS = TJ + 4;
-  static constexpr int FIELD = ROWS * PW;                  // complex values per variable and plane
-  static constexpr int SLOT_B = 5 * FIELD * 16;            // bytes of a ring slot
-  static constexpr int SLOT = (SLOT_B + 127) / 128 * 128;
-  static constexpr int Y_N = WARPS * 32;                   // points of a Y plane
-  static constexpr int PARK_N = TJ * 32;                   // own points, by thread
-  static constexpr size_t SMEM = (size_t)PST * SLOT + 2 * (size_t)Y_COUNT * Y_N * 16 + (size_t)5 * PARK_N * 16 +
-                                 (size_t)PT_COUNT * FIELD * 8 + 64 + 128;
+  static constexpr int FULL = ROWS * PW, PART = WARPS * PW;  // complex values per variable and plane
+  static constexpr uint32_t TX_B = 5 * FULL * 16;            // bytes of a plane's box
+  static constexpr int SLOT = (TX_B + 127) / 128 * 128;
+  static constexpr int Y_WIDE = WARPS * 32, Y_OWN = TJ * 32;  // points of a Y array: region rows, own rows
+  // a Y plane: E and H on the region's rows, then the other four on the own rows
+  static __host__ __device__ constexpr int y_at(int w) {
+    return w == Y_E ? 0 : w == Y_H ? Y_WIDE : 2 * Y_WIDE + (w == Y_P1 ? 0 : w == Y_AP ? 1 : w == Y_G ? 2 : 3) * Y_OWN;
+  }
+  static constexpr int Y_PLANE = 2 * Y_WIDE + 4 * Y_OWN;
+  static constexpr int PARK_N = TJ * 32;  // own points, by thread
+  // metric tables: alpha, beta, H factor with the row halo, the others on the region's rows
+  static __host__ __device__ constexpr bool m_full(int t) { return t == PT_AL || t == PT_BE || t == PT_HT; }
+  static __host__ __device__ constexpr int m_at(int t) {
+    return t == PT_AL ? 0
+         : t == PT_BE ? FULL
+         : t == PT_HT ? 2 * FULL
+                      : 3 * FULL + (t == PT_A ? 0 : t == PT_GRR ? 1 : t == PT_GRP ? 2 : 3) * PART;
+  }
+  static constexpr int M_ALL = 3 * FULL + 4 * PART;
+  static constexpr size_t SMEM =
+      (size_t)PST * SLOT + 2 * (size_t)Y_PLANE * 16 + (size_t)10 * PARK_N * 16 + (size_t)M_ALL * 8 + 64 + 128;
   static_assert(SMEM <= 227 * 1024, "one CTA per SM");
 };
 
@@ -248,9 +269,9 @@ __global__ void __launch_bounds__(PGeom<TJ>::WARPS * 32, 1)
     ring = smem_raw + ((128u - (b & 127u)) & 127u);
   }
   double2* ybuf = reinterpret_cast<double2*>(ring + (size_t)PST * GT::SLOT);  // 2 planes of products
-  double2* park = ybuf + 2 * Y_COUNT * GT::Y_N;  // increment sum at P[s-1], by own thread
-  double* mt = reinterpret_cast<double*>(park + 5 * GT::PARK_N);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(mt + PT_COUNT * GT::FIELD);
+  double2* park = ybuf + 2 * GT::Y_PLANE;  // increment sum and u at P[s-1], by own thread
+  double* mt = reinterpret_cast<double*>(park + 10 * GT::PARK_N);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(mt + GT::M_ALL);
   const Grid& g = a.g;
   const Metric& M = a.m;
   const int lane = threadIdx.x, w = threadIdx.y, tid = w * 32 + lane;
@@ -271,7 +292,7 @@ __global__ void __launch_bounds__(PGeom<TJ>::WARPS * 32, 1)
   __syncthreads();
   auto issue = [&](int t) {
     uint64_t* b = &bars[t % PST];
-    mbar_expect_tx(b, GT::SLOT_B);
+    mbar_expect_tx(b, GT::TX_B);
     tma_load_4d(ring + (size_t)(t % PST) * GT::SLOT, &tmX, 2 * (i0 - 4), j0 - 2, plane_of(t), 0, b);
   };
   // the point-wise operands of a plane, pulled into L2 ahead of their loads
@@ -288,17 +309,20 @@ __global__ void __launch_bounds__(PGeom<TJ>::WARPS * 32, 1)
     prefetch(1);
     prefetch(2);
   }
-  for (int t = tid; t < GT::FIELD; t += GT::WARPS * 32) {
-    const int gi = i0 - 4 + t % PW, gj = j0 - 2 + t / PW;
+  for (int t = tid; t < GT::FULL; t += GT::WARPS * 32) {
+    const int row = t / PW, gi = i0 - 4 + t % PW, gj = j0 - 2 + row;
     const bool in = gi >= 0 && gi < g.NI && gj < g.NJ;
     const int q = in ? off2(g, gi, gj) : 0;
-    mt[PT_AL * GT::FIELD + t] = in ? ldm(M.alpha, q) : 0.0;
-    mt[PT_BE * GT::FIELD + t] = in ? ldm(M.beta, q) : 0.0;
-    mt[PT_A * GT::FIELD + t] = in ? ldm(MK == MK_KS ? M.asg : M.asg_grr, q) : 0.0;
-    mt[PT_GRR * GT::FIELD + t] = in ? ldm(M.grr, q) : 0.0;
-    mt[PT_GRP * GT::FIELD + t] = in ? ldm(M.grp, q) : 0.0;
-    mt[PT_SG * GT::FIELD + t] = in ? ldm(M.sqrtg, q) : 0.0;
-    mt[PT_HT * GT::FIELD + t] = in ? ldm(M.asg_gtt, q) : 0.0;
+    mt[GT::m_at(PT_AL) + t] = in ? ldm(M.alpha, q) : 0.0;
+    mt[GT::m_at(PT_BE) + t] = in ? ldm(M.beta, q) : 0.0;
+    mt[GT::m_at(PT_HT) + t] = in ? ldm(M.asg_gtt, q) : 0.0;
+    if (row >= 1 && row <= GT::WARPS) {
+      const int u = t - PW;
+      mt[GT::m_at(PT_A) + u] = in ? ldm(MK == MK_KS ? M.asg : M.asg_grr, q) : 0.0;
+      mt[GT::m_at(PT_GRR) + u] = in ? ldm(M.grr, q) : 0.0;
+      mt[GT::m_at(PT_GRP) + u] = in ? ldm(M.grp, q) : 0.0;
+      mt[GT::m_at(PT_SG) + u] = in ? ldm(M.sqrtg, q) : 0.0;
+    }
   }
   Own o = {0, 0, 0, 1, 1, 0, 0, 0, 0};
   if (vcol && jj < g.NJ) {
@@ -321,25 +345,27 @@ __global__ void __launch_bounds__(PGeom<TJ>::WARPS * 32, 1)
   const long long pcol = form ? off3(g, ii, jj, 0) : 0;
   const long long ps = (long long)g.NK * g.PI;  // variable stride of the pole rows
   const double2* pole = a.pole + (jj == 2 ? 0 : 5 * ps) + ii;
-  auto XS = [&](int t) { return reinterpret_cast<const double2*>(ring + (size_t)(t % PST) * GT::SLOT); };
-  const int xo = (w + 1) * PW + lane + 2;  // own point in a ring slot and in the metric tile
-  auto MT = [&](int which, int dx, int dy) { return mt[which * GT::FIELD + xo + dy * PW + dx]; };
+  // variable v of X's plane t at an offset from the own point
+  auto XV = [&](int t, int v, int dx, int dy) -> double2 {
+    return reinterpret_cast<const double2*>(ring + (size_t)(t % PST) * GT::SLOT)[v * GT::FULL + (w + 1 + dy) * PW +
+                                                                                  lane + 2 + dx];
+  };
+  auto MT = [&](int which, int dx, int dy) {
+    return mt[GT::m_at(which) + (w + (GT::m_full(which) ? 1 : 0) + dy) * PW + lane + 2 + dx];
+  };
   const double dt = g.dt;
 
   int timed_out = 0;
   if (!mbar_wait_bounded(&bars[0], 0u) || !mbar_wait_bounded(&bars[1], 0u)) timed_out = 1;
   double2 Ep = c2(0, 0), Ec = Ep, Fp = Ep, Fc = Ep;          // X's phi arguments at P[s-1], P[s]
   double2 Yep = Ep, Yec = Ep, Yfp = Ep, Yfc = Ep;            // Y's at P[s-2], P[s-1]
-  double2 uo[5], yphi = Ep, ypi = Ep;                        // u and Y's phi and Pi at P[s-1]
-#pragma unroll
-  for (int v = 0; v < 5; ++v) uo[v] = c2(0, 0);
+  double2 yphi = Ep, ypi = Ep;                               // Y's phi and Pi at P[s-1]
   park += own ? (w - 1) * 32 + lane : 0;
   if (!timed_out) {
-    const double2 *x0 = XS(0) + xo, *x1 = XS(1) + xo;
-    Ep = arg_e<MK>(o, x0[GT::FIELD], x0[4 * GT::FIELD]);
-    Fp = arg_f<MK>(o, x0[GT::FIELD], x0[3 * GT::FIELD]);
-    Ec = arg_e<MK>(o, x1[GT::FIELD], x1[4 * GT::FIELD]);
-    Fc = arg_f<MK>(o, x1[GT::FIELD], x1[3 * GT::FIELD]);
+    Ep = arg_e<MK>(o, XV(0, 1, 0, 0), XV(0, 4, 0, 0));
+    Fp = arg_f<MK>(o, XV(0, 1, 0, 0), XV(0, 3, 0, 0));
+    Ec = arg_e<MK>(o, XV(1, 1, 0, 0), XV(1, 4, 0, 0));
+    Fc = arg_f<MK>(o, XV(1, 1, 0, 0), XV(1, 3, 0, 0));
   }
   bool failed = __syncthreads_or(timed_out) != 0;
   const bool fast = __all_sync(0xffffffffu, form && ii >= 2 && ii <= g.NI - 3 && o.be > 0.0);
@@ -362,9 +388,7 @@ __global__ void __launch_bounds__(PGeom<TJ>::WARPS * 32, 1)
 #pragma unroll
       for (int v = 0; v < 5; ++v) un[v] = kn[v] = y[v] = c2(0, 0);
       if (form && !timed_out) {
-        const double2* x = XS(s) + xo;
-        const double2* xn = XS(s + 1) + xo;
-        auto RF = [&](int v, int dx, int dy) { return x[v * GT::FIELD + dy * PW + dx]; };
+        auto RF = [&](int v, int dx, int dy) { return XV(s, v, dx, dy); };
         if (PAIR == 0) {
 #pragma unroll
           for (int v = 0; v < 5; ++v) un[v] = RF(v, 0, 0);
@@ -372,8 +396,8 @@ __global__ void __launch_bounds__(PGeom<TJ>::WARPS * 32, 1)
 #pragma unroll
           for (int v = 0; v < 5; ++v) un[v] = lds(a.base, v * fs + p);
         }
-        const double2 En = arg_e<MK>(o, xn[GT::FIELD], xn[4 * GT::FIELD]);
-        const double2 Fn = arg_f<MK>(o, xn[GT::FIELD], xn[3 * GT::FIELD]);
+        const double2 En = arg_e<MK>(o, XV(s + 1, 1, 0, 0), XV(s + 1, 4, 0, 0));
+        const double2 Fn = arg_f<MK>(o, XV(s + 1, 1, 0, 0), XV(s + 1, 3, 0, 0));
         double2 r[5];
         pair_rhs<FAST, MK>(g, o, ii, RF, MT, RF(0, 0, 0), Ep, En, Fp, Fn, r);
 #pragma unroll
@@ -420,40 +444,49 @@ __global__ void __launch_bounds__(PGeom<TJ>::WARPS * 32, 1)
       // Y's products with the metric at this point
       const double2 ap = rmul(o.al, y[4]);
       const double2 Yen = cadd(ap, rmul(o.be, y[1])), Yfn = arg_f<MK>(o, y[1], y[3]);
-      double2* yb = ybuf + (size_t)(s & 1) * Y_COUNT * GT::Y_N + tid;
-      yb[Y_P1 * GT::Y_N] = y[1];
-      yb[Y_AP * GT::Y_N] = ap;
-      yb[Y_E * GT::Y_N] = Yen;
-      yb[Y_G * GT::Y_N] =
-          MK == MK_KS ? rmul(MT(PT_A, 0, 0), cadd(rmul(MT(PT_GRR, 0, 0), y[1]), rmul(MT(PT_GRP, 0, 0), y[3])))
-                      : rmul(MT(PT_A, 0, 0), y[1]);
-      yb[Y_H * GT::Y_N] = rmul(MT(PT_HT, 0, 0), y[2]);
-      yb[Y_Q * GT::Y_N] = rmul(o.sg, y[4]);
+      double2* yb = ybuf + (size_t)(s & 1) * GT::Y_PLANE + tid;
+      yb[GT::y_at(Y_E)] = Yen;
+      yb[GT::y_at(Y_H)] = rmul(MT(PT_HT, 0, 0), y[2]);
+      if (w >= 1 && w <= TJ) {
+        yb -= 32;  // arrays of the own rows
+        yb[GT::y_at(Y_P1)] = y[1];
+        yb[GT::y_at(Y_AP)] = ap;
+        yb[GT::y_at(Y_G)] =
+            MK == MK_KS ? rmul(MT(PT_A, 0, 0), cadd(rmul(MT(PT_GRR, 0, 0), y[1]), rmul(MT(PT_GRP, 0, 0), y[3])))
+                        : rmul(MT(PT_A, 0, 0), y[1]);
+        yb[GT::y_at(Y_Q)] = rmul(o.sg, y[4]);
+      }
       // the second right-hand side on the own points of P[s-1]
       if (own && s >= 3 && !timed_out) {
         const long long pm = pcol + (long long)plane_of(s - 1) * g.plane;
-        const double2* ym = ybuf + (size_t)((s - 1) & 1) * Y_COUNT * GT::Y_N + tid;
-        auto Y = [&](int v, int dx, int dy) { return ym[v * GT::Y_N + dy * 32 + dx]; };
-        double2 r[5];
+        const double2* ym = ybuf + (size_t)((s - 1) & 1) * GT::Y_PLANE + tid;
+        auto Y = [&](int v, int dx, int dy) {
+          return ym[GT::y_at(v) - (v == Y_E || v == Y_H ? 0 : 32) + dy * 32 + dx];
+        };
+        double2 r[5], ul[5];
+        if (PAIR == 1)
+#pragma unroll
+          for (int v = 0; v < 5; ++v) ul[v] = lds(a.base, v * fs + pm);
         pair_rhs_y<FAST>(g, o, ii, MK == MK_KS, Y, yphi, ypi, Yep, Yen, Yfp, Yfn, r);
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
           const long long q = v * fs + pm;
-          const double2 kk = rmul(dt, r[v]), ko = park[v * GT::PARK_N];
+          const double2 kk = rmul(dt, r[v]), ko = park[v * GT::PARK_N], uo = PAIR == 0 ? park[(5 + v) * GT::PARK_N] : ul[v];
           if (PAIR == 0) {
             a.acc_out[q] = cadd(ko, rmul(2.0, kk));
-            a.out[q] = cadd(uo[v], rmul(0.50, kk));
+            a.out[q] = cadd(uo, rmul(0.50, kk));
           } else {
-            a.out[q] = cadd(uo[v], pcdiv(cadd(ko, kk), 6.0, 1.0 / 6.0));
+            a.out[q] = cadd(uo, pcdiv(cadd(ko, kk), 6.0, 1.0 / 6.0));
           }
         }
       }
       if (own) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) park[v * GT::PARK_N] = PAIR == 1 ? cadd(an[v], rmul(2.0, kn[v])) : kn[v];
+        for (int v = 0; v < 5; ++v) {
+          park[v * GT::PARK_N] = PAIR == 1 ? cadd(an[v], rmul(2.0, kn[v])) : kn[v];
+          if (PAIR == 0) park[(5 + v) * GT::PARK_N] = un[v];
+        }
       }
-#pragma unroll
-      for (int v = 0; v < 5; ++v) uo[v] = un[v];
       yphi = y[0];
       ypi = y[4];
       Yep = Yec;
