@@ -13,6 +13,7 @@
 // `face` launches run one reference routine at a time (parity hook).
 #include "kg_device.cuh"
 #include "kg_internal.h"
+#include "kg_refine.cuh"
 
 namespace kg {
 
@@ -40,145 +41,243 @@ __device__ __forceinline__ int ghost_src_row(const Grid& g, int jj) {
 // No point that a unit reads is written by another one, with one exception: the
 // partner of plane kp = Nz - 1 - Nz/2 is plane 0, so the ghost rows of kp take
 // rows 3..5 and NJ-6..NJ-4 of plane 0 as the stage left them, and C overwrites
-// those rows.  The C unit of such a row therefore writes kp's ghost rows first
-// and the row itself behind a block barrier (A leaves plane kp out).
+// those rows.  The C unit of such a row therefore reads it as well as its own
+// source, and writes both copies behind a block barrier (A leaves plane kp out).
 // What bounds it: on small grids the launch and the latency of one load-store
 // chain per thread, so one launch replaces the former two (ghost rows and faces,
 // then the phi planes); on large ones memory, 2 x 80 B per point of the ghost rows.
 // Event-timed, two launches before and one after: 301 x 46 x 90 21.5 -> 17.1 us,
 // 1024 x 65 x 129 43.1 -> 33.9 us (FP32 states 37.4 -> 22.1 us).  With the x faces
 // apart (PIRK2) 64 x 17 x 33 13.0 -> 12.1 us, 2048 x 129 x 257 123.8 -> 119.9 us.
-template <class T>
-__device__ __forceinline__ T xval_t(const Grid& g, const T* u, const double2* up, int inflow, int ii, int jj, int k);
-template <>
-__device__ __forceinline__ double2 xval_t<double2>(const Grid& g, const double2* u, const double2* up, int inflow,
-                                                   int ii, int jj, int k) {
-  return xval(g, u, up, inflow, ii, jj, k);
+//
+// On a refined level the outermost planes then take the coarser level's values
+// (kg_refine.cuh): with WithProlong the same launch writes those instead, in A and C
+// for the ghost rows and planes 0 and Nz and in B for the interior rows (one launch
+// in the place of two: 384 x 33 x 65, four columns, 12.6 + 13.3 -> 17.9 us).  No
+// unit reads these columns: the x fill of the outermost one falls away.
+//
+// A thread requests all that it reads before it stores any of it, and the rows of
+// plane 0 read both their sources before either is written: one or two round trips
+// to memory a unit, where there were up to four (301 x 46 x 90: 17.9 -> 13.8 us with the rows shared out).
+// Rows longer than a block are shared among blocks (row_parts).
+
+// excision extrapolation 3 u1 - 3 u2 + u3; FP32 stage states form it in FP64
+__device__ __forceinline__ double2 excise(double2 a, double2 b, double2 c) {
+  return cadd(csub(rmul(3.0, a), rmul(3.0, b)), c);
 }
-// FP32 stage states: the excision extrapolation is formed in FP64, the inflow
-// hold reads u^n (FP64)
-template <>
-__device__ __forceinline__ float2 xval_t<float2>(const Grid& g, const float2* u, const double2* up, int inflow, int ii,
-                                                 int jj, int k) {
+__device__ __forceinline__ float2 excise(float2 a, float2 b, float2 c) {
+  const double2 e = excise(c2(a.x, a.y), c2(b.x, b.y), c2(c.x, c.y));
+  return make_float2((float)e.x, (float)e.y);
+}
+__device__ __forceinline__ void hold(double2 v, double2& o) { o = v; }
+__device__ __forceinline__ void hold(double2 v, float2& o) { o = make_float2((float)v.x, (float)v.y); }
+
+template <class T>
+struct Fill {
+  T* u;
+  const double2* up;
+  int inflow;
+  int cyclic;  // plane 0 was not computed and stands for plane Nz-1
+};
+
+// the values of row (js, ks) at column ii after the x fill
+template <class T>
+__device__ __forceinline__ void row_values(const Grid& g, const Fill<T>& F, int ii, int js, int ks, T (&v)[5]) {
+  const bool outer = ii == g.NI - 1;
+  const long long s = off3(g, ii == 0 ? 1 : outer ? ii - 1 : ii, js, ks);
+  T b[5], c[5];
+#pragma unroll
+  for (int w = 0; w < 5; ++w) v[w] = F.u[w * g.fs + s];
   if (ii == 0) {
-    const float2 a = u[off3(g, 1, jj, k)], b = u[off3(g, 2, jj, k)], c = u[off3(g, 3, jj, k)];
-    const double rx = (3.0 * (double)a.x - 3.0 * (double)b.x) + (double)c.x;
-    const double ry = (3.0 * (double)a.y - 3.0 * (double)b.y) + (double)c.y;
-    return make_float2((float)rx, (float)ry);
-  }
-  if (ii == g.NI - 1) {
-    if (inflow) {
-      const double2 v = up[off3(g, ii, jj, k)];
-      return make_float2((float)v.x, (float)v.y);
+#pragma unroll
+    for (int w = 0; w < 5; ++w) {
+      b[w] = F.u[w * g.fs + s + 1];
+      c[w] = F.u[w * g.fs + s + 2];
     }
-    return u[off3(g, ii - 1, jj, k)];
+#pragma unroll
+    for (int w = 0; w < 5; ++w) v[w] = excise(v[w], b[w], c[w]);
+  } else if (outer && F.inflow) {
+#pragma unroll
+    for (int w = 0; w < 5; ++w) hold(F.up[w * g.fs + s + 1], v[w]);
   }
-  return u[off3(g, ii, jj, k)];
 }
-
-// row (jd, kd) <- row (js, ks) after the x fill, all five variables
 template <class T>
-__device__ __forceinline__ void ghost_row(const Grid& g, T* u, const double2* up, int inflow, int jd, int kd, int js,
-                                          int ks) {
-  const long long d = off3(g, 0, jd, kd), s = off3(g, 0, js, ks);
-  for (int ii = threadIdx.x; ii < g.NI; ii += blockDim.x) {
-    T v[5];
-    if (ii == 0 || ii == g.NI - 1) {
+__device__ __forceinline__ void store_row(const Grid& g, const Fill<T>& F, int ii, int jd, int kd, const T (&v)[5]) {
+  const long long d = off3(g, ii, jd, kd);
 #pragma unroll
-      for (int w = 0; w < 5; ++w) v[w] = xval_t<T>(g, u + w * g.fs, up + w * g.fs, inflow, ii, js, ks);
-    } else {
-#pragma unroll
-      for (int w = 0; w < 5; ++w) v[w] = u[w * g.fs + s + ii];
-    }
-#pragma unroll
-    for (int w = 0; w < 5; ++w) u[w * g.fs + d + ii] = v[w];
-  }
+  for (int w = 0; w < 5; ++w) F.u[w * g.fs + d] = v[w];
 }
 
-__host__ __device__ __forceinline__ int ghost_units(const Grid& g, int threads) {
-  const int faces = 2 * (g.NJ - 6) * (g.Nz - 1);
+// the outermost planes of a refined level
+struct NoProlong {
+  static constexpr bool on = false;
+  int nbuf = 0;
+  __device__ void values(const Grid&, int, int, int, double2 (&)[5]) const {}
+  __device__ void values(const Grid&, int, int, int, float2 (&)[5]) const {}
+};
+struct WithProlong {
+  static constexpr bool on = true;
+  Prolong p;
+  int nbuf;
+  __device__ void values(const Grid&, int ii, int jj, int k, double2 (&v)[5]) const {
+#pragma unroll
+    for (int w = 0; w < 5; ++w) v[w] = prolong_value(p, w, ii, jj, k);
+  }
+};
+
+__host__ __device__ __forceinline__ int ghost_units(const Grid& g, int threads, int nbuf = 0) {
+  const int faces = (2 + nbuf) * (g.NJ - 6) * (g.Nz - 1);
   return 2 * g.NJ + 6 * (g.Nz - 1) + (faces + threads - 1) / threads;
 }
 
-template <class T>
-__device__ __forceinline__ void ghost_unit(const Grid& g, T* u, const double2* up, int inflow, int unit,
-                                           int cyclic = 0) {
+template <class T, class PR>
+__device__ __forceinline__ void ghost_unit(const Grid& g, const Fill<T>& F, const PR& pr, int unit, int part = 0, int parts = 1) {
   const int nC = 2 * g.NJ, nA = 6 * (g.Nz - 1);
-  if (unit < nC) {  // row jj of plane 0 or Nz
-    const int jj = unit % g.NJ;
-    const bool last = unit >= g.NJ;
-    const int ks = last ? 1 : g.Nz - 1;
-    const bool ghost = jj < 3 || jj >= g.NJ - 3;
-    if (!last && !ghost && !cyclic) {
-      const int kp = g.Nzm1 - g.dis;
-      const bool north = jj <= 5, south = jj >= g.NJ - 6;
-      if (north) ghost_row(g, u, up, inflow, 5 - jj, kp, jj, 0);
-      if (south) ghost_row(g, u, up, inflow, 2 * g.NJ - 7 - jj, kp, jj, 0);
-      if (north || south) __syncthreads();
+  const int end = PR::on ? g.NI - pr.nbuf : g.NI;  // columns from here on are the coarser level's
+  if (unit < nC + nA) {
+    int jd, kd, js, ks;
+    bool both = false;  // a row of plane 0 that ghost rows of plane kp copy before it is overwritten
+    if (unit < nC) {    // row jj of plane 0 or Nz
+      jd = unit % g.NJ;
+      const bool last = unit >= g.NJ;
+      const bool ghost = jd < 3 || jd >= g.NJ - 3;
+      kd = last ? g.Nz : 0;
+      ks = last ? 1 : g.Nz - 1;
+      js = ghost ? ghost_src_row(g, jd) : jd;
+      if (ghost) ks = ktarget(g, ks);
+      both = !last && !ghost && !F.cyclic && (jd <= 5 || jd >= g.NJ - 6);
+    } else {  // ghost row of an inner plane
+      const int q = unit - nC, r = q % 6;
+      kd = 1 + q / 6;
+      ks = ktarget(g, kd);
+      if (ks == 0) {
+        if (!F.cyclic) return;  // with plane 0's own rows
+        ks = g.Nzm1;
+      }
+      jd = (r < 3) ? r : (g.NJ - 6 + r);
+      js = ghost_src_row(g, jd);
     }
-    ghost_row(g, u, up, inflow, jj, last ? g.Nz : 0, ghost ? ghost_src_row(g, jj) : jj, ghost ? ktarget(g, ks) : ks);
-  } else if (unit < nC + nA) {  // ghost row of an inner plane
-    const int q = unit - nC;
-    const int r = q % 6, k = 1 + q / 6;
-    int kt = ktarget(g, k);
-    if (kt == 0) {
-      if (!cyclic) return;  // with plane 0's own rows
-      kt = g.Nzm1;          // plane 0 was not computed: it equals plane Nz - 1
+    const int kp = g.Nzm1 - g.dis;
+    // the column that the outermost one copies may lie in a part of the row that is
+    // overwritten before the outermost one's turn
+    T edge[5];
+    if (both)
+#pragma unroll
+      for (int w = 0; w < 5; ++w) edge[w] = F.u[w * g.fs + off3(g, g.NI - 2, jd, 0)];
+    for (int i0 = part * blockDim.x; i0 < g.NI; i0 += parts * blockDim.x) {
+      const int ii = i0 + threadIdx.x;
+      const bool in = ii < g.NI;
+      T v[5], z[5];
+      if (in) {
+        if (PR::on && ii >= end) pr.values(g, ii, jd, kd, v);
+        else row_values(g, F, ii, js, ks, v);
+        if (both) {
+          if (PR::on && ii >= end) {
+          } else if (ii == g.NI - 1 && !F.inflow) {
+#pragma unroll
+            for (int w = 0; w < 5; ++w) z[w] = edge[w];
+          } else {
+            row_values(g, F, ii, jd, 0, z);
+          }
+        }
+      }
+      if (both) __syncthreads();  // both rows have been read
+      if (in) {
+        store_row(g, F, ii, jd, kd, v);
+        if (both) {
+          if (jd <= 5) {
+            if (PR::on && ii >= end) pr.values(g, ii, 5 - jd, kp, z);
+            store_row(g, F, ii, 5 - jd, kp, z);
+          }
+          if (jd >= g.NJ - 6) {
+            if (PR::on && ii >= end) pr.values(g, ii, 2 * g.NJ - 7 - jd, kp, z);
+            store_row(g, F, ii, 2 * g.NJ - 7 - jd, kp, z);
+          }
+        }
+      }
     }
-    const int jj = (r < 3) ? r : (g.NJ - 6 + r);
-    ghost_row(g, u, up, inflow, jj, k, ghost_src_row(g, jj), kt);
-  } else {  // x-face points
+  } else if (part == 0) {  // x-face points of the interior rows, then their columns from the coarser level
     const int f = (unit - nC - nA) * blockDim.x + threadIdx.x;
     const int nin = g.NJ - 6;
-    if (f >= 2 * nin * (g.Nz - 1)) return;
-    const int jj = 3 + f % nin, sk = f / nin;
-    const int k = 1 + (sk >> 1), ii = (sk & 1) ? g.NI - 1 : 0;
-#pragma unroll
-    for (int w = 0; w < 5; ++w)
-      u[w * g.fs + off3(g, ii, jj, k)] = xval_t<T>(g, u + w * g.fs, up + w * g.fs, inflow, ii, jj, k);
+    const int sk = f / nin, jj = 3 + f % nin, sides = 2 + pr.nbuf;
+    if (sk >= sides * (g.Nz - 1)) return;
+    const int side = sk % sides, k = 1 + sk / sides;
+    T v[5];
+    if (side < 2) {
+      if (PR::on && side == 1) return;
+      const int ii = side ? g.NI - 1 : 0;
+      row_values(g, F, ii, jj, k, v);
+      store_row(g, F, ii, jj, k, v);
+    } else {
+      const int ii = g.NI - pr.nbuf + side - 2;
+      pr.values(g, ii, jj, k, v);
+      store_row(g, F, ii, jj, k, v);
+    }
   }
 }
 
-// threads of a block: a row of a small grid in one pass, 256 for longer rows
-static int row_threads(int ni) { return ni >= 256 ? 256 : (ni + 31) / 32 * 32; }
+// threads of a block
+static int row_threads(int ni) { return ni >= 128 ? 128 : (ni + 31) / 32 * 32; }
+// Blocks that share a row: one per row_threads columns, unless the outermost column
+// would be alone in the last (it copies its neighbour, which must not be overwritten before).
+static int row_parts(int ni) {
+  const int nt = row_threads(ni);
+  return ni % nt == 1 ? 1 : (ni + nt - 1) / nt;
+}
 
-template <class T>
-__global__ void ghost_kernel(Grid g, T* u, const double2* up, int inflow, int unit0, int cyclic) {
+// 64 registers a thread let 1024 threads run on an SM: the rows of a large grid are
+// bound by the bytes in flight (1024 x 65 x 129: 31.8 us; 33.3 with 768 threads, 39.5
+// with 512).  The coarser level's stencil takes 40 values at once and is the faster
+// for room (384 x 33 x 65: 17.9 us with 128 registers, 20.1 with 80 or 64).  Blocks of
+// 256 threads and one block a row took 15.7 us in the place of 13.8 (301 x 46 x 90).
+template <class T, class PR>
+__global__ void __launch_bounds__(128, PR::on ? 4 : 8) ghost_kernel(Grid g, Fill<T> F, PR pr, int unit0) {
   pdl_wait();
-  ghost_unit(g, u, up, inflow, unit0 + blockIdx.x, cyclic);
+  ghost_unit(g, F, pr, unit0 + blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 void launch_ghost_fill(const Grid& g, double2* u, const double2* up, int inflow, cudaStream_t st, bool faces_apart,
                        bool cyclic) {
-  const int nt = row_threads(g.NI), n = ghost_units(g, nt), rows = 2 * g.NJ + 6 * (g.Nz - 1);
+  const int nt = row_threads(g.NI), parts = row_parts(g.NI), n = ghost_units(g, nt), rows = 2 * g.NJ + 6 * (g.Nz - 1);
+  const Fill<double2> F = {u, up, inflow, (int)cyclic};
+  auto kern = ghost_kernel<double2, NoProlong>;
   if (!faces_apart) {
-    launch_pdl(ghost_kernel<double2>, n, nt, 0, st, g, u, up, inflow, 0, (int)cyclic);
+    launch_pdl(kern, dim3(n, parts), nt, 0, st, g, F, NoProlong(), 0);
     return;
   }
-  launch_pdl(ghost_kernel<double2>, rows, nt, 0, st, g, u, up, inflow, 0, (int)cyclic);
-  launch_pdl(ghost_kernel<double2>, n - rows, nt, 0, st, g, u, up, inflow, rows, (int)cyclic);
+  launch_pdl(kern, dim3(rows, parts), nt, 0, st, g, F, NoProlong(), 0);
+  launch_pdl(kern, n - rows, nt, 0, st, g, F, NoProlong(), rows);
 }
 
 void launch_ghost_fill_f32(const Grid& g, float2* u, const double2* up, int inflow, cudaStream_t st) {
   const int nt = row_threads(g.NI);
-  launch_pdl(ghost_kernel<float2>, ghost_units(g, nt), nt, 0, st, g, u, up, inflow, 0, 0);
+  launch_pdl(ghost_kernel<float2, NoProlong>, dim3(ghost_units(g, nt), row_parts(g.NI)), nt, 0, st, g, Fill<float2>{u, up, inflow, 0},
+             NoProlong(), 0);
+}
+
+void launch_ghost_prolong(const Grid& g, double2* u, const double2* up, int inflow, const Prolong& p, int nbuf,
+                          cudaStream_t st) {
+  const int nt = row_threads(g.NI);
+  launch_pdl(ghost_kernel<double2, WithProlong>, dim3(ghost_units(g, nt, nbuf), row_parts(g.NI)), nt, 0, st,
+             g, Fill<double2>{u, up, inflow, 0}, WithProlong{p, nbuf}, 0);
 }
 
 // ---- many solves at once (batched engine): one block row per solve -----------
-constexpr int GB_THREADS = 128;
+constexpr int GB_THREADS = 128, GB_PARTS = 4;
 template <class T>
-__global__ void ghost_batch_kernel(const GhostDesc* __restrict__ d) {
+__global__ void __launch_bounds__(GB_THREADS, 8) ghost_batch_kernel(const GhostDesc* __restrict__ d) {
   pdl_wait();
   const GhostDesc& D = d[blockIdx.y];
-  if ((int)blockIdx.x < ghost_units(D.g, GB_THREADS))
-    ghost_unit(D.g, static_cast<T*>(D.u), D.up, D.inflow, blockIdx.x);
+  const int parts = D.g.NI % GB_THREADS == 1 ? 1 : gridDim.z;  // see row_parts
+  if ((int)blockIdx.x < ghost_units(D.g, GB_THREADS) && (int)blockIdx.z < parts)
+    ghost_unit(D.g, Fill<T>{static_cast<T*>(D.u), D.up, D.inflow, 0}, NoProlong(), blockIdx.x, blockIdx.z, parts);
 }
 
 int ghost_batch_units(const Grid& g) { return ghost_units(g, GB_THREADS); }
 
 void launch_ghost_fill_batch(const GhostDesc* d_desc, int n, int max_units, int f32, cudaStream_t st) {
   if (n <= 0) return;
-  launch_pdl(f32 ? ghost_batch_kernel<float2> : ghost_batch_kernel<double2>, dim3(max_units, n), GB_THREADS, 0, st,
+  launch_pdl(f32 ? ghost_batch_kernel<float2> : ghost_batch_kernel<double2>, dim3(max_units, n, GB_PARTS), GB_THREADS, 0, st,
              d_desc);
 }
 

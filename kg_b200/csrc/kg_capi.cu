@@ -25,6 +25,7 @@
 #include "kg_device.cuh"
 #include "kg_internal.h"
 #include "kg_diag.h"
+#include "kg_refine.cuh"
 
 using kg::Grid;
 using kg::Metric;
@@ -1388,6 +1389,16 @@ int step_rk4_cfg(kg_solver* h, int nsteps) {
   return KG_OK;
 }
 
+// ghost fill of a refined level's state, with the outermost planes from the coarser level
+int fill_level(kg_solver* h, kg_solver* c, const double2* c_old, double2* u, double alpha, int inflow, int nbuf) {
+  if (!kg::prolong_fits(h->g, c->g, nbuf))
+    return set_err(h, KG_EINVAL, "refined level does not fit inside its coarser level");
+  h->seam_filled = false;
+  Prof pf(h, PK_GHOST, 1);
+  kg::launch_ghost_prolong(h->g, u, h->U, inflow, kg::Prolong{c->g, c_old, c->U, alpha}, nbuf, h->stream);
+  return KG_OK;
+}
+
 // RK4 step of a refined level whose outermost planes follow the coarser level:
 // after every stage the stage output's buffer planes take the coarse values
 // interpolated to the time of the stage that reads them (alpha = position in
@@ -1420,8 +1431,7 @@ int step_rk4_bo(kg_solver* h, kg_solver* c, const double2* c_old, double a0, dou
     L.out = outs[st];
     L.skip_last_i = (st == 3) ? inflow : 0;
     run_stage(h, kinds[st], L);
-    run_ghost(h, outs[st], h->U, inflow);
-    if ((rc = prolong(outs[st], at[st]))) return rc;
+    if ((rc = fill_level(h, c, c_old, outs[st], at[st], inflow, nbuf))) return rc;
   }
   h->t = h->t + h->dt;
   KG_CK(cudaGetLastError());
@@ -1458,8 +1468,7 @@ int step_rk3_bo(kg_solver* h, kg_solver* c, const double2* c_old, double a0, dou
     L.out = outs[st];
     L.skip_last_i = (st == 2) ? inflow : 0;
     run_stage(h, kinds[st], L);
-    run_ghost(h, outs[st], h->U, inflow);
-    if ((rc = prolong(outs[st], at[st]))) return rc;
+    if ((rc = fill_level(h, c, c_old, outs[st], at[st], inflow, nbuf))) return rc;
   }
   h->t = h->t + h->dt;
   KG_CK(cudaGetLastError());
@@ -1514,8 +1523,7 @@ int step_pirk_bo(kg_solver* h, kg_solver* c, const double2* c_old, double a0, do
     L.skip_last_i = inflow;
     run_stage(h, kg::ST_P2_S2, L);
   }
-  run_ghost(h, h->U, h->U, inflow);
-  if ((rc = prolong(h->U, nullptr, a0 + da))) return rc;
+  if ((rc = fill_level(h, c, c_old, h->U, a0 + da, inflow, nbuf))) return rc;
   h->s_cur = 9 - h->s_cur;
   h->t = h->t + h->dt;
   KG_CK(cudaGetLastError());

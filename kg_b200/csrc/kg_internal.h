@@ -196,6 +196,11 @@ void launch_ghost_fill_cfg(const Grid& g, double2* u, cudaStream_t st);
 // uf_pi: where the fine Pi variable lives (nullptr: uf + 4 fs, the 5-variable layout)
 int launch_prolong(const Grid& gf, double2* uf, const Grid& gc, const double2* c_old, const double2* c_new,
                    double alpha, int nbuf, cudaStream_t st, double2* uf_pi = nullptr);
+struct Prolong;  // kg_refine.cuh
+bool prolong_fits(const Grid& gf, const Grid& gc, int nbuf);
+// the ghost fill of a refined level's state, its outermost nbuf planes from the coarser level
+void launch_ghost_prolong(const Grid& g, double2* u, const double2* up, int inflow, const Prolong& p, int nbuf,
+                          cudaStream_t st);
 int launch_restrict(const Grid& gc, double2* uc, const Grid& gf, const double2* uf, int keep_out, cudaStream_t st);
 void launch_rhs(const Grid& g, const Metric& m, int metric_kind, const double2* const in[5], double2* out,
                 unsigned mask, cudaStream_t st);

@@ -14,20 +14,12 @@
 #include <cuda_runtime.h>
 #include "kg_device.cuh"
 #include "kg_internal.h"
+#include "kg_refine.cuh"
 
 namespace kg {
 namespace {
 
-__device__ __forceinline__ double2 prolong_r(const Grid& gc, const double2* c, int iif, int jj, int k) {
-  if ((iif & 1) == 0) return c[off3(gc, iif >> 1, jj, k)];
-  const int a = iif >> 1;
-  const double2 cm = c[off3(gc, a - 1, jj, k)], c0 = c[off3(gc, a, jj, k)], c1 = c[off3(gc, a + 1, jj, k)],
-                c2v = c[off3(gc, a + 2, jj, k)];
-  return rmul(1.0 / 16.0, csub(cadd(cadd(cneg(cm), rmul(9.0, c0)), rmul(9.0, c1)), c2v));
-}
-
-__global__ void prolong_kernel(Grid gf, double2* uf, double2* uf_pi, Grid gc, const double2* c_old,
-                               const double2* c_new, double alpha, int nbuf) {
+__global__ void prolong_kernel(Grid gf, double2* uf, double2* uf_pi, Prolong p, int nbuf) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long n = (long long)nbuf * gf.NJ * gf.NK;
   if (t >= n) return;
@@ -37,10 +29,8 @@ __global__ void prolong_kernel(Grid gf, double2* uf, double2* uf_pi, Grid gc, co
   const int iif = gf.NI - nbuf + b;
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
-    const double2 po = prolong_r(gc, c_old + (long long)v * gc.fs, iif, jj, k);
-    const double2 pn = prolong_r(gc, c_new + (long long)v * gc.fs, iif, jj, k);
     double2* dst = (v == 4) ? uf_pi : uf + (long long)v * gf.fs;
-    dst[off3(gf, iif, jj, k)] = cadd(rmul(1.0 - alpha, po), rmul(alpha, pn));
+    dst[off3(gf, iif, jj, k)] = prolong_value(p, v, iif, jj, k);
   }
 }
 
@@ -58,15 +48,18 @@ __global__ void restrict_kernel(Grid gc, double2* uc, Grid gf, const double2* uf
 
 }  // namespace
 
+// the stencil reaches coarse plane (NI_f - 1) / 2 + 2, which must lie inside the coarse grid
+bool prolong_fits(const Grid& gf, const Grid& gc, int nbuf) {
+  return nbuf >= 1 && nbuf <= gf.NI && gf.NJ == gc.NJ && gf.NK == gc.NK && (gf.NI - 1) / 2 + 2 <= gc.NI - 1 &&
+         (gf.NI - nbuf) / 2 - 1 >= 0;
+}
+
 int launch_prolong(const Grid& gf, double2* uf, const Grid& gc, const double2* c_old, const double2* c_new,
                    double alpha, int nbuf, cudaStream_t st, double2* uf_pi) {
-  // the stencil reaches coarse plane (NI_f - 1) / 2 + 2, which must lie inside the coarse grid
-  if (nbuf < 1 || nbuf > gf.NI || gf.NJ != gc.NJ || gf.NK != gc.NK || (gf.NI - 1) / 2 + 2 > gc.NI - 1 ||
-      (gf.NI - nbuf) / 2 - 1 < 0)
-    return -1;
+  if (!prolong_fits(gf, gc, nbuf)) return -1;
   const long long n = (long long)nbuf * gf.NJ * gf.NK;
   if (!uf_pi) uf_pi = uf + 4 * gf.fs;
-  prolong_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(gf, uf, uf_pi, gc, c_old, c_new, alpha, nbuf);
+  prolong_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(gf, uf, uf_pi, Prolong{gc, c_old, c_new, alpha}, nbuf);
   return 0;
 }
 
