@@ -36,7 +36,8 @@ constexpr int TI = 32, RH = 2;
 constexpr int RW = 2 * (TI + 2 * RH);  // ring row width in elements (two per complex value)
 constexpr int NST = 3;
 constexpr int MW = TI + 2 * RH;
-enum { MT_AL = 0, MT_BE, MT_A, MT_GRR, MT_GRP, MT_SG, MT_HT, MT_COUNT };
+// metric tiles: with one theta row on either side, then the tile's own rows alone
+enum { MT_AL = 0, MT_BE, MT_HT, MT_HALO, MT_A = MT_HALO, MT_GRR, MT_GRP, MT_SG, MT_COUNT };
 // tile geometry for TJ theta rows (one warp per row): 8 (256 threads, 2 CTAs
 // per SM) or 4 (128 threads, 3 CTAs per SM)
 template <int TJ>
@@ -44,7 +45,12 @@ struct MGeom {
   static constexpr int RROWS = TJ + 2;
   static constexpr int FIELD_E = RROWS * RW;
   static constexpr int STAGE_E = 5 * FIELD_E;
-  static constexpr int MH = TJ + 2, MT_N = MW * MH;
+  static constexpr int MH = TJ + 2, MT_N = MW * MH, MT_R = MW * TJ;
+  static constexpr int MT_ALL = MT_HALO * MT_N + (MT_COUNT - MT_HALO) * MT_R;
+  // value of tile `which` at column dx, row dy
+  static __device__ __forceinline__ int mt_at(int which, int dx, int dy) {
+    return dx + RH + (which < MT_HALO ? which * MT_N + (dy + 1) * MW : MT_HALO * MT_N + (which - MT_HALO) * MT_R + dy * MW);
+  }
   // stages 2-4 (FP32 ring) stage their point-wise operands -- u^n (FP64) and the
   // increment sum (FP32), five variables of the thread's own point -- in shared
   // memory with cp.async issued at the start of each plane, so the loads run
@@ -58,8 +64,8 @@ struct MGeom {
   }
   template <class T>
   static __host__ __device__ constexpr size_t smem() {
-    return (size_t)NST * slot_e<T>() * sizeof(T) + (size_t)MT_COUNT * MT_N * 8 + 64 + 128 +
-           (sizeof(T) == 4 ? (size_t)STG_BYTES + (size_t)MT_COUNT * MT_N * 4 : 0);
+    return (size_t)NST * slot_e<T>() * sizeof(T) + (size_t)MT_ALL * (8 + 4) + 64 + 128 +
+           (sizeof(T) == 4 ? (size_t)STG_BYTES : 0);
   }
 };
 
@@ -109,6 +115,22 @@ __device__ __forceinline__ cx<R> ld2(const T* p) {
   return CX<R>((R)p[0], (R)p[1]);
 }
 
+// What a thread keeps in arithmetic type R across planes (its own point's metric,
+// the phi-derivative arguments) lies in FP64 registers, as FP32 bit patterns for
+// R = float: a value is converted once, not at each use.  Conversions from and to 64
+// bits bound stage 1, whose ring is FP64 (their pipe 63 % busy, the next one 19 %).
+// With this and the FP32 metric tiles in every stage, 1024 x 65 x 129: stage 1 325 ->
+// 307 us, the others (240 B a point, 0.92 of the copy bandwidth) as before.
+template <class R>
+__device__ __forceinline__ R kept(double v);
+template <>
+__device__ __forceinline__ double kept<double>(double v) { return v; }
+template <>
+__device__ __forceinline__ float kept<float>(double v) { return __int_as_float(__double2loint(v)); }
+__device__ __forceinline__ double keep(float v) { return __hiloint2double(0, __float_as_int(v)); }
+__device__ __forceinline__ double2 keep(cx<double> v) { return make_double2(v.x, v.y); }
+__device__ __forceinline__ double2 keep(cx<float> v) { return make_double2(keep(v.x), keep(v.y)); }
+
 struct MxArgs {
   Grid g;
   Metric m;
@@ -142,19 +164,20 @@ template <class R, int MK, class TIN, int TJ, bool FAST = false>
 __device__ __forceinline__ void mx_rhs(const MxArgs& a, const TIN* cu, const double* mt, const float* mtf, int tx,
                                        int ty, int ii, int jj, int k, const double* own, double2 Epv, double2 Enx,
                                        double2 Fpv, double2 Fnx, cx<R> r[5]) {
-  constexpr int FIELD_E = MGeom<TJ>::FIELD_E, MT_N = MGeom<TJ>::MT_N;
+  constexpr int FIELD_E = MGeom<TJ>::FIELD_E;
   const Grid& g = a.g;
-  const R al = (R)own[0], be = (R)own[1], dxb = (R)own[2], sg = (R)own[3], rs = (R)own[4], am2 = (R)own[5];
+  const R al = kept<R>(own[0]), be = kept<R>(own[1]), dxb = kept<R>(own[2]), sg = kept<R>(own[3]),
+          rs = kept<R>(own[4]), am2 = kept<R>(own[5]);
   const R rdx = (R)g.rdx, rdy = (R)g.rdy, rdz = (R)g.rdz;
   const int n = g.NI - 1;
   auto RF = [&](int f, int dx, int dy) -> cx<R> {
     return ld2<R>(cu + (size_t)f * FIELD_E + (dy + 1) * RW + 2 * (dx + RH));
   };
   // metric at tile point (dx, dy); the FP32 arithmetic reads the FP32 copy of the
-  // tile where there is one (stages with an FP32 ring), without a conversion per use
+  // tile, without a conversion per use
   auto MTV = [&](int which, int dx, int dy) -> R {
-    const int o = which * MT_N + (dy + 1) * MW + dx + RH;
-    if (sizeof(R) == 4 && sizeof(TIN) == 4) return (R)mtf[o];
+    const int o = MGeom<TJ>::mt_at(which, dx, dy);
+    if (sizeof(R) == 4) return (R)mtf[o];
     return (R)mt[o];
   };
   cx<R> fcu[5];
@@ -191,7 +214,7 @@ __device__ __forceinline__ void mx_rhs(const MxArgs& a, const TIN* cu, const dou
   }
   // rhs_psi3 (:704-713)
   {
-    const cx<R> ep = CX<R>((R)Epv.x, (R)Epv.y), en = CX<R>((R)Enx.x, (R)Enx.y);
+    const cx<R> ep = CX<R>(kept<R>(Epv.x), kept<R>(Epv.y)), en = CX<R>(kept<R>(Enx.x), kept<R>(Enx.y));
     cx<R> z;
     if (k == 0) z = add(neg(ep), en);
     else if (k == g.Nz) z = add(neg(en), ep);
@@ -214,7 +237,7 @@ __device__ __forceinline__ void mx_rhs(const MxArgs& a, const TIN* cu, const dou
     const cx<R> r1 = dsg(sm(rdx, d), sg, rs);
     auto H = [&](int dy) { return sm(MTV(MT_HT, tx, ty + dy), RF(2, tx, ty + dy)); };
     const cx<R> r2 = dsg(sm(rdy, cc(H(-1), H(1))), sg, rs);
-    const cx<R> fp = CX<R>((R)Fpv.x, (R)Fpv.y), fn = CX<R>((R)Fnx.x, (R)Fnx.y);
+    const cx<R> fp = CX<R>(kept<R>(Fpv.x), kept<R>(Fpv.y)), fn = CX<R>(kept<R>(Fnx.x), kept<R>(Fnx.y));
     cx<R> z;
     if (k == 0) z = add(neg(fp), fn);
     else if (k == g.Nz) z = add(neg(fn), fp);
@@ -238,18 +261,19 @@ __device__ __forceinline__ void mx_rhs(const MxArgs& a, const TIN* cu, const dou
   }
 }
 
-// phi-derivative arguments at the own point of a ring slot, in R, widened
+// phi-derivative arguments at the own point of a ring slot, in R (see kept)
 template <class R, int MK, class TIN, int TJ>
 __device__ __forceinline__ void mx_EF(const TIN* st, int tx, int ty, const double* own, double2& E, double2& F) {
   constexpr int FIELD_E = MGeom<TJ>::FIELD_E;
   auto RF = [&](int f) -> cx<R> { return ld2<R>(st + (size_t)f * FIELD_E + (ty + 1) * RW + 2 * (tx + RH)); };
-  const R al = (R)own[0], be = (R)own[1], fa = (R)own[6], fgrp = (R)own[7], fgpp = (R)own[8];
+  const R al = kept<R>(own[0]), be = kept<R>(own[1]), fa = kept<R>(own[6]), fgrp = kept<R>(own[7]),
+          fgpp = kept<R>(own[8]);
   const cx<R> e = add(sm(al, RF(4)), sm(be, RF(1)));
   cx<R> f;
   if (MK == MK_KS) f = sm(fa, add(sm(fgrp, RF(1)), sm(fgpp, RF(3))));
   else f = sm(fa, RF(3));
-  E = make_double2((double)e.x, (double)e.y);
-  F = make_double2((double)f.x, (double)f.y);
+  E = keep(e);
+  F = keep(f);
 }
 
 template <int KIND, int MK, class TIN, int TJ>
@@ -261,8 +285,8 @@ __device__ __forceinline__ int mx_item(const CUtensorMap* tinp, const CUtensorMa
   constexpr bool STG = sizeof(TIN) == 4;
   double2* base_s = reinterpret_cast<double2*>(stg);
   float2* acc_s = reinterpret_cast<float2*>(stg + (size_t)TI * TJ * 5 * 16);
-  // FP32 copy of the metric tile (stages with an FP32 ring; it sits after the FP64 tile)
-  float* mtf = reinterpret_cast<float*>(mt + (size_t)MT_COUNT * MT_N);
+  // FP32 copy of the metric tiles
+  float* mtf = reinterpret_cast<float*>(mt + GT::MT_ALL);
   const Grid& g = a.g;
   const Metric& M = a.m;
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TI + tx;
@@ -323,15 +347,20 @@ __device__ __forceinline__ int mx_item(const CUtensorMap* tinp, const CUtensorMa
     const int gi = ii0 - RH + mx, gj = jj0 - 1 + my;
     const bool in = gi >= 0 && gi < g.NI && gj >= 0 && gj < g.NJ;
     const int q = in ? off2(g, gi, gj) : 0;
-    mt[MT_AL * MT_N + t] = in ? ldm(M.alpha, q) : 0.0;
-    mt[MT_BE * MT_N + t] = in ? ldm(M.beta, q) : 0.0;
-    mt[MT_A * MT_N + t] = in ? ldm(MK == MK_KS ? M.asg : M.asg_grr, q) : 0.0;
-    mt[MT_GRR * MT_N + t] = in ? ldm(M.grr, q) : 0.0;
-    mt[MT_GRP * MT_N + t] = in ? ldm(M.grp, q) : 0.0;
-    mt[MT_SG * MT_N + t] = in ? ldm(M.sqrtg, q) : 0.0;
-    mt[MT_HT * MT_N + t] = in ? ldm(M.asg_gtt, q) : 0.0;
-    if (STG)
-      for (int w = 0; w < MT_COUNT; ++w) mtf[w * MT_N + t] = (float)mt[w * MT_N + t];
+    auto put = [&](int which, double v) {
+      const int o = GT::mt_at(which, mx - RH, my - 1);
+      mt[o] = v;
+      mtf[o] = (float)v;
+    };
+    put(MT_AL, in ? ldm(M.alpha, q) : 0.0);
+    put(MT_BE, in ? ldm(M.beta, q) : 0.0);
+    put(MT_HT, in ? ldm(M.asg_gtt, q) : 0.0);
+    if (my >= 1 && my <= TJ) {
+      put(MT_A, in ? ldm(MK == MK_KS ? M.asg : M.asg_grr, q) : 0.0);
+      put(MT_GRR, in ? ldm(M.grr, q) : 0.0);
+      put(MT_GRP, in ? ldm(M.grp, q) : 0.0);
+      put(MT_SG, in ? ldm(M.sqrtg, q) : 0.0);
+    }
   }
   __syncthreads();
   pdl_wait();  // ahead of this thread's own reads and writes of the state
@@ -361,6 +390,9 @@ __device__ __forceinline__ int mx_item(const CUtensorMap* tinp, const CUtensorMa
   const bool hp = (ii <= 1) || (jj == 3) || (jj == 4) || (jj == g.NJ - 5) || (jj == g.NJ - 4);
   const bool fast =
       __all_sync(0xffffffffu, act && !hp && ii <= g.NI - 3 && (float)own[1] > 0.0f);  // warp-uniform
+  if (!hp)
+#pragma unroll
+    for (int w = 0; w < 9; ++w) own[w] = keep((float)own[w]);
   auto EF = [&](const TIN* st, double2& E, double2& F) {
     if (hp) mx_EF<double, MK, TIN, TJ>(st, tx, ty, own, E, F);
     else mx_EF<float, MK, TIN, TJ>(st, tx, ty, own, E, F);
@@ -504,12 +536,10 @@ __global__ void __launch_bounds__(TI * TJ, MGeom<TJ>::MIN_BLOCKS)
     mx_stage_kernel(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tp0,
                     const __grid_constant__ CUtensorMap tp1, MxArgs a) {
   using GT = MGeom<TJ>;
-  constexpr int MT_N = GT::MT_N;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   TIN* ring = reinterpret_cast<TIN*>(align128(smem_raw));
   double* mt = reinterpret_cast<double*>(ring + (size_t)NST * GT::template slot_e<TIN>());
-  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(mt + (size_t)MT_COUNT * MT_N) +
-                                               (sizeof(TIN) == 4 ? (size_t)MT_COUNT * MT_N * 4 : 0));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<float*>(mt + GT::MT_ALL) + GT::MT_ALL);
   unsigned char* stg = reinterpret_cast<unsigned char*>(bars + 8);
   init_bars<TJ>(bars);
   (void)mx_item<KIND, MK, TIN, TJ>(&tin, &tp0, &tp1, a, blockIdx.x, blockIdx.y, blockIdx.z, ring, mt, bars, 0u, stg);
@@ -519,12 +549,10 @@ template <int KIND, int MK, class TIN, int TJ>
 __global__ void __launch_bounds__(TI * TJ, MGeom<TJ>::MIN_BLOCKS)
     mx_batch_kernel(const MxItem* __restrict__ solves, int n_solves, int n_items, BatchCounter* ctr) {
   using GT = MGeom<TJ>;
-  constexpr int MT_N = GT::MT_N;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   TIN* ring = reinterpret_cast<TIN*>(align128(smem_raw));
   double* mt = reinterpret_cast<double*>(ring + (size_t)NST * GT::template slot_e<TIN>());
-  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(mt + (size_t)MT_COUNT * MT_N) +
-                                               (sizeof(TIN) == 4 ? (size_t)MT_COUNT * MT_N * 4 : 0));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<float*>(mt + GT::MT_ALL) + GT::MT_ALL);
   unsigned char* stg = reinterpret_cast<unsigned char*>(bars + 8);
   __shared__ MxArgs sa;
   __shared__ int s_bx, s_by, s_bz, s_solve, s_next;
