@@ -813,8 +813,8 @@ bool direct_buffer(const kg_solver* h, const void* p) {
 
 // copy a Fortran-layout state (host or device memory) into 5 device planes, in
 // pieces through the staging buffer; a device buffer is converted where it lies
-// (2048 x 129 x 257, set and get: 8.0 -> 4.2 ms, the conversion's own 23 GB at
-// 5.5 TB/s)
+// (2048 x 129 x 257, set and get: 8.0 -> 3.6 ms, the conversion's own 23 GB at
+// 6.4 TB/s)
 int load_view(kg_solver* h, const View& V, const double* src, cudaMemcpyKind kind) {
   int rc;
   const Grid& g = h->g;
