@@ -2732,7 +2732,8 @@ void* kg_batch_get_stream(const kg_batch* b) { return b ? (void*)b->stream : nul
 // space and time; then it is restricted onto the parent.
 struct kg_hier {
   std::vector<kg_solver*> lv;
-  std::vector<double2*> uold;  // state of each non-finest level at the start of its current step
+  // state of each non-finest level at the start of its current step (the columns that its finer level's edge needs)
+  std::vector<double2*> uold;
   std::vector<cudaEvent_t> ev;
   int nbuf = 4, keep_out = 8;
   long long coarse_steps = 0;
@@ -2755,7 +2756,8 @@ int hier_step(kg_hier* H, int l, double a0, double da, int method) {
   const int n = (int)H->lv.size();
   int rc;
   if (l + 1 < n) {
-    if (cudaMemcpyAsync(H->uold[l], h->U, 5 * field_bytes(h), cudaMemcpyDeviceToDevice, h->stream) != cudaSuccess) {
+    kg::launch_keep_columns(h->g, h->U, H->uold[l], H->lv[l + 1]->g, H->nbuf, h->stream);
+    if (cudaGetLastError() != cudaSuccess) {
       H->err = "level state copy failed";
       return KG_ECUDA;
     }

@@ -201,6 +201,8 @@ bool prolong_fits(const Grid& gf, const Grid& gc, int nbuf);
 // the ghost fill of a refined level's state, its outermost nbuf planes from the coarser level
 void launch_ghost_prolong(const Grid& g, double2* u, const double2* up, int inflow, const Prolong& p, int nbuf,
                           cudaStream_t st);
+// columns of the coarser level's state u that the prolongation to gf reads, at their place in `to`
+void launch_keep_columns(const Grid& gc, const double2* u, double2* to, const Grid& gf, int nbuf, cudaStream_t st);
 int launch_restrict(const Grid& gc, double2* uc, const Grid& gf, const double2* uf, int keep_out, cudaStream_t st);
 void launch_rhs(const Grid& g, const Metric& m, int metric_kind, const double2* const in[5], double2* out,
                 unsigned mask, cudaStream_t st);

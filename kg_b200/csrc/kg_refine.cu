@@ -12,6 +12,7 @@
 //   restriction: every coarse point under the fine level's interior (all but
 //     the last `keep_out` fine planes) takes the coincident fine value.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include "kg_device.cuh"
 #include "kg_internal.h"
 #include "kg_refine.cuh"
@@ -20,6 +21,7 @@ namespace kg {
 namespace {
 
 __global__ void prolong_kernel(Grid gf, double2* uf, double2* uf_pi, Prolong p, int nbuf) {
+  pdl_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long n = (long long)nbuf * gf.NJ * gf.NK;
   if (t >= n) return;
@@ -34,7 +36,19 @@ __global__ void prolong_kernel(Grid gf, double2* uf, double2* uf_pi, Prolong p, 
   }
 }
 
+// the columns lo .. lo + nc - 1 of a state
+__global__ void columns_kernel(Grid g, const double2* u, double2* to, int lo, int nc) {
+  pdl_wait();
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)nc * g.NJ * g.NK) return;
+  const long long r = t / nc;
+  const long long o = off3(g, lo + (int)(t % nc), (int)(r % g.NJ), (int)(r / g.NJ));
+#pragma unroll
+  for (int v = 0; v < 5; ++v) to[(long long)v * g.fs + o] = u[(long long)v * g.fs + o];
+}
+
 __global__ void restrict_kernel(Grid gc, double2* uc, Grid gf, const double2* uf, int nc) {
+  pdl_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long n = (long long)nc * gc.NJ * gc.NK;
   if (t >= n) return;
@@ -59,8 +73,20 @@ int launch_prolong(const Grid& gf, double2* uf, const Grid& gc, const double2* c
   if (!prolong_fits(gf, gc, nbuf)) return -1;
   const long long n = (long long)nbuf * gf.NJ * gf.NK;
   if (!uf_pi) uf_pi = uf + 4 * gf.fs;
-  prolong_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(gf, uf, uf_pi, Prolong{gc, c_old, c_new, alpha}, nbuf);
+  launch_pdl(prolong_kernel, (unsigned)((n + 255) / 256), 256, 0, st, gf, uf, uf_pi, Prolong{gc, c_old, c_new, alpha},
+             nbuf);
   return 0;
+}
+
+// Of the coarser level's state at its step's start the prolongation reads the few
+// columns about the fine level's edge, so only these are kept in the place of the
+// whole state (three levels of RK4 on 512 x 33 x 65, twelve copies: 8.41 -> 8.09 ms).
+void launch_keep_columns(const Grid& gc, const double2* u, double2* to, const Grid& gf, int nbuf, cudaStream_t st) {
+  const int lo = std::max((gf.NI - nbuf) / 2 - 1, 0), hi = std::min((gf.NI - 1) / 2 + 2, gc.NI - 1);
+  if (hi < lo) return;
+  const int nc = hi - lo + 1;
+  const long long n = (long long)nc * gc.NJ * gc.NK;
+  launch_pdl(columns_kernel, (unsigned)((n + 255) / 256), 256, 0, st, gc, u, to, lo, nc);
 }
 
 int launch_restrict(const Grid& gc, double2* uc, const Grid& gf, const double2* uf, int keep_out, cudaStream_t st) {
@@ -68,7 +94,7 @@ int launch_restrict(const Grid& gc, double2* uc, const Grid& gf, const double2* 
   const int nc = last_f / 2 + 1;            // coarse planes 0..nc-1
   if (nc < 1 || nc > gc.NI || gf.NJ != gc.NJ || gf.NK != gc.NK) return -1;
   const long long n = (long long)nc * gc.NJ * gc.NK;
-  restrict_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(gc, uc, gf, uf, nc);
+  launch_pdl(restrict_kernel, (unsigned)((n + 255) / 256), 256, 0, st, gc, uc, gf, uf, nc);
   return 0;
 }
 
