@@ -551,7 +551,7 @@ bool encode_state(CUtensorMap* tm, const Grid& g, const double2* base, int cols,
 // chunk costs c + 3 plane times, a launch whole waves of them, and half a chunk at
 // the end behind the tiles at the r ends, whose warps take the general path.  At
 // most 24 planes: longer chunks measured slower on large grids (1024 x 65 x 129,
-// pair 0: 668 us at 24, 710 at 32, 790 at 43, 714 at 16).
+// pair 0: 661 us at 24, 699 at 32, 712 at 43, 709 at 16).
 int pair_chunk(int planes, long long tiles) {
   int best = planes;
   double cost = 1e300;
@@ -615,10 +615,10 @@ int pair_dispatch(int pair, const PairLaunch& L, const double* rsg, int* err, cu
 // The pairs pay from about 17 tile planes per SM on: below that the march is a
 // serial chain of planes twice as long as a single stage's, on a few SMs, and the
 // two pole-row launches show.  us per RK4 step, four stage kernels against two
-// pairs (tile planes per SM): 64 x 17 x 33 (1) 46 / 57, 128 x 33 x 65 (9) 112 / 132,
-// 256 x 33 x 65 (17) 196 / 195, 2000 x 17 x 33 (31) 404 / 301, 512 x 33 x 65 (33)
-// 323 / 310, 301 x 46 x 90 (40) 409 / 365, 512 x 65 x 129 (131) 1110 / 930, 1024 x 65 x
-// 129 (256) 2168 / 1655.
+// pairs (tile planes per SM): 64 x 17 x 33 (1) 33 / 53, 128 x 33 x 65 (9) 101 / 121,
+// 256 x 33 x 65 (17) 191 / 181, 2000 x 17 x 33 (31) 377 / 285, 512 x 33 x 65 (33)
+// 317 / 298, 301 x 46 x 90 (40) 396 / 337, 512 x 65 x 129 (131) 1101 / 914, 1024 x 65 x
+// 129 (256) 2163 / 1643.
 bool rk4_pairs_pay(const Grid& g) {
   const long long tiles = (long long)((g.NI - 2 + PO - 1) / PO) * ((g.NJ - 6 + 7) / 8);
   return tiles * (g.Nz - 1) >= 17LL * 148;
