@@ -80,6 +80,28 @@ __device__ __forceinline__ double2 d4r(const Grid& g, const F& f, int ii, double
     r = csub(cadd(csub(f(ii - 2), rmul(8.0, f(ii - 1))), rmul(8.0, f(ii + 1))), f(ii + 2));
   return c2(r.x * res, r.y * res);
 }
+// what a point takes from the planes k+-1..3 of its own column: the dissipation's
+// neighbours, and the fourth-order differences (times 12 h) that psi_3 and Pi need
+struct Phi {
+  double2 ko[5];
+  double2 e;  // of alpha Pi + beta psi_1
+  double2 f;  // of gamma^rphi psi_1 + gamma^phiphi psi_3
+};
+template <class PF>
+__device__ __forceinline__ Phi cfg_phi(const CfgArgs& a, int q, const PF& P) {
+  const Metric& M = a.m;
+  Phi w;
+  double2 d[5];
+#pragma unroll
+  for (int v = 0; v < 5; ++v) {
+    const double2 m3 = P(v, -3), m2 = P(v, -2), m1 = P(v, -1), p1 = P(v, 1), p2 = P(v, 2), p3 = P(v, 3);
+    w.ko[v] = cadd(csub(cadd(m3, p3), rmul(6.0, cadd(m2, p2))), rmul(15.0, cadd(m1, p1)));
+    d[v] = csub(csub(m2, p2), rmul(8.0, csub(m1, p1)));
+  }
+  w.e = cadd(rmul(ldm(M.alpha, q), d[4]), rmul(ldm(M.beta, q), d[1]));
+  w.f = cadd(rmul(ldm(M.grp, q), d[1]), rmul(ldm(M.gpp, q), d[3]));
+  return w;
+}
 __device__ __forceinline__ double2 d4c(double2 m2, double2 m1, double2 p1, double2 p2, double res) {
   const double2 r = csub(cadd(csub(m2, rmul(8.0, m1)), rmul(8.0, p1)), p2);
   return c2(r.x * res, r.y * res);
@@ -104,11 +126,12 @@ constexpr double kSixth = 1.0 / 6.0;
 
 // RHS and RK4 combination at one interior point (ii, jj, k): rows 3..NJ-4, planes
 // 1..Nz-1 (the ghost fill behind every stage writes the others).  S(v, i, j) returns
-// variable v of the stage input at (i, j) on plane k, P(v, d) at the point's
-// own (ii, jj) on the plane d steps away in phi (d = -3..3, d != 0); the two kernels below differ only in where S and P read
-// from, so they produce the same bits.
-template <int KIND, class SF, class PF>
-__device__ __forceinline__ void cfg_point(const CfgArgs& a, int ii, int jj, int k, const SF& S, const PF& P) {
+// variable v of the stage input at (i, j) on plane k, w holds what the point's own
+// column gives on the planes around it (cfg_phi, whose P(v, d) is the value d planes
+// away); the two kernels below differ only in where S and P read from, so they
+// produce the same bits.
+template <int KIND, class SF>
+__device__ __forceinline__ void cfg_point(const CfgArgs& a, int ii, int jj, int k, const SF& S, const Phi& w) {
   const Grid& g = a.g;
   const Metric& M = a.m;
   const long long p = off3(g, ii, jj, k);
@@ -123,14 +146,10 @@ __device__ __forceinline__ void cfg_point(const CfgArgs& a, int ii, int jj, int 
     }
   } else {
     const double al = ldm(M.alpha, q), b1 = ldm(M.beta, q), sg = ldm(M.sqrtg, q), dxb = ldm(a.dxb4, q);
-    // alpha Pi + beta psi_1 on this plane (ES) and in the own column (EP)
+    // alpha Pi + beta psi_1 on this plane
     auto ES = [&](int i2, int j2) {
       const int q2 = off2(g, i2, j2);
       return cadd(rmul(ldm(M.alpha, q2), S(4, i2, j2)), rmul(ldm(M.beta, q2), S(1, i2, j2)));
-    };
-    auto EP = [&](int d) { return cadd(rmul(ldm(M.alpha, q), P(4, d)), rmul(ldm(M.beta, q), P(1, d))); };
-    auto Fp = [&](int d) {
-      return rmul(ldm(M.asg, q), cadd(rmul(ldm(M.grp, q), P(1, d)), rmul(ldm(M.gpp, q), P(3, d))));
     };
     // sqrt(gamma) carries the sign of sin(theta) through the pole: negative on the ghost rows
     auto H = [&](int j2) {
@@ -145,21 +164,21 @@ __device__ __forceinline__ void cfg_point(const CfgArgs& a, int ii, int jj, int 
       r[1] = cadd(cadd(d4r(g, fA, ii, a.rr), rmul(b1, d4r(g, fP, ii, a.rr))), rmul(dxb, ps1));
     }
     r[2] = d4c(ES(ii, jj - 2), ES(ii, jj - 1), ES(ii, jj + 1), ES(ii, jj + 2), a.rt);
-    r[3] = d4c(EP(-2), EP(-1), EP(1), EP(2), a.rp);
+    r[3] = rmul(a.rp, w.e);
     {
       auto fG = [&](int i2) {
         const int q2 = off2(g, i2, jj);
         return rmul(ldm(M.asg, q2), cadd(rmul(ldm(M.grr, q2), S(1, i2, jj)), rmul(ldm(M.grp, q2), S(3, i2, jj))));
       };
       auto fQ = [&](int i2) {
-        const double2 w = S(4, i2, jj);
+        const double2 x = S(4, i2, jj);
         const double s2 = ldm(M.sqrtg, off2(g, i2, jj));
-        return c2(w.x * s2, w.y * s2);
+        return c2(x.x * s2, x.y * s2);
       };
       const double rs = ldm(a.rsg, q);
       const double2 t1 = cqdiv(d4r(g, fG, ii, a.rr), sg, rs);
       const double2 t2 = cqdiv(d4c(H(jj - 2), H(jj - 1), H(jj + 1), H(jj + 2), a.rt), sg, rs);
-      const double2 t3 = cqdiv(d4c(Fp(-2), Fp(-1), Fp(1), Fp(2), a.rp), sg, rs);
+      const double2 t3 = cqdiv(rmul(a.rp, rmul(ldm(M.asg, q), w.f)), sg, rs);
       const double2 t4 = c2(pi.x * dxb, pi.y * dxb);
       const double2 t5 = cqdiv(rmul(b1, d4r(g, fQ, ii, a.rr)), sg, rs);
       const double2 t6 = rmul(ldm(M.am2, q), S(0, ii, jj));
@@ -174,7 +193,7 @@ __device__ __forceinline__ void cfg_point(const CfgArgs& a, int ii, int jj, int 
                                    S(v, ii + 1, jj), S(v, ii + 2, jj), S(v, ii + 3, jj))));
       s = cadd(s, rmul(a.kt, ko6(S(v, ii, jj - 3), S(v, ii, jj - 2), S(v, ii, jj - 1), S(v, ii, jj),
                                  S(v, ii, jj + 1), S(v, ii, jj + 2), S(v, ii, jj + 3))));
-      s = cadd(s, rmul(a.kp, ko6(P(v, -3), P(v, -2), P(v, -1), S(v, ii, jj), P(v, 1), P(v, 2), P(v, 3))));
+      s = cadd(s, rmul(a.kp, csub(w.ko[v], rmul(20.0, S(v, ii, jj)))));
       r[v] = s;
     }
   }
@@ -220,7 +239,7 @@ __global__ void __launch_bounds__(128) cfg_stage_kernel(CfgArgs a) {
   const double2* U = a.in;
   auto S = [&](int v, int i2, int j2) { return ldf(U + (long long)v * g.fs, off3(g, i2, j2, k)); };
   auto P = [&](int v, int d) { return ldf(U + (long long)v * g.fs, off3(g, ii, jj, kper(g, k, d))); };
-  cfg_point<KIND>(a, ii, jj, k, S, P);
+  cfg_point<KIND>(a, ii, jj, k, S, cfg_phi(a, off2(g, ii, jj), P));
 }
 
 // Tiled form: a CTA owns a 32 x 8 tile of (r, theta) columns of the interior rows
@@ -232,9 +251,14 @@ __global__ void __launch_bounds__(128) cfg_stage_kernel(CfgArgs a) {
 // and plane, each with its index arithmetic, did before).  With that, only the
 // interior rows and planes, the point-wise operands requested together and the fill
 // in one launch, 20 RK4 steps on 256 x 33 x 65 went from 13.3 to 9.7 ms (a stage 164
-// -> 125 us); the phi neighbours' latency from L2 bounds it.  Those (planes k+-1..3
-// of the thread's own column) are plain loads; the same values serve seven
-// consecutive planes of the march.  (Holding them in a rolling register window
+// -> 125 us).  The phi neighbours (planes k+-1..3 of the thread's own column) are plain
+// loads, and their latency from L2 bound it: read where the formulas name them, they
+// came in many short batches, some twice.  cfg_phi reads them first, ahead of the
+// wait for the tile, a variable's six together, and keeps seven sums of them: 9.64 ->
+// 7.92 ms, a stage 125 -> 99 us.  What bounds it now is the chain of one plane's
+// loads and fifteen stencils at 16 warps per SM.  Not kept: the point-wise operands
+// prefetched into L2 a plane ahead (7.99 ms), u^n staged in shared memory (9.2 ms,
+// with 8 KB of L1 left).  (Holding them in a rolling register window
 // instead needs 255 registers per thread and one CTA per SM, and ran the C0
 // grid at half the speed.)
 constexpr int CTI = 32, CTJ = 8, CRH = 4, CTH = 3;
@@ -279,13 +303,15 @@ __global__ void __launch_bounds__(CTI * CTJ, 2)
       if (tid == 0) load(k + 1, buf ^ 1);  // that buffer was last read before the barrier of the plane before
       last = k + 1;
     }
+    auto P = [&](int v, int d) { return lds(col + (long long)v * g.fs, (long long)kper(g, k, d) * g.plane); };
+    Phi w = {};
+    if (act) w = cfg_phi(a, off2(g, ii, jj), P);
     if (!mbar_wait_bounded(&bars[buf], (uint32_t)((k - k0) >> 1) & 1u)) timed_out = 1;
     if (act && !timed_out) {
       // every same-plane neighbour lies inside the halo tile
       const double2* T = tiles + (size_t)buf * 5 * CT_N + (ty + CTH) * CW + (tx + CRH);
       auto S = [&](int v, int i2, int j2) { return T[v * CT_N + (j2 - jj) * CW + (i2 - ii)]; };
-      auto P = [&](int v, int d) { return lds(col + (long long)v * g.fs, (long long)kper(g, k, d) * g.plane); };
-      cfg_point<KIND>(a, ii, jj, k, S, P);
+      cfg_point<KIND>(a, ii, jj, k, S, w);
     }
     failed = __syncthreads_or(timed_out) != 0;
   }
