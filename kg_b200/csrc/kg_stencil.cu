@@ -249,13 +249,14 @@ void launch_rhs(const Grid& g, const Metric& m, int metric_kind, const double2* 
 // First stage of a pair of RK4 stages (kg_pair.cu) on the theta rows 3 and NJ-4,
 // planes 1..Nz-1, with its x fill: what the pair's tiles next to a pole take as
 // their ghost row.  Two rows of the grid, so every neighbour comes from the caches.
+// The planes are the grid's x extent: y and z end at 65535 blocks, Nz does not.
 constexpr int POLE_T = 128;
 template <int PAIR, int MK>
 __global__ void __launch_bounds__(POLE_T) pole_rows_kernel(Grid g, Metric M, const double* rsg, const double2* X,
                                                            const double2* base, int inflow, double2* pole) {
   __shared__ double2 first[4][5];
-  const int ii = blockIdx.x * POLE_T + threadIdx.x;
-  const int side = blockIdx.y, k = 1 + blockIdx.z;
+  const int ii = blockIdx.z * POLE_T + threadIdx.x;
+  const int side = blockIdx.y, k = 1 + blockIdx.x;
   const int jj = side ? g.NJ - 4 : 3;
   const bool hold = ii == g.NI - 1 && inflow;
   const int ic = ii == g.NI - 1 ? ii - 1 : ii;  // the outer copy forms its source
@@ -291,7 +292,7 @@ __global__ void __launch_bounds__(POLE_T) pole_rows_kernel(Grid g, Metric M, con
 }
 
 void launch_pole_rows(int pair, const PairLaunch& L, const double* rsg, double2* pole, cudaStream_t st) {
-  const dim3 grid((L.g.NI + POLE_T - 1) / POLE_T, 2, L.g.Nz - 1);
+  const dim3 grid(L.g.Nz - 1, 2, (L.g.NI + POLE_T - 1) / POLE_T);
   auto kern = pair == 0 ? (L.metric_kind == MK_KS ? pole_rows_kernel<0, MK_KS> : pole_rows_kernel<0, MK_SCHW>)
                         : (L.metric_kind == MK_KS ? pole_rows_kernel<1, MK_KS> : pole_rows_kernel<1, MK_SCHW>);
   kern<<<grid, POLE_T, 0, st>>>(L.g, L.m, rsg, L.X, L.base, L.inflow, pole);

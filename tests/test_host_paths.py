@@ -1,0 +1,68 @@
+"""Host paths of libkg_b200.so that a GPU test cannot reach -- limits of launches,
+refused allocations and launches, a second device -- on the library's own objects
+linked with a CUDA runtime that launches nothing (fake_cudart.cpp)."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from kg_b200 import capi
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("the library's objects cannot be brought up to date here: no nvcc")
+    subprocess.run(["make", "-s", "-C", os.path.join(ROOT, "kg_b200", "csrc"), "-j4"], check=True)
+    objdir = os.path.join(ROOT, "_build", "kg")
+    src = os.path.join(ROOT, "kg_b200", "csrc")
+    objs = [os.path.join(objdir, f[:-3] + ".o") for f in sorted(os.listdir(src)) if f.endswith(".cu")]
+    out = str(tmp_path_factory.mktemp("fake") / "libkg_fake.so")
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    # -Bsymbolic: the runtime calls bind here even when the process has loaded the real runtime
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I", include, os.path.join(HERE, "fake_cudart.cpp"),
+                    *objs, "-o", out, "-Wl,-Bsymbolic,--no-undefined", "-lpthread"], check=True)
+    lib = C.CDLL(out)
+    for name, restype, argtypes in capi.SIGNATURES:
+        f = getattr(lib, name)
+        f.restype, f.argtypes = restype, argtypes
+    lib.fake_refuse_alloc.argtypes = [C.c_size_t]
+    lib.fake_refuse_kernel.argtypes = [C.c_char_p]
+    lib.fake_launches.argtypes = [C.c_char_p]
+    return lib
+
+
+class Solve:
+    def __init__(self, lib, Nx, Ny, Nz, device=0, metric=capi.KG_KERR_SCHILD):
+        self.lib, self.h = lib, C.c_void_p()
+        lib.fake_reset()
+        p = capi.KgParams(Nx=Nx, Ny=Ny, Nz=Nz, g_pts=2, xmin=1.8, xmax=20.0, tmax=1.0, CFL=0.25, M_bh=1.0, m=0.3,
+                          metric=metric, bc_rmax=capi.KG_OUTFLOW, n_det=2, l_max=2, save_=0.1)
+        assert lib.kg_create(C.byref(p), device, C.byref(self.h)) == capi.KG_OK
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        self.lib.kg_destroy(self.h)
+        self.lib.fake_reset()
+
+    def __call__(self, name, *args):
+        """status and error text of an entry point"""
+        rc = getattr(self.lib, name)(self.h, *args)
+        return rc, self.lib.kg_last_error(self.h).decode()
+
+
+@pytest.mark.parametrize("pairs", [0, 2])
+@pytest.mark.parametrize("Nz", [65534, 65535, 65536, 65537, 70000])
+def test_rk4_takes_more_planes_than_a_launch_has_blocks_in_z(fake, Nz, pairs):
+    with Solve(fake, 4, 5, Nz) as s:
+        assert s("kg_set_rk4_pairs", pairs)[0] == capi.KG_OK
+        assert s("kg_rk4", 1) == (capi.KG_OK, "")
+        assert s("kg_rk4", 3) == (capi.KG_OK, "")
