@@ -62,6 +62,7 @@ struct kg_solver {
   // that a solve created after another has gone takes over its blocks one for one
   double2* RK[3] = {nullptr, nullptr, nullptr};
   double2* pole = nullptr;               // first-stage rows next to the poles (kg_pair.cu)
+  bool no_pairs = false;                 // there was no room for them: four stages from then on
   // u as a ghost fill leaves it: plane 0 = plane Nz-1 and plane Nz = plane 1 in
   // every row, which the paired stages take for granted.  Cleared by whatever
   // writes u otherwise.
@@ -1261,14 +1262,24 @@ bool wants_pairs(const kg_solver* h) {
   return h->variant >= 2 && (h->rk4_pairs == 2 || (h->rk4_pairs == 1 && kg::rk4_pairs_pay(h->g)));
 }
 
+// Room for the pole rows, asked for once in a handle's life.  A refusal is no error:
+// the four stage kernels run instead, in this step and in all later ones, so that
+// the captured steps behind a direct one never ask again.
+bool has_pole_rows(kg_solver* h) {
+  if (!h->pole && !h->no_pairs) {
+    const std::string err = h->err;
+    h->no_pairs = dalloc(h, (void**)&h->pole, (size_t)10 * h->NK * h->PI * sizeof(double2)) != KG_OK;
+    h->err = err;
+  }
+  return h->pole != nullptr;
+}
+
 int step_rk4(kg_solver* h, int nsteps) {
   int rc;
   if ((rc = ensure_rk(h, 3))) return rc;
-  // without room for the pole rows the four stage kernels run instead
-  const bool pairs = wants_pairs(h);
-  if (pairs && !h->pole) (void)dalloc(h, (void**)&h->pole, (size_t)10 * h->NK * h->PI * sizeof(double2));
+  const bool pairs = wants_pairs(h) && has_pole_rows(h);
   for (int s = 0; s < nsteps;) {
-    if (!pairs || !h->pole || !h->seam_filled) {
+    if (!pairs || !h->seam_filled) {
       rk4_step_single(h);
       ++s;
       continue;

@@ -66,3 +66,18 @@ def test_rk4_takes_more_planes_than_a_launch_has_blocks_in_z(fake, Nz, pairs):
         assert s("kg_set_rk4_pairs", pairs)[0] == capi.KG_OK
         assert s("kg_rk4", 1) == (capi.KG_OK, "")
         assert s("kg_rk4", 3) == (capi.KG_OK, "")
+
+
+def test_refused_pole_rows_leave_the_four_stages(fake):
+    """no room for the pairs' pole rows: asked for once, outside any capture, and no
+    error of a step that the four stage kernels then take"""
+    Nx, Ny, Nz = 300, 30, 60
+    with Solve(fake, Nx, Ny, Nz) as s:
+        assert s("kg_set_rk4_pairs", 2)[0] == capi.KG_OK
+        fake.fake_refuse_alloc(10 * (Nz + 1) * ((Nx + 5 + 7) // 8 * 8) * 16)
+        for n in (6, 6, 1, 3):
+            assert s("kg_rk4", n) == (capi.KG_OK, "")
+        assert fake.fake_refused() == 2  # dalloc tries again behind a trim of the pool
+        assert fake.fake_capture_allocs() == 0
+        assert fake.fake_launches(b"rk4_pair") == 0
+        assert fake.fake_launches(b"tma_stage") > 0
