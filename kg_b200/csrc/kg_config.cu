@@ -386,13 +386,8 @@ bool cfg_encode(CUtensorMap* tm, const Grid& g, const double2* base) {
 
 template <int KIND>
 int cfg_march_launch(const CfgArgs& a, cudaStream_t st) {
-  static bool attr = false;  // dynamic shared memory above 48 KB, set once per stage kind
   constexpr int SMEM = 2 * (int)CFG_TILE_BYTES + 128;
-  if (!attr) {
-    if (cudaFuncSetAttribute(cfg_march_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
-      return -1;
-    attr = true;
-  }
+  if (!allow_smem<cfg_march_kernel<KIND>>(SMEM)) return -1;
   const Grid& g = a.g;
   CUtensorMap tm;
   if (!cfg_encode(&tm, g, a.in)) return -1;

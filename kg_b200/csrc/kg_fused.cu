@@ -510,13 +510,7 @@ bool encode_box(CUtensorMap* tm, const Grid& g, const double2* base, int nvars, 
 
 template <int MK>
 int fused_launch(const CUtensorMap* tms, FusedArgs a, cudaStream_t st) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(pirk_s1_fused_kernel<MK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) !=
-        cudaSuccess)
-      return -1;
-    attr_set = true;
-  }
+  if (!allow_smem<pirk_s1_fused_kernel<MK>>(SMEM)) return -1;
   const Grid& g = a.g;
   const int tiles_x = (g.NI <= FO) ? 1 : (g.NI + FO - 1) / FO;
   dim3 grid(tiles_x, (g.NJ + FJ - 1) / FJ, 1);

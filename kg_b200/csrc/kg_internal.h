@@ -2,6 +2,7 @@
 // libkg_b200.so (not part of the public C ABI).
 #pragma once
 #include <cuda_runtime.h>
+#include <atomic>
 #include "kg_device.cuh"
 
 namespace kg {
@@ -75,6 +76,20 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+// Dynamic shared memory above 48 KB has to be allowed on every device that launches
+// the kernel: one bit a device, set once it is (devices beyond 64 at every launch).
+template <auto Kernel>
+inline bool allow_smem(size_t bytes) {
+  static std::atomic<unsigned long long> allowed{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (e == cudaSuccess && (allowed.load() & bit)) return true;
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e != cudaSuccess) return false;
+  allowed.fetch_or(bit);
+  return true;
 }
 // until the kernel before this one has finished and its writes are visible
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -651,13 +651,7 @@ template <int KIND, int MK, class TIN, int TJ>
 int mx_launch_one(const CUtensorMap& tin, const CUtensorMap& tp0, const CUtensorMap& tp1, MxArgs a,
                   cudaStream_t st) {
   constexpr size_t SMEM = MGeom<TJ>::template smem<TIN>();
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(mx_stage_kernel<KIND, MK, TIN, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)SMEM) != cudaSuccess)
-      return -1;
-    attr = true;
-  }
+  if (!allow_smem<mx_stage_kernel<KIND, MK, TIN, TJ>>(SMEM)) return -1;
   const Grid& g = a.g;
   const int planes = g.NK - 1;
   dim3 grid((g.NI + TI - 1) / TI, (g.NJ - 6 + TJ - 1) / TJ, 1);
@@ -684,13 +678,7 @@ int mx_launch_mk(int kind, const CUtensorMap& tin, const CUtensorMap& tp0, const
 template <int KIND, int MK, class TIN, int TJ>
 int mx_batch_one(const void* items, int n_solves, int n_items, int blocks, BatchCounter* ctr, cudaStream_t st) {
   constexpr size_t SMEM = MGeom<TJ>::template smem<TIN>();
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(mx_batch_kernel<KIND, MK, TIN, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)SMEM) != cudaSuccess)
-      return -1;
-    attr = true;
-  }
+  if (!allow_smem<mx_batch_kernel<KIND, MK, TIN, TJ>>(SMEM)) return -1;
   if (n_items <= 0) return 0;
   return launch_pdl(mx_batch_kernel<KIND, MK, TIN, TJ>, blocks, dim3(TI, TJ, 1), SMEM, st,
                     reinterpret_cast<const MxItem*>(items), n_solves, n_items, ctr) == cudaSuccess

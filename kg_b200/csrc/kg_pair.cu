@@ -570,13 +570,7 @@ int pair_chunk(int planes, long long tiles) {
 template <int PAIR, int MK, int TJ>
 int pair_launch(const PairLaunch& L, const double* rsg, int* err, cudaStream_t st) {
   using GT = PGeom<TJ>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(rk4_pair_kernel<PAIR, MK, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)GT::SMEM) != cudaSuccess)
-      return -1;
-    attr_set = true;
-  }
+  if (!allow_smem<rk4_pair_kernel<PAIR, MK, TJ>>(GT::SMEM)) return -1;
   const Grid& g = L.g;
   CUtensorMap tmX, tmU, tmA;
   if (!encode_state(&tmX, g, L.X, PW, GT::ROWS) || !encode_state(&tmU, g, L.base, 32, GT::WARPS) ||

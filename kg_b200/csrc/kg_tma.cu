@@ -622,13 +622,7 @@ struct Maps {
 template <int KIND, int MK, int TJ>
 int launch_one(const Maps& m, TmaArgs a, cudaStream_t st) {
   constexpr size_t SMEM = Geom<TJ>::SMEM_BYTES;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(tma_stage_kernel<KIND, MK, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)SMEM) != cudaSuccess)
-      return -1;
-    attr_set = true;
-  }
+  if (!allow_smem<tma_stage_kernel<KIND, MK, TJ>>(SMEM)) return -1;
   const Grid& g = a.g;
   dim3 block(TI, TJ, 1);
   const int planes = plane_end<KIND>(g), rows = row_end<KIND>(g) - row_first<KIND>();
@@ -719,13 +713,7 @@ namespace {
 template <int KIND, int MK, int TJ>
 int batch_one(const void* items, int n_solves, int n_items, int blocks, BatchCounter* ctr, cudaStream_t st) {
   constexpr size_t SMEM = Geom<TJ>::SMEM_BYTES;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(tma_batch_kernel<KIND, MK, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)SMEM) != cudaSuccess)
-      return -1;
-    attr_set = true;
-  }
+  if (!allow_smem<tma_batch_kernel<KIND, MK, TJ>>(SMEM)) return -1;
   if (n_items <= 0) return 0;
   return launch_pdl(tma_batch_kernel<KIND, MK, TJ>, blocks, dim3(TI, TJ, 1), SMEM, st,
                     reinterpret_cast<const BatchItem*>(items), n_solves, n_items, ctr) == cudaSuccess

@@ -502,13 +502,7 @@ int launch_ylm_gemm(const __nv_bfloat16* Ahi, const __nv_bfloat16* Alo, const __
   if (!map_kmajor(&a0, Ahi, Kp, Mp, BM) || !map_kmajor(&a1, Alo, Kp, Mp, BM) || !map_kmajor(&b0, Bhi, Kp, Np, BN) ||
       !map_kmajor(&b1, Blo, Kp, Np, BN))
     return -1;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(ylm_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM) !=
-        cudaSuccess)
-      return -1;
-    attr = true;
-  }
+  if (!allow_smem<ylm_gemm_kernel>(GEMM_SMEM)) return -1;
   ylm_gemm_kernel<<<dim3(Np / BN, Mp / BM, ylm_gemm_splits(Kp)), 128, GEMM_SMEM, st>>>(
       a0, a1, b0, b1, C, Np, Mp, Np, Kp, (long long)Mp * Np, err);
   return 0;

@@ -81,3 +81,33 @@ def test_refused_pole_rows_leave_the_four_stages(fake):
         assert fake.fake_capture_allocs() == 0
         assert fake.fake_launches(b"rk4_pair") == 0
         assert fake.fake_launches(b"tma_stage") > 0
+
+
+@pytest.mark.parametrize("metric", [capi.KG_KERR_SCHILD, capi.KG_SCHW_EF])
+def test_every_kernel_launches_on_a_second_device(fake, metric):
+    """what a launch needs is set on the device that launches, not once a process"""
+    seen = []
+    for device in (0, 1):
+        with Solve(fake, 60, 12, 20, device=device, metric=metric) as s:
+            for name in ("kg_pirk2", "kg_pirk3", "kg_rk3", "kg_rk4"):
+                assert s(name, 1) == (capi.KG_OK, "")
+            for rows in (4, 8):
+                for precision in (0, 1):
+                    for pairs in (0, 2):
+                        s("kg_set_tile_rows", rows), s("kg_set_precision", precision), s("kg_set_rk4_pairs", pairs)
+                        assert s("kg_rk4", 2) == (capi.KG_OK, "")
+                    b = C.c_void_p()
+                    assert fake.kg_batch_create(device, C.byref(b)) == capi.KG_OK
+                    assert fake.kg_batch_set_precision(b, precision) == capi.KG_OK
+                    assert fake.kg_batch_set_tile_rows(b, rows) == capi.KG_OK
+                    assert fake.kg_batch_add(b, s.h) == capi.KG_OK
+                    assert fake.kg_batch_rk4(b, 2) == capi.KG_OK, fake.kg_batch_last_error(b)
+                    assert fake.kg_batch_destroy(b) == capi.KG_OK
+            alm = (C.c_double * (2 * 3 * 5 * 60))()
+            assert s("kg_project_all_shells", 2, 1, alm) == (capi.KG_OK, "")
+            if metric == capi.KG_KERR_SCHILD:
+                assert s("kg_set_precision", 0)[0] == s("kg_set_scheme", 1, 0.02)[0] == capi.KG_OK
+                assert s("kg_rk4", 2) == (capi.KG_OK, "")
+            seen.append([fake.fake_launches(k) for k in (b"tma_stage", b"tma_batch", b"mx_stage", b"mx_batch", b"rk4_pair",
+                                                         b"pirk_s1_fused", b"cfg_march", b"ylm_gemm", b"2kg12march_kernel")])
+    assert seen[0] == seen[1] and all(seen[0][:6]) and not seen[0][-1]
