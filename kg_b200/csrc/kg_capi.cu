@@ -62,7 +62,7 @@ struct kg_solver {
   // that a solve created after another has gone takes over its blocks one for one
   double2* RK[3] = {nullptr, nullptr, nullptr};
   double2* pole = nullptr;               // first-stage rows next to the poles (kg_pair.cu)
-  bool no_pairs = false;                 // there was no room for them: four stages from then on
+  bool no_pairs = false;                 // no room for them, or a pair's launch refused: four stages from then on
   // u as a ghost fill leaves it: plane 0 = plane Nz-1 and plane Nz = plane 1 in
   // every row, which the paired stages take for granted.  Cleared by whatever
   // writes u otherwise.
@@ -1223,8 +1223,9 @@ void rk4_step_single(kg_solver* h) {
 }
 
 // one RK4 step of two paired kernels (kg_pair.cu), u in `from` -> u in `to`; the
-// other of the two buffers is the first stage buffer R1, which pairs do not use
-int rk4_step_pairs(kg_solver* h, double2* from, double2* to) {
+// other of the two buffers is the first stage buffer R1, which pairs do not use.
+// false: a launch was refused, with u in `from` as it was
+bool rk4_step_pairs(kg_solver* h, double2* from, double2* to) {
   const Grid& g = h->g;
   const int inflow = h->p.bc_rmax == KG_INFLOW;
   const double* rsg = h->dmet + (size_t)T_RSG * h->NJ * h->PI;
@@ -1248,18 +1249,21 @@ int rk4_step_pairs(kg_solver* h, double2* from, double2* to) {
     }
     {
       Prof pf(h, pair ? PK_PAIR34 : PK_PAIR12, 1);
-      if (kg::launch_rk4_pair(pair, L, rsg, h->derr, h->stream))
-        return set_err(h, KG_ECUDA, "paired RK4 stages could not be configured (tensor maps)");
+      if (kg::launch_rk4_pair(pair, L, rsg, h->derr, h->stream)) {
+        pf.n = 0;
+        h->no_pairs = true;
+        return false;
+      }
     }
     run_ghost(h, L.out, from, inflow, false, true);
   }
   h->t = h->t + h->dt;
-  return KG_OK;
+  return true;
 }
 
 // the paired form (kg_pair.cu): with the TMA stage forms, where it pays
 bool wants_pairs(const kg_solver* h) {
-  return h->variant >= 2 && (h->rk4_pairs == 2 || (h->rk4_pairs == 1 && kg::rk4_pairs_pay(h->g)));
+  return !h->no_pairs && h->variant >= 2 && (h->rk4_pairs == 2 || (h->rk4_pairs == 1 && kg::rk4_pairs_pay(h->g)));
 }
 
 // Room for the pole rows, asked for once in a handle's life.  A refusal is no error:
@@ -1277,18 +1281,16 @@ bool has_pole_rows(kg_solver* h) {
 int step_rk4(kg_solver* h, int nsteps) {
   int rc;
   if ((rc = ensure_rk(h, 3))) return rc;
-  const bool pairs = wants_pairs(h) && has_pole_rows(h);
   for (int s = 0; s < nsteps;) {
-    if (!pairs || !h->seam_filled) {
+    if (!wants_pairs(h) || !has_pole_rows(h) || !h->seam_filled) {
       rk4_step_single(h);
       ++s;
       continue;
     }
-    // two steps, u -> R1 -> u; a last odd one is copied back
-    if ((rc = rk4_step_pairs(h, h->U, h->RK[0]))) return rc;
+    // two steps, u -> R1 -> u; a last odd one is copied back, as is u behind a refused second one
+    if (!rk4_step_pairs(h, h->U, h->RK[0])) continue;
     ++s;
-    if (s < nsteps) {
-      if ((rc = rk4_step_pairs(h, h->RK[0], h->U))) return rc;
+    if (s < nsteps && rk4_step_pairs(h, h->RK[0], h->U)) {
       ++s;
     } else {
       KG_CK(cudaMemcpyAsync(h->U, h->RK[0], 5 * field_bytes(h), cudaMemcpyDeviceToDevice, h->stream));

@@ -393,10 +393,8 @@ int cfg_march_launch(const CfgArgs& a, cudaStream_t st) {
   if (!cfg_encode(&tm, g, a.in)) return -1;
   const int tx = (g.NI + CTI - 1) / CTI, ty = (g.NJ - 6 + CTJ - 1) / CTJ, planes = g.Nz - 1;
   const int kchunk = phi_chunk(planes, (long long)tx * ty, 148 * 2, 32);
-  return launch_pdl(cfg_march_kernel<KIND>, dim3(tx, ty, (planes + kchunk - 1) / kchunk), dim3(CTI, CTJ, 1), SMEM, st,
-                    tm, a, kchunk) == cudaSuccess
-             ? 0
-             : -1;
+  return launch_pdl_or_refuse(cfg_march_kernel<KIND>, dim3(tx, ty, (planes + kchunk - 1) / kchunk), dim3(CTI, CTJ, 1),
+                              SMEM, st, tm, a, kchunk);
 }
 
 }  // namespace

@@ -516,10 +516,8 @@ int fused_launch(const CUtensorMap* tms, FusedArgs a, cudaStream_t st) {
   dim3 grid(tiles_x, (g.NJ + FJ - 1) / FJ, 1);
   a.kchunk = phi_chunk(g.NK, (long long)grid.x * grid.y, 148 * 2, 64);
   grid.z = (g.NK + a.kchunk - 1) / a.kchunk;
-  return launch_pdl(pirk_s1_fused_kernel<MK>, grid, dim3(FL, FJ, 1), SMEM, st, tms[0], tms[1], tms[2], tms[3], a) ==
-                 cudaSuccess
-             ? 0
-             : -1;
+  return launch_pdl_or_refuse(pirk_s1_fused_kernel<MK>, grid, dim3(FL, FJ, 1), SMEM, st, tms[0], tms[1], tms[2],
+                              tms[3], a);
 }
 
 }  // namespace

@@ -77,17 +77,34 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
+// The same for a kernel that has another form to fall back on, or whose refusal the
+// caller reports: 0, or -1 with the refusal taken out of the thread's last-error
+// slot, where it would fail the next call that looks there (an error that was in the
+// slot before stays).
+template <class... P, class... A>
+inline int launch_pdl_or_refuse(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                const A&... args) {
+  const bool clear = cudaPeekAtLastError() == cudaSuccess;
+  if (launch_pdl(kernel, grid, block, smem, st, args...) == cudaSuccess) return 0;
+  if (clear) cudaGetLastError();
+  return -1;
+}
+
 // Dynamic shared memory above 48 KB has to be allowed on every device that launches
 // the kernel: one bit a device, set once it is (devices beyond 64 at every launch).
 template <auto Kernel>
 inline bool allow_smem(size_t bytes) {
   static std::atomic<unsigned long long> allowed{0};
+  const bool clear = cudaPeekAtLastError() == cudaSuccess;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
   if (e == cudaSuccess && (allowed.load() & bit)) return true;
   if (e == cudaSuccess) e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) return false;
+  if (e != cudaSuccess) {
+    if (clear) cudaGetLastError();
+    return false;
+  }
   allowed.fetch_or(bit);
   return true;
 }

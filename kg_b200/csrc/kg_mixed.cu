@@ -657,10 +657,7 @@ int mx_launch_one(const CUtensorMap& tin, const CUtensorMap& tp0, const CUtensor
   dim3 grid((g.NI + TI - 1) / TI, (g.NJ - 6 + TJ - 1) / TJ, 1);
   a.kchunk = phi_chunk(planes, (long long)grid.x * grid.y, 148 * MGeom<TJ>::MIN_BLOCKS, 32);
   grid.z = (planes + a.kchunk - 1) / a.kchunk;
-  return launch_pdl(mx_stage_kernel<KIND, MK, TIN, TJ>, grid, dim3(TI, TJ, 1), SMEM, st, tin, tp0, tp1, a) ==
-                 cudaSuccess
-             ? 0
-             : -1;
+  return launch_pdl_or_refuse(mx_stage_kernel<KIND, MK, TIN, TJ>, grid, dim3(TI, TJ, 1), SMEM, st, tin, tp0, tp1, a);
 }
 
 template <int MK, int TJ>
@@ -680,10 +677,8 @@ int mx_batch_one(const void* items, int n_solves, int n_items, int blocks, Batch
   constexpr size_t SMEM = MGeom<TJ>::template smem<TIN>();
   if (!allow_smem<mx_batch_kernel<KIND, MK, TIN, TJ>>(SMEM)) return -1;
   if (n_items <= 0) return 0;
-  return launch_pdl(mx_batch_kernel<KIND, MK, TIN, TJ>, blocks, dim3(TI, TJ, 1), SMEM, st,
-                    reinterpret_cast<const MxItem*>(items), n_solves, n_items, ctr) == cudaSuccess
-             ? 0
-             : -1;
+  return launch_pdl_or_refuse(mx_batch_kernel<KIND, MK, TIN, TJ>, blocks, dim3(TI, TJ, 1), SMEM, st,
+                              reinterpret_cast<const MxItem*>(items), n_solves, n_items, ctr);
 }
 
 template <int MK, int TJ>

@@ -590,10 +590,8 @@ int pair_launch(const PairLaunch& L, const double* rsg, int* err, cudaStream_t s
   dim3 grid((g.NI - 2 + PO - 1) / PO, (g.NJ - 6 + TJ - 1) / TJ, 1);
   a.kchunk = pair_chunk(g.Nz - 1, (long long)grid.x * grid.y);
   grid.z = (g.Nz - 1 + a.kchunk - 1) / a.kchunk;
-  return launch_pdl(rk4_pair_kernel<PAIR, MK, TJ>, grid, dim3(32, GT::WARPS), GT::SMEM, st, tmX, tmU, tmA, a) ==
-                 cudaSuccess
-             ? 0
-             : -1;
+  return launch_pdl_or_refuse(rk4_pair_kernel<PAIR, MK, TJ>, grid, dim3(32, GT::WARPS), GT::SMEM, st, tmX, tmU,
+                              tmA, a);
 }
 template <int TJ>
 int pair_dispatch(int pair, const PairLaunch& L, const double* rsg, int* err, cudaStream_t st) {

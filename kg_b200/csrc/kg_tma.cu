@@ -629,9 +629,7 @@ int launch_one(const Maps& m, TmaArgs a, cudaStream_t st) {
   dim3 grid((g.NI + TI - 1) / TI, (rows + TJ - 1) / TJ, 1);
   a.kchunk = phi_chunk(planes, (long long)grid.x * grid.y, 148 * Geom<TJ>::MIN_BLOCKS, 32);
   grid.z = (planes + a.kchunk - 1) / a.kchunk;
-  return launch_pdl(tma_stage_kernel<KIND, MK, TJ>, grid, block, SMEM, st, m.tm4, m.tm1, m.tp0, m.tp1, a) == cudaSuccess
-             ? 0
-             : -1;
+  return launch_pdl_or_refuse(tma_stage_kernel<KIND, MK, TJ>, grid, block, SMEM, st, m.tm4, m.tm1, m.tp0, m.tp1, a);
 }
 
 // the 4-row tiles are built for the RK4 stages (the batched forms' stepper) only
@@ -715,10 +713,8 @@ int batch_one(const void* items, int n_solves, int n_items, int blocks, BatchCou
   constexpr size_t SMEM = Geom<TJ>::SMEM_BYTES;
   if (!allow_smem<tma_batch_kernel<KIND, MK, TJ>>(SMEM)) return -1;
   if (n_items <= 0) return 0;
-  return launch_pdl(tma_batch_kernel<KIND, MK, TJ>, blocks, dim3(TI, TJ, 1), SMEM, st,
-                    reinterpret_cast<const BatchItem*>(items), n_solves, n_items, ctr) == cudaSuccess
-             ? 0
-             : -1;
+  return launch_pdl_or_refuse(tma_batch_kernel<KIND, MK, TJ>, blocks, dim3(TI, TJ, 1), SMEM, st,
+                              reinterpret_cast<const BatchItem*>(items), n_solves, n_items, ctr);
 }
 template <int KIND>
 int batch_kind(const void* items, int n_solves, int n_items, int blocks, int mk, int tj, BatchCounter* ctr,

@@ -178,6 +178,7 @@ cudaError_t cudaGetLastError() {
   last = cudaSuccess;
   return e;
 }
+cudaError_t cudaPeekAtLastError() { return last; }
 const char* cudaGetErrorString(cudaError_t e) {
   static thread_local std::string s;
   s = "error " + std::to_string((int)e);

@@ -25,9 +25,9 @@ def fake(tmp_path_factory):
     objs = [os.path.join(objdir, f[:-3] + ".o") for f in sorted(os.listdir(src)) if f.endswith(".cu")]
     out = str(tmp_path_factory.mktemp("fake") / "libkg_fake.so")
     include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
-    # -Bsymbolic: the runtime calls bind here even when the process has loaded the real runtime
-    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I", include, os.path.join(HERE, "fake_cudart.cpp"),
-                    *objs, "-o", out, "-Wl,-Bsymbolic,--no-undefined", "-lpthread"], check=True)
+    # -Bsymbolic: the runtime calls bind here even when the real runtime is loaded as well
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I", include,
+                    os.path.join(HERE, "fake_cudart.cpp"), *objs, "-o", out, "-Wl,-Bsymbolic,--no-undefined", "-lpthread"], check=True)
     lib = C.CDLL(out)
     for name, restype, argtypes in capi.SIGNATURES:
         f = getattr(lib, name)
@@ -108,6 +108,51 @@ def test_every_kernel_launches_on_a_second_device(fake, metric):
             if metric == capi.KG_KERR_SCHILD:
                 assert s("kg_set_precision", 0)[0] == s("kg_set_scheme", 1, 0.02)[0] == capi.KG_OK
                 assert s("kg_rk4", 2) == (capi.KG_OK, "")
-            seen.append([fake.fake_launches(k) for k in (b"tma_stage", b"tma_batch", b"mx_stage", b"mx_batch", b"rk4_pair",
-                                                         b"pirk_s1_fused", b"cfg_march", b"ylm_gemm", b"2kg12march_kernel")])
+            seen.append([fake.fake_launches(k)
+                         for k in (b"tma_stage", b"tma_batch", b"mx_stage", b"mx_batch", b"rk4_pair", b"pirk_s1_fused",
+                                   b"cfg_march", b"ylm_gemm", b"2kg12march_kernel")])
     assert seen[0] == seen[1] and all(seen[0][:6]) and not seen[0][-1]
+
+
+REFUSED = [("tma_stage_kernel", "kg_pirk2", "2kg12march_kernel"), ("tma_stage_kernel", "kg_pirk3", "2kg12march_kernel"),
+           ("tma_stage_kernel", "kg_rk3", "2kg12march_kernel"), ("tma_stage_kernel", "kg_rk4", "2kg12march_kernel"),
+           ("pirk_s1_fused", "kg_pirk2", "tma_stage_kernel"), ("pirk_s1_fused", "kg_pirk3", "tma_stage_kernel"),
+           ("cfg_march_kernel", "configured", "cfg_stage_kernel"),
+           ("rk4_pair_kernelILi0", "paired", "tma_stage_kernel"), ("rk4_pair_kernelILi1", "paired", "tma_stage_kernel")]
+
+
+@pytest.mark.parametrize("kernel,call,instead", REFUSED)
+@pytest.mark.parametrize("later", [False, True])
+def test_refused_launch_takes_the_other_form(fake, kernel, call, instead, later):
+    """a launch that the device refuses -- at once, or behind steps that it took -- is
+    no error of a step that another form takes, nor of the calls after it"""
+    with Solve(fake, 40, 12, 20) as s:
+        name = call if call.startswith("kg_") else "kg_rk4"
+        assert s("kg_set_rk4_pairs", 2 if call == "paired" else 0)[0] == capi.KG_OK
+        if call == "configured":
+            assert s("kg_set_scheme", 1, 0.02)[0] == capi.KG_OK
+        assert s(name, 3 if later else 0)[0] == capi.KG_OK
+        sc = (C.c_double * 9)()
+        assert s("kg_get_scalars", sc)[0] == capi.KG_OK
+        t, dt = sc[4], sc[3]
+        fake.fake_refuse_kernel(kernel.encode())
+        before = fake.fake_launches(instead.encode())
+        assert s("kg_set_graphs", 0)[0] == capi.KG_OK
+        for n in (1, 4, 3):
+            assert s(name, n) == (capi.KG_OK, "")
+            for _ in range(n):
+                t = t + dt
+        assert fake.fake_launches(instead.encode()) > before
+        assert s("kg_get_scalars", sc)[0] == capi.KG_OK and sc[4] == t
+        fake.fake_refuse_kernel(None)
+        assert s(name, 2) == (capi.KG_OK, "")
+        assert fake.fake_last_error() == 0
+
+
+@pytest.mark.parametrize("kernel", ["mx_stage_kernelILi9", "mx_stage_kernelILi11"])
+def test_refused_mixed_stage_does_not_fail_the_next_call(fake, kernel):
+    with Solve(fake, 40, 12, 20) as s:
+        assert s("kg_set_precision", 1)[0] == capi.KG_OK
+        fake.fake_refuse_kernel(kernel.encode())
+        assert s("kg_rk4", 1)[0] == capi.KG_ECUDA
+        assert s("kg_pirk2", 1)[0] == capi.KG_OK
