@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <atomic>
+#include "kg_chunk.h"
 #include "kg_device.cuh"
 
 namespace kg {
@@ -23,34 +24,6 @@ enum StageKind {
   ST_RK4_3,
   ST_RK4_4
 };
-
-// Phi planes per chunk of a marching kernel: `planes` planes of each of `tiles`
-// (r, theta) tiles, on `slots` CTAs that run at once, at most `longest` planes.
-// A chunk of c planes costs c + 1 plane times (its two halo planes and its
-// prologue overlap the other CTA of the SM) and the launch's last wave a quarter
-// of a chunk, so the rule takes the c that minimises
-//   max(1, tiles * chunks / slots + 1/4) * (c + 1);
-// a grid whose tiles alone leave SMs idle gets short chunks, a large one the
-// longest.  Constants fitted to a sweep of 19 lengths over ten grids from
-// 64 x 17 x 33 to 1024 x 65 x 129 (within 2 % of the best length on average, 14 %
-// at worst).  Against chunks of about 32 planes on every grid (64 in the fused PIRK stage 1),
-// us per launch: 64 x 17 x 33 PIRK2 stage 2 71 -> 12 and fused stage 1 94 -> 18,
-// 256 x 33 x 65 66 -> 37 and 103 -> 52, RK4 stage 2 98 -> 55.
-inline int phi_chunk(int planes, long long tiles, int slots, int longest, int extra = 1) {
-  int best = planes;
-  double cost = 1e300;
-  for (int n = (planes + longest - 1) / longest; n <= planes; ++n) {
-    const int c = (planes + n - 1) / n;
-    const int m = (planes + c - 1) / c;
-    const double waves = (double)tiles * m / slots + 0.25;
-    const double t = (waves > 1.0 ? waves : 1.0) * (c + extra);
-    if (t < cost) {
-      cost = t;
-      best = c;
-    }
-  }
-  return best;
-}
 
 // Launches a kernel whose blocks may be set up while the last blocks of the
 // kernel before it on the stream finish (programmatic dependent launch), so that

@@ -547,26 +547,6 @@ bool encode_state(CUtensorMap* tm, const Grid& g, const double2* base, int cols,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Phi planes per chunk.  One CTA runs on an SM at a time, so its start shows: a
-// chunk costs c + 3 plane times, a launch whole waves of them, and half a chunk at
-// the end behind the tiles at the r ends, whose warps take the general path.  At
-// most 24 planes: longer chunks measured slower on large grids (1024 x 65 x 129,
-// pair 0: 661 us at 24, 699 at 32, 712 at 43, 709 at 16).
-int pair_chunk(int planes, long long tiles) {
-  int best = planes;
-  double cost = 1e300;
-  for (int n = (planes + 23) / 24; n <= planes; ++n) {
-    const int c = (planes + n - 1) / n;
-    const int m = (planes + c - 1) / c;
-    const double t = ((double)((tiles * m + 147) / 148) + 0.5) * (c + 3);
-    if (t < cost) {
-      cost = t;
-      best = c;
-    }
-  }
-  return best;
-}
-
 template <int PAIR, int MK, int TJ>
 int pair_launch(const PairLaunch& L, const double* rsg, int* err, cudaStream_t st) {
   using GT = PGeom<TJ>;

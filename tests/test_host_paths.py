@@ -5,6 +5,7 @@ import ctypes as C
 import os
 import shutil
 import subprocess
+import time
 
 import pytest
 
@@ -156,3 +157,38 @@ def test_refused_mixed_stage_does_not_fail_the_next_call(fake, kernel):
         fake.fake_refuse_kernel(kernel.encode())
         assert s("kg_rk4", 1)[0] == capi.KG_ECUDA
         assert s("kg_pirk2", 1)[0] == capi.KG_OK
+
+
+@pytest.mark.parametrize("method", ["kg_pirk2", "kg_pirk3", "kg_rk3", "kg_rk4"])
+def test_host_time_of_a_step_does_not_grow_with_the_planes(fake, method):
+    """the chunk rule runs at every launch: a step of a grid with many planes is
+    enqueued in the microseconds of its launches (about 50), not in a search over all
+    numbers of chunks (5 to 14 ms here)"""
+    with Solve(fake, 4, 5, 200000) as s:
+        best = 1.0
+        for _ in range(6):
+            t0 = time.perf_counter()
+            assert s(method, 1)[0] == capi.KG_OK
+            best = min(best, time.perf_counter() - t0)
+        assert best < 1e-3
+
+
+def test_chunk_rules_equal_the_search_over_all_numbers_of_chunks(tmp_path):
+    src, so = tmp_path / "c.cpp", str(tmp_path / "c.so")
+    src.write_text('#include "kg_chunk.h"\n'
+                   'extern "C" int phi(int p, int t, int s, int l) { return kg::phi_chunk(p, t, s, l); }\n'
+                   'extern "C" int pair(int p, int t) { return kg::pair_chunk(p, t); }\n')
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I", os.path.join(ROOT, "kg_b200", "csrc"), str(src),
+                    "-o", so], check=True)
+    lib = C.CDLL(so)
+
+    def search(planes, longest, cost):
+        tried = [-(-planes // n) for n in range(-(-planes // longest), planes + 1)]
+        return min(((cost(c, -(-planes // c)), i, c) for i, c in enumerate(tried)))[2]
+
+    for planes in [*range(1, 70), 128, 129, 256, 257, 333, 1025]:
+        for tiles in (1, 2, 3, 7, 12, 40, 90, 111, 148, 296, 297, 1000, 4321):
+            for slots, longest in ((296, 32), (444, 32), (296, 64)):
+                want = search(planes, longest, lambda c, m: max(tiles * m / slots + 0.25, 1.0) * (c + 1))
+                assert lib.phi(planes, tiles, slots, longest) == want
+            assert lib.pair(planes, tiles) == search(planes, 24, lambda c, m: ((tiles * m + 147) // 148 + 0.5) * (c + 3))
