@@ -878,14 +878,16 @@ bool run_stage(kg_solver* h, int kind, const kg::StageLaunch& L) {
 }
 
 // Who writes the ghost values of the RK stages that start from u as it is now: the
-// stages themselves on a state with filled seam planes and on grids below the pairs'
-// size, where the fill's launch behind each stage counts; on larger ones the
-// scattered stores cost as much as the fill.  us per RK4 step, fills / by the
-// stages: 40 x 9 x 17 37 / 24, 64 x 17 x 33 46 / 33, 256 x 17 x 33 68 / 53, 128 x 33 x 65
-// 111 / 101; in the paired and the mixed kernels, whose registers are full, it was
-// slower at every size (1024 x 65 x 129 1658 / 1938, mixed 1617 / 1663).
+// stages themselves on a state with filled seam planes, a fill behind each stage
+// otherwise.  us per step, fills / by the stages: RK4 60 x 60 x 60 120 / 88, 128 x 33 x
+// 65 107 / 100, 384 x 65 x 129 901 / 866, 2048 x 129 x 257 17470 / 17173; SSP-RK3 256 x 33 x
+// 65 112 / 108, 384 x 65 x 129 485 / 452, 1024 x 65 x 129 1148 / 1107, 2048 x 129 x 257
+// 8648 / 8455; of 47 grids the fills were the faster on two, 576 x 33 x 65 219 / 229 and
+// 640 x 33 x 65 233 / 237.  In the paired and the mixed kernels, whose registers are
+// full, the fills are faster at every size (1024 x 65 x 129 1658 / 1938, mixed 1617 /
+// 1663).
 int ghosts_by(const kg_solver* h) {
-  if (h->variant < 2 || !h->seam_filled || kg::rk4_pairs_pay(h->g)) return kg::GH_FILL;
+  if (h->variant < 2 || !h->seam_filled) return kg::GH_FILL;
   return h->p.bc_rmax == KG_INFLOW ? kg::GH_INFLOW : kg::GH_OUTFLOW;
 }
 

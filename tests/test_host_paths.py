@@ -192,3 +192,15 @@ def test_chunk_rules_equal_the_search_over_all_numbers_of_chunks(tmp_path):
                 want = search(planes, longest, lambda c, m: max(tiles * m / slots + 0.25, 1.0) * (c + 1))
                 assert lib.phi(planes, tiles, slots, longest) == want
             assert lib.pair(planes, tiles) == search(planes, 24, lambda c, m: ((tiles * m + 147) // 148 + 0.5) * (c + 3))
+
+
+@pytest.mark.parametrize("method", ["kg_rk3", "kg_rk4"])
+@pytest.mark.parametrize("grid", [(40, 9, 17), (128, 33, 65), (1024, 65, 129)])
+def test_stages_store_their_ghost_values_on_a_filled_state(fake, method, grid):
+    with Solve(fake, *grid) as s:
+        assert s("kg_set_rk4_pairs", 0)[0] == s("kg_set_graphs", 0)[0] == capi.KG_OK
+        assert s(method, 1)[0] == capi.KG_OK
+        fills = fake.fake_launches(b"ghost_kernel")
+        assert fills > 0
+        assert s(method, 3)[0] == capi.KG_OK
+        assert fake.fake_launches(b"ghost_kernel") == fills
