@@ -236,9 +236,12 @@ int kg_set_kernel_variant(kg_solver *h, int variant);
  * counterpart. */
 int kg_set_tile_rows(kg_solver *h, int rows);
 /* FP64 RK4 with stages 1, 2 and 3, 4 in one kernel each (forms 2 and 3): 0 never,
- * 1 on grids where it is the faster form (default), 2 always.  The same bits either
- * way; the first step after a kg_set_state runs the four stage kernels, which fill
- * the seam planes the pairs rely on.  No reference counterpart. */
+ * 1 where it is the faster form (default), 2 always.  The same bits either way.  The
+ * pairs put u into a second buffer, so the last of an odd number of steps needs a
+ * copy of u behind it; with 1 it runs by the four stage kernels where these are
+ * faster than that.  They also take the first step after a kg_set_state, which
+ * fills the seam planes the pairs rely on, and all steps of a handle whose device
+ * had no room for the pairs' pole rows.  No reference counterpart. */
 int kg_set_rk4_pairs(kg_solver *h, int mode);
 /* No reference counterpart (the reference stops on errors).  Exercises the
  * failure path every TMA-fed kernel takes when a bounded wait runs out, without

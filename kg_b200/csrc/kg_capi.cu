@@ -1283,13 +1283,15 @@ bool has_pole_rows(kg_solver* h) {
 int step_rk4(kg_solver* h, int nsteps) {
   int rc;
   if ((rc = ensure_rk(h, 3))) return rc;
+  // a last odd step by pairs: with a copy of u behind it
+  const bool odd_pairs = h->rk4_pairs == 2 || kg::rk4_pairs_and_copy_pay(h->g);
   for (int s = 0; s < nsteps;) {
-    if (!wants_pairs(h) || !has_pole_rows(h) || !h->seam_filled) {
+    if (!wants_pairs(h) || !has_pole_rows(h) || !h->seam_filled || (nsteps - s == 1 && !odd_pairs)) {
       rk4_step_single(h);
       ++s;
       continue;
     }
-    // two steps, u -> R1 -> u; a last odd one is copied back, as is u behind a refused second one
+    // two steps, u -> R1 -> u; behind an odd or a refused second one u is copied back
     if (!rk4_step_pairs(h, h->U, h->RK[0])) continue;
     ++s;
     if (s < nsteps && rk4_step_pairs(h, h->RK[0], h->U)) {
@@ -1559,10 +1561,12 @@ int run_steps(kg_solver* h, int which, int nsteps, int (*step)(kg_solver*, int))
   }
   int key = ((h->s_cur == 5) ? 1 : 0) + ((h->t_cur == 5) ? 2 : 0);
   if (!h->graphs[which][key].exec || h->graphs[which][key].gen != h->graph_gen) {
-    // one direct step first: buffers, kernel attributes and tensor-map encoders
-    // are set up outside of any capture
-    if ((rc = step(h, 1))) return rc;
-    nsteps -= 1;
+    // direct steps first: buffers, kernel attributes and tensor-map encoders are set
+    // up outside of any capture (two of FP64 RK4, which may take one step and two by
+    // different kernels)
+    const int direct = which == 3 ? 2 : 1;
+    if ((rc = step(h, direct))) return rc;
+    nsteps -= direct;
     if (nsteps < 2) return nsteps ? step(h, nsteps) : KG_OK;
     key = ((h->s_cur == 5) ? 1 : 0) + ((h->t_cur == 5) ? 2 : 0);
   }

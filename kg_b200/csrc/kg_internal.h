@@ -129,7 +129,9 @@ struct PairLaunch {
   int inflow;
 };
 int launch_rk4_pair(int pair, const PairLaunch& L, const double* rsg, int* err, cudaStream_t st);
-bool rk4_pairs_pay(const Grid& g);  // whether pairs beat the four stage kernels on this grid
+// whether pairs beat the four stage kernels on this grid, over two steps and in one step with a copy of u behind it
+bool rk4_pairs_pay(const Grid& g);
+bool rk4_pairs_and_copy_pay(const Grid& g);
 // the first stage's output (after its x fill) on the first and last interior theta
 // row, [side][variable][k][PI], into `pole`: 10 NK PI complex values
 void launch_pole_rows(int pair, const PairLaunch& L, const double* rsg, double2* pole, cudaStream_t st);

@@ -584,17 +584,27 @@ int pair_dispatch(int pair, const PairLaunch& L, const double* rsg, int* err, cu
 
 }  // namespace
 
-// The pairs pay from about 17 tile planes per SM on: below that the march is a
-// serial chain of planes twice as long as a single stage's, on a few SMs, and the
-// two pole-row launches show.  us per RK4 step, four stage kernels against two
-// pairs (tile planes per SM): 64 x 17 x 33 (1) 33 / 53, 128 x 33 x 65 (9) 101 / 121,
-// 256 x 33 x 65 (17) 191 / 181, 2000 x 17 x 33 (31) 377 / 285, 512 x 33 x 65 (33)
-// 317 / 298, 301 x 46 x 90 (40) 396 / 337, 512 x 65 x 129 (131) 1101 / 914, 1024 x 65 x
-// 129 (256) 2163 / 1643.
-bool rk4_pairs_pay(const Grid& g) {
-  const long long tiles = (long long)((g.NI - 2 + PO - 1) / PO) * ((g.NJ - 6 + 7) / 8);
-  return tiles * (g.Nz - 1) >= 17LL * 148;
+// About the time of an RK4 step by pairs over that by the four stage kernels, which
+// store their own ghost values: 0.68 for each point that the tiles' 28 x 8 columns
+// span over those of the grid, 0.2 where every tile lies at an r end (its warps take
+// the general path), and a start that shows below some tens of tile planes per SM.
+// Fitted to 49 grids, 22 x 65 x 513 to 2048 x 129 x 257.  us per step, pairs / stages
+// (tile planes per SM): 128 x 33 x 65 (9) 119 / 100, 64 x 65 x 129 (21) 230 / 197, 256 x
+// 33 x 65 (17) 177 / 181, 512 x 33 x 65 (33) 296 / 302, 301 x 46 x 90 (40) 334 / 377,
+// 64 x 129 x 257 (83) 711 / 674, 384 x 65 x 129 (97) 691 / 866, 1024 x 65 x 129 (256)
+// 1853 / 2149, 2048 x 129 x 257 (2048) 13064 / 17173.  On the wrong side of the line by
+// 1 to 8 %: 160 x 33 x 65, 320 x 33 x 65, 80 x 65 x 129, 1000 x 17 x 33.
+static double pair_time(const Grid& g) {
+  const int cols = g.NI - 2, rows = g.NJ - 6;
+  const int tx = (cols + PO - 1) / PO, ty = (rows + 7) / 8;
+  const double tiles = (double)tx * ty;
+  return 0.68 * tiles * (PO * 8) / ((double)cols * rows) + 3.5 * 148 / (tiles * (g.Nz - 1)) + 0.2 * (tx > 2 ? 2.0 / tx : 1.0);
 }
+bool rk4_pairs_pay(const Grid& g) { return pair_time(g) < 1.0; }
+// a step whose result has to be copied back from the second u buffer: us, pairs and
+// copy / stages: 512 x 33 x 65 338 / 301, 192 x 65 x 129 470 / 461, 576 x 33 x 65 362 / 405,
+// 384 x 65 x 129 793 / 855, 2048 x 129 x 257 14788 / 17160
+bool rk4_pairs_and_copy_pay(const Grid& g) { return pair_time(g) < 0.815; }
 
 int launch_rk4_pair(int pair, const PairLaunch& L, const double* rsg, int* err, cudaStream_t st) {
   return pair_dispatch<8>(pair, L, rsg, err, st);

@@ -194,6 +194,30 @@ def test_chunk_rules_equal_the_search_over_all_numbers_of_chunks(tmp_path):
             assert lib.pair(planes, tiles) == search(planes, 24, lambda c, m: ((tiles * m + 147) // 148 + 0.5) * (c + 3))
 
 
+@pytest.mark.parametrize("grid,two,one", [((64, 17, 33), 0, 0), ((64, 65, 129), 0, 0), ((512, 33, 65), 4, 0),
+                                          ((1024, 65, 129), 4, 2)])
+def test_rk4_steps_by_pairs_where_they_pay(fake, grid, two, one):
+    """pair kernels of two steps in a call and of one, which needs a copy of u as well"""
+    with Solve(fake, *grid) as s:
+        assert s("kg_set_graphs", 0)[0] == capi.KG_OK
+        assert s("kg_rk4", 1)[0] == capi.KG_OK  # fills the seam planes
+        for n, want in ((2, two), (1, one), (3, two + one), (1, one)):
+            before = fake.fake_launches(b"rk4_pair")
+            assert s("kg_rk4", n)[0] == capi.KG_OK
+            assert fake.fake_launches(b"rk4_pair") - before == want
+
+
+@pytest.mark.parametrize("n", range(2, 9))
+def test_rk4_kernels_run_once_ahead_of_their_capture(fake, n):
+    with Solve(fake, 512, 33, 65) as s:
+        before = [fake.fake_launches(k) for k in (b"rk4_pair", b"tma_stage")]
+        assert s("kg_rk4", n) == (capi.KG_OK, "")
+        steps = [fake.fake_launches(k) - b for k, b in zip((b"rk4_pair", b"tma_stage"), before)]
+        # one step that fills the seam planes, two direct ones, two in the capture, an odd last one by stages
+        left = n - 1 if n < 5 else 4 + (n - 3) % 2
+        assert steps == [4 * (left // 2), 4 * (1 + left % 2)]
+
+
 @pytest.mark.parametrize("method", ["kg_rk3", "kg_rk4"])
 @pytest.mark.parametrize("grid", [(40, 9, 17), (128, 33, 65), (1024, 65, 129)])
 def test_stages_store_their_ghost_values_on_a_filled_state(fake, method, grid):
