@@ -250,7 +250,9 @@ def engine_leg(reqs, device, tune, steps=10):
     import torch
     from kg_b200.serve import _make_solve
     from kg_b200.batch import Batch
-    pts = sum((r.Nr + 5) * (r.Ntheta + 6) * (2 * r.Ntheta + 2) for r in reqs)
+    from kg_b200.profile_cases import step_bytes
+    each = [(r.Nr + 5) * (r.Ntheta + 6) * (2 * r.Ntheta + 2) for r in reqs]
+    pts = sum(each)
     plain_ms = 0.0
     for r in reqs:
         s = _make_solve(r, 8, device)
@@ -283,7 +285,11 @@ def engine_leg(reqs, device, tune, steps=10):
             e1.synchronize()
             best = min(best, e0.elapsed_time(e1))
         out[f"batched_{prec}_ms"] = best
-        out[f"batched_{prec}_alg_gbs"] = pts * (1360 if prec == "fp64" else 880) * steps / (best / 1e3) / 1e9
+        # a persistent launch runs the four stages; in concurrent launches each solve's grid decides
+        per = [1360 if prec == "fp64" else 880] * len(solves)
+        if tune[prec].dispatch == 1:
+            per = step_bytes(solves[0]._lib, [s.handle for s in solves], lambda: b.rk4(2), 2)
+        out[f"batched_{prec}_alg_gbs"] = sum(n * v for n, v in zip(each, per)) * steps / (best / 1e3) / 1e9
         for s in solves:
             b.remove(s)
             s.close()

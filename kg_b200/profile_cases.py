@@ -54,7 +54,29 @@ def _device_ic(s, Nx, Ny, Nz, xmin, xmax, seed=7):
 STAGE_BYTES = {"stage_pirk_s1_fused": 176, "stage_pirk_s1_psi": 144, "stage_pirk_s1_pi": 112, "stage_pirk2_s2": 240,
                "stage_pirk3_s2_psi": 208, "stage_pirk3_s2_pi": 128, "stage_pirk3_s3": 240,
                "stage_rk3_1": 160, "stage_rk3_2": 240, "stage_rk3_3": 240,
-               "stage_rk4_1": 240, "stage_rk4_2": 400, "stage_rk4_3": 400, "stage_rk4_4": 320}
+               "stage_rk4_1": 240, "stage_rk4_2": 400, "stage_rk4_3": 400, "stage_rk4_4": 320,
+               "stage_rk4_12": 240, "stage_rk4_34": 320,
+               "mixed_rk4_1": 160, "mixed_rk4_2": 240, "mixed_rk4_3": 240, "mixed_rk4_4": 240}
+
+
+def step_bytes(lib, handles, run, steps):
+    """Algorithmic bytes per stored point and step that the stage kernels of each handle
+    move, counted over run(), which advances all of them by `steps` steps.  (What a
+    handle's steps launch depends on its grid: RK4 in pairs moves 560 B, in four
+    stages 1360.)"""
+    nk = lib.kg_profile_kinds()
+    names = [lib.kg_profile_kind_name(i).decode() for i in range(nk)]
+    ms, cnt = (C.c_double * nk)(), (C.c_longlong * nk)()
+    for h in handles:
+        lib.kg_profile_enable(h, 1)
+        lib.kg_profile_read(h, ms, cnt)
+    run()
+    out = []
+    for h in handles:
+        lib.kg_profile_read(h, ms, cnt)
+        lib.kg_profile_enable(h, 0)
+        out.append(sum(STAGE_BYTES.get(names[i], 0) * cnt[i] for i in range(nk)) / steps)
+    return out
 
 
 def _steppers(a):

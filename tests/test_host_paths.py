@@ -228,3 +228,21 @@ def test_stages_store_their_ghost_values_on_a_filled_state(fake, method, grid):
         assert fills > 0
         assert s(method, 3)[0] == capi.KG_OK
         assert fake.fake_launches(b"ghost_kernel") == fills
+
+
+@pytest.mark.parametrize("grid,precision,want", [((64, 17, 33), 0, 1360), ((1024, 65, 129), 0, 560),
+                                                 ((1024, 65, 129), 1, 880)])
+def test_step_bytes_follow_the_kernels(fake, grid, precision, want):
+    from kg_b200.profile_cases import step_bytes
+    with Solve(fake, *grid) as s:
+        b = C.c_void_p()
+        assert fake.kg_batch_create(0, C.byref(b)) == fake.kg_batch_set_precision(b, precision) == capi.KG_OK
+        assert fake.kg_batch_set_dispatch(b, 1, -1) == fake.kg_batch_add(b, s.h) == fake.kg_batch_rk4(b, 1) == capi.KG_OK
+        assert step_bytes(fake, [s.h], lambda: fake.kg_batch_rk4(b, 2), 2) == [want]
+        fake.kg_batch_destroy(b)
+
+
+def test_every_stage_kernel_has_its_bytes(fake):
+    from kg_b200.profile_cases import STAGE_BYTES
+    names = [fake.kg_profile_kind_name(i).decode() for i in range(fake.kg_profile_kinds())]
+    assert {n for n in names if n.startswith(("stage_", "mixed_"))} == set(STAGE_BYTES)
