@@ -217,7 +217,6 @@ __device__ __forceinline__ void mx_rhs(const MxArgs& a, const TIN* cu, const dou
     const cx<R> ep = CX<R>(kept<R>(Epv.x), kept<R>(Epv.y)), en = CX<R>(kept<R>(Enx.x), kept<R>(Enx.y));
     cx<R> z;
     if (k == 0) z = add(neg(ep), en);
-    else if (k == g.Nz) z = add(neg(en), ep);
     else z = cc(ep, en);
     r[3] = sm(rdz, z);
   }
@@ -240,7 +239,6 @@ __device__ __forceinline__ void mx_rhs(const MxArgs& a, const TIN* cu, const dou
     const cx<R> fp = CX<R>(kept<R>(Fpv.x), kept<R>(Fpv.y)), fn = CX<R>(kept<R>(Fnx.x), kept<R>(Fnx.y));
     cx<R> z;
     if (k == 0) z = add(neg(fp), fn);
-    else if (k == g.Nz) z = add(neg(fn), fp);
     else z = cc(fp, fn);
     z = sm(rdz, z);
     const cx<R> r3 = (MK == MK_KS) ? dsg(z, sg, rs) : z;
@@ -314,7 +312,7 @@ __device__ __forceinline__ int mx_item(const CUtensorMap* tinp, const CUtensorMa
   auto plane_of = [&](int t) -> int {
     if (t == 0) return (k0 == 0) ? g.Nz - 2 : k0 - 1;
     if (t <= k1 - k0) return k0 + t - 1;
-    return (k1 - 1 == g.Nz) ? 2 : k1;
+    return k1;
   };
   auto slot = [&](int t) -> int { return (int)((tb + (uint32_t)t) % NST); };
   auto parity = [&](int t) -> uint32_t { return ((tb + (uint32_t)t) / NST) & 1u; };

@@ -60,7 +60,8 @@ namespace kg {
 using namespace tmaops;
 namespace {
 
-constexpr int PO = 28;      // own r columns of a tile (rows: 8)
+constexpr int PO = 28;      // own r columns of a tile
+constexpr int TJ = 8;       // and theta rows
 constexpr int PW = 36;      // ring and metric tile width: the 32 region columns +- 2
 constexpr int PST = 3;      // ring depth
 enum { PT_AL = 0, PT_BE, PT_A, PT_GRR, PT_GRP, PT_SG, PT_HT, PT_COUNT };
@@ -68,10 +69,9 @@ enum { PT_AL = 0, PT_BE, PT_A, PT_GRR, PT_GRP, PT_SG, PT_HT, PT_COUNT };
 // difference, each formed once by its own point
 enum { Y_P1 = 0, Y_AP, Y_E, Y_G, Y_H, Y_Q, Y_COUNT };
 
-// Shared memory of a tile with TJ own rows.  Of the Y planes and the metric tables
+// Shared memory of a tile.  Of the Y planes and the metric tables
 // only E, H and alpha, beta, (alpha sqrtg) gamma^thth are read beyond the own (the
 // region's) rows.
-template <int TJ>
 struct PGeom {
   static constexpr int WARPS = TJ + 2, ROWS = TJ + 4;
   static constexpr int FULL = ROWS * PW, PART = WARPS * PW;  // complex values per variable and plane
@@ -138,7 +138,6 @@ struct Own {  // metric at the thread's own point
   double al, be, dxb, sg, rs, am2, fa, fgrp, fgpp;
 };
 // phi-derivative arguments of the psi and Pi right-hand sides
-template <int MK>
 __device__ __forceinline__ double2 arg_e(const Own& o, double2 ps1, double2 pi) {
   return cadd(rmul(o.al, pi), rmul(o.be, ps1));
 }
@@ -257,11 +256,11 @@ __device__ __forceinline__ void pair_rhs_y(const Grid& g, const Own& o, int ii, 
 
 }  // namespace
 
-template <int PAIR, int MK, int TJ>
-__global__ void __launch_bounds__(PGeom<TJ>::WARPS * 32, 1)
+template <int PAIR, int MK>
+__global__ void __launch_bounds__(PGeom::WARPS * 32, 1)
     rk4_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmU,
                     const __grid_constant__ CUtensorMap tmA, PairArgs a) {
-  using GT = PGeom<TJ>;
+  using GT = PGeom;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* ring;
   {
@@ -362,9 +361,9 @@ __global__ void __launch_bounds__(PGeom<TJ>::WARPS * 32, 1)
   double2 yphi = Ep, ypi = Ep;                               // Y's phi and Pi at P[s-1]
   park += own ? (w - 1) * 32 + lane : 0;
   if (!timed_out) {
-    Ep = arg_e<MK>(o, XV(0, 1, 0, 0), XV(0, 4, 0, 0));
+    Ep = arg_e(o, XV(0, 1, 0, 0), XV(0, 4, 0, 0));
     Fp = arg_f<MK>(o, XV(0, 1, 0, 0), XV(0, 3, 0, 0));
-    Ec = arg_e<MK>(o, XV(1, 1, 0, 0), XV(1, 4, 0, 0));
+    Ec = arg_e(o, XV(1, 1, 0, 0), XV(1, 4, 0, 0));
     Fc = arg_f<MK>(o, XV(1, 1, 0, 0), XV(1, 3, 0, 0));
   }
   bool failed = __syncthreads_or(timed_out) != 0;
@@ -396,7 +395,7 @@ __global__ void __launch_bounds__(PGeom<TJ>::WARPS * 32, 1)
 #pragma unroll
           for (int v = 0; v < 5; ++v) un[v] = lds(a.base, v * fs + p);
         }
-        const double2 En = arg_e<MK>(o, XV(s + 1, 1, 0, 0), XV(s + 1, 4, 0, 0));
+        const double2 En = arg_e(o, XV(s + 1, 1, 0, 0), XV(s + 1, 4, 0, 0));
         const double2 Fn = arg_f<MK>(o, XV(s + 1, 1, 0, 0), XV(s + 1, 3, 0, 0));
         double2 r[5];
         pair_rhs<FAST, MK>(g, o, ii, RF, MT, RF(0, 0, 0), Ep, En, Fp, Fn, r);
@@ -547,10 +546,10 @@ bool encode_state(CUtensorMap* tm, const Grid& g, const double2* base, int cols,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int PAIR, int MK, int TJ>
+template <int PAIR, int MK>
 int pair_launch(const PairLaunch& L, const double* rsg, int* err, cudaStream_t st) {
-  using GT = PGeom<TJ>;
-  if (!allow_smem<rk4_pair_kernel<PAIR, MK, TJ>>(GT::SMEM)) return -1;
+  using GT = PGeom;
+  if (!allow_smem<rk4_pair_kernel<PAIR, MK>>(GT::SMEM)) return -1;
   const Grid& g = L.g;
   CUtensorMap tmX, tmU, tmA;
   if (!encode_state(&tmX, g, L.X, PW, GT::ROWS) || !encode_state(&tmU, g, L.base, 32, GT::WARPS) ||
@@ -570,18 +569,9 @@ int pair_launch(const PairLaunch& L, const double* rsg, int* err, cudaStream_t s
   dim3 grid((g.NI - 2 + PO - 1) / PO, (g.NJ - 6 + TJ - 1) / TJ, 1);
   a.kchunk = pair_chunk(g.Nz - 1, (long long)grid.x * grid.y);
   grid.z = (g.Nz - 1 + a.kchunk - 1) / a.kchunk;
-  return launch_pdl_or_refuse(rk4_pair_kernel<PAIR, MK, TJ>, grid, dim3(32, GT::WARPS), GT::SMEM, st, tmX, tmU,
+  return launch_pdl_or_refuse(rk4_pair_kernel<PAIR, MK>, grid, dim3(32, GT::WARPS), GT::SMEM, st, tmX, tmU,
                               tmA, a);
 }
-template <int TJ>
-int pair_dispatch(int pair, const PairLaunch& L, const double* rsg, int* err, cudaStream_t st) {
-  if (pair == 0)
-    return L.metric_kind == MK_KS ? pair_launch<0, MK_KS, TJ>(L, rsg, err, st)
-                                  : pair_launch<0, MK_SCHW, TJ>(L, rsg, err, st);
-  return L.metric_kind == MK_KS ? pair_launch<1, MK_KS, TJ>(L, rsg, err, st)
-                                : pair_launch<1, MK_SCHW, TJ>(L, rsg, err, st);
-}
-
 }  // namespace
 
 // About the time of an RK4 step by pairs over that by the four stage kernels, which
@@ -596,9 +586,10 @@ int pair_dispatch(int pair, const PairLaunch& L, const double* rsg, int* err, cu
 // 1 to 8 %: 160 x 33 x 65, 320 x 33 x 65, 80 x 65 x 129, 1000 x 17 x 33.
 static double pair_time(const Grid& g) {
   const int cols = g.NI - 2, rows = g.NJ - 6;
-  const int tx = (cols + PO - 1) / PO, ty = (rows + 7) / 8;
+  const int tx = (cols + PO - 1) / PO, ty = (rows + TJ - 1) / TJ;
   const double tiles = (double)tx * ty;
-  return 0.68 * tiles * (PO * 8) / ((double)cols * rows) + 3.5 * 148 / (tiles * (g.Nz - 1)) + 0.2 * (tx > 2 ? 2.0 / tx : 1.0);
+  const double padding = tiles * (PO * TJ) / ((double)cols * rows), ends = tx > 2 ? 2.0 / tx : 1.0;
+  return 0.68 * padding + 3.5 * 148 / (tiles * (g.Nz - 1)) + 0.2 * ends;
 }
 bool rk4_pairs_pay(const Grid& g) { return pair_time(g) < 1.0; }
 // a step whose result has to be copied back from the second u buffer: us, pairs and
@@ -607,7 +598,9 @@ bool rk4_pairs_pay(const Grid& g) { return pair_time(g) < 1.0; }
 bool rk4_pairs_and_copy_pay(const Grid& g) { return pair_time(g) < 0.815; }
 
 int launch_rk4_pair(int pair, const PairLaunch& L, const double* rsg, int* err, cudaStream_t st) {
-  return pair_dispatch<8>(pair, L, rsg, err, st);
+  if (pair == 0)
+    return L.metric_kind == MK_KS ? pair_launch<0, MK_KS>(L, rsg, err, st) : pair_launch<0, MK_SCHW>(L, rsg, err, st);
+  return L.metric_kind == MK_KS ? pair_launch<1, MK_KS>(L, rsg, err, st) : pair_launch<1, MK_SCHW>(L, rsg, err, st);
 }
 
 }  // namespace kg
