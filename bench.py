@@ -44,13 +44,13 @@ sys.path.insert(0, ROOT)
 WORKLOAD = dict(Nx=2048, Ny=129, Nz=257, xmin=1.8, xmax=400.0, m=0.3, CFL=0.25, seed=20240601)
 METRIC = "RK point-updates/s (FP64 PIRK2, Nr=2048 x Ntheta=128 x Nphi=256)"
 UNIT = "GPSU/s"
-# algorithmic bytes per stored point of each PIRK2 kernel (complex128 = 16 B per variable)
+# algorithmic bytes per point of each PIRK2 kernel (complex128 = 16 B per variable), at the points that it
+# computes (profile_cases.stage_points: stage 2 leaves the rows and the plane of the ghost fill out)
 #   stage_pirk_s1_fused: read u (5 vars), stale u_stage(5); write u_stage(1:5) = 80 + 16 + 80
 #   stage_pirk_s1_psi  : read u (5 vars) + write u_stage(1:4)               = 80 + 64   (two-launch form)
 #   stage_pirk_s1_pi   : read u_stage(1:4), stale u_stage(5), u(5); write u_stage(5) = 64 + 16 + 16 + 16
 #   stage_pirk2_s2     : read u_stage, u_p(=u); write u                     = 80 + 80 + 80
 ALG_BYTES = {"stage_pirk_s1_fused": 176, "stage_pirk_s1_psi": 144, "stage_pirk_s1_pi": 112, "stage_pirk2_s2": 240}
-PIRK2_MIN_BYTES = 416  # fused minimum per point-step: read u, stale Pi, u_stage, u; write u_stage, u
 
 
 def workload_config(w):
@@ -250,9 +250,9 @@ def engine_leg(reqs, device, tune, steps=10):
     import torch
     from kg_b200.serve import _make_solve
     from kg_b200.batch import Batch
-    from kg_b200.profile_cases import step_bytes
-    each = [(r.Nr + 5) * (r.Ntheta + 6) * (2 * r.Ntheta + 2) for r in reqs]
-    pts = sum(each)
+    from kg_b200.profile_cases import stage_points, step_bytes
+    pts = sum((r.Nr + 5) * (r.Ntheta + 6) * (2 * r.Ntheta + 2) for r in reqs)
+    each = [stage_points("stage_rk4_1", r.Nr, r.Ntheta + 1, 2 * r.Ntheta + 1) for r in reqs]
     plain_ms = 0.0
     for r in reqs:
         s = _make_solve(r, 8, device)
@@ -767,6 +767,7 @@ def main():
     import torch
     from kg_b200 import ScalarField, replicas
     from kg_b200.initial_data import shell_ylm_device
+    from kg_b200.profile_cases import stage_points
 
     world, rank, local = replicas.rank_env()
     torch.cuda.set_device(local)
@@ -867,13 +868,14 @@ def main():
     dom = max(stage_kinds.items(), key=lambda kv: kv[1][0])[0] if stage_kinds else "stage_pirk2_s2"
     dms, dcnt = kinds.get(dom, (0.0, 1))
     peak, peak_kind = measured_peaks()
-    alg = ALG_BYTES.get(dom, 0) * stored_points(w)
+    alg_bytes = lambda k: ALG_BYTES.get(k, 0) * stage_points(k, w["Nx"], w["Ny"], w["Nz"])
+    alg = alg_bytes(dom)
     achieved = alg / (dms / dcnt / 1e3) / 1e9 if dcnt else 0.0
     tr = profile_traffic(dom)
     roofline = {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": peak_kind, "traffic": tr,
                 "algorithmic_bytes_per_launch": alg, "avg_launch_ms": dms / dcnt if dcnt else None}
-    step_bytes = PIRK2_MIN_BYTES * stored_points(w)
+    step_bytes = sum(alg_bytes(k) * v[1] for k, v in stage_kinds.items()) / args.steps  # the fill's are left out
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": el_ms / args.steps, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "c128", "data": "synthetic (seeded Gaussian shell x Y_lm, l<=4)",

@@ -50,17 +50,27 @@ def _device_ic(s, Nx, Ny, Nz, xmin, xmax, seed=7):
     s.synchronize()
 
 
-# algorithmic bytes per stored point of each stage kernel (FP64 complex: 16 B per variable)
+# algorithmic bytes per point of each stage kernel (FP64 complex: 16 B per variable), at the points of stage_points
 STAGE_BYTES = {"stage_pirk_s1_fused": 176, "stage_pirk_s1_psi": 144, "stage_pirk_s1_pi": 112, "stage_pirk2_s2": 240,
                "stage_pirk3_s2_psi": 208, "stage_pirk3_s2_pi": 128, "stage_pirk3_s3": 240,
                "stage_rk3_1": 160, "stage_rk3_2": 240, "stage_rk3_3": 240,
                "stage_rk4_1": 240, "stage_rk4_2": 400, "stage_rk4_3": 400, "stage_rk4_4": 320,
                "stage_rk4_12": 240, "stage_rk4_34": 320,
                "mixed_rk4_1": 160, "mixed_rk4_2": 240, "mixed_rk4_3": 240, "mixed_rk4_4": 240}
+# no ghost fill follows these, so they compute every stored point
+WHOLE_GRID = ("stage_pirk_s1_fused", "stage_pirk_s1_psi", "stage_pirk_s1_pi", "stage_pirk3_s2_psi",
+              "stage_pirk3_s2_pi")
+
+
+def stage_points(kind, Nx, Ny, Nz):
+    """points that a stage kernel computes: a stage with a ghost fill behind it leaves
+    out what the fill writes, six theta rows and one phi plane"""
+    rows, planes = (Ny + 5, Nz + 1) if kind in WHOLE_GRID else (Ny - 1, Nz)
+    return (Nx + 5) * rows * planes
 
 
 def step_bytes(lib, handles, run, steps):
-    """Algorithmic bytes per stored point and step that the stage kernels of each handle
+    """Algorithmic bytes per computed point and step that the stage kernels of each handle
     move, counted over run(), which advances all of them by `steps` steps.  (What a
     handle's steps launch depends on its grid: RK4 in pairs moves 560 B, in four
     stages 1360.)"""
@@ -90,7 +100,6 @@ def _steppers(a):
     lib = s._lib
     nk = lib.kg_profile_kinds()
     names = [lib.kg_profile_kind_name(i).decode() for i in range(nk)]
-    pts = (Nx + 5) * (Ny + 5) * (Nz + 1)
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     peaks = os.path.join(root, "MEASURED_PEAKS.json")
     peak = float(json.load(open(peaks)).get("hbm_gbs", 6650.0)) if os.path.exists(peaks) else 6650.0
@@ -112,7 +121,7 @@ def _steppers(a):
         for i in range(nk):
             if cnt[i]:
                 per = ms[i] / cnt[i]
-                b = STAGE_BYTES.get(names[i], 0) * pts
+                b = STAGE_BYTES.get(names[i], 0) * stage_points(names[i], Nx, Ny, Nz)
                 out[names[i]] = {"ms": round(per, 3), "hbm_frac": round(b / (per / 1e3) / 1e9 / peak, 3) if b else None}
         print(meth, json.dumps(out))
 

@@ -21,3 +21,18 @@ def test_stage_bytes_agree_with_bench():
     from kg_b200.profile_cases import STAGE_BYTES
     for k, v in bench.ALG_BYTES.items():
         assert STAGE_BYTES[k] == v
+
+
+def test_stage_points_leave_out_what_the_fill_writes():
+    """The launch that the committed counters belong to moves at least the bytes that
+    the roofline counts for it."""
+    sys.path.insert(0, ROOT)
+    import bench
+    from kg_b200.profile_cases import STAGE_BYTES, WHOLE_GRID, stage_points
+    w = bench.WORKLOAD
+    grid = (w["Nx"], w["Ny"], w["Nz"])
+    for k in STAGE_BYTES:
+        n = stage_points(k, *grid)
+        assert n == (bench.stored_points(w) if k in WHOLE_GRID else 2053 * 128 * 257)
+    counted = bench.ALG_BYTES["stage_pirk2_s2"] * stage_points("stage_pirk2_s2", *grid)
+    assert 1.0 <= bench.profile_traffic("stage_pirk2_s2") / counted < 1.1
