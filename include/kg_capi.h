@@ -232,8 +232,9 @@ long long kg_launch_count(const kg_solver *h);
 int kg_set_kernel_variant(kg_solver *h, int variant);
 /* theta rows of the TMA tiles of the RK4 stages (FP64 forms 2, 3 and the mixed
  * form): 8 (default; 32 x 8 tiles, 2 CTAs per SM) or 4 (32 x 4 tiles, 3 CTAs per
- * SM, twice the tiles per grid).  The same bits either way.  No reference
- * counterpart. */
+ * SM, twice the tiles per grid).  The same bits either way.  FP64 steps that run
+ * in pairs (kg_set_rk4_pairs) have one tile height and do not heed it.  No
+ * reference counterpart. */
 int kg_set_tile_rows(kg_solver *h, int rows);
 /* FP64 RK4 with stages 1, 2 and 3, 4 in one kernel each (forms 2 and 3): 0 never,
  * 1 where it is the faster form (default), 2 always.  The same bits either way.  The
@@ -271,7 +272,8 @@ int kg_batch_size(const kg_batch *b);
 /* rk4 (MoL/lines_method_lib.f90:411-474) for every member, nsteps times */
 int kg_batch_rk4(kg_batch *b, int nsteps);
 int kg_batch_synchronize(kg_batch *b);
-/* launch shape: phi planes per work item and persistent CTAs (the tuner's knobs) */
+/* launch shape: phi planes per work item, at most, and persistent CTAs (the tuner's
+ * knobs); the chunks are shortened where the list has few items per CTA */
 int kg_batch_set_tuning(kg_batch *b, int kchunk, int blocks);
 /* 0 = FP64 RK4 for every member (default), 1 = mixed precision as kg_set_precision */
 int kg_batch_set_precision(kg_batch *b, int mode);
@@ -293,8 +295,8 @@ int kg_batch_get_tuning(const kg_batch *b, int *kchunk, int *blocks);
 int kg_batch_set_dispatch(kg_batch *b, int dispatch, int variant);
 int kg_batch_get_dispatch(const kg_batch *b, int *dispatch, int *variant);
 /* theta rows of the TMA tiles (8 or 4, as kg_set_tile_rows): the persistent
- * launch's work items, and in dispatch 1 every member's RK4 stage kernels.  The
- * tuner's fifth knob. */
+ * launch's work items, and in dispatch 1 every member's RK4 stage kernels (not the
+ * pairs, where a member's steps run in those).  The tuner's fifth knob. */
 int kg_batch_set_tile_rows(kg_batch *b, int rows);
 int kg_batch_get_tile_rows(const kg_batch *b, int *rows);
 long long kg_batch_launch_count(const kg_batch *b);

@@ -15,7 +15,9 @@ the same grid shapes (the live solves are never advanced by the tuning):
   * dispatch 1, every member's own single-solve kernels on its own stream, all
     members concurrently: the stage-kernel form, i.e. the tile shape of the
     stage kernels (32 x 8 or 32 x 4 tiles fed by TMA, 32 x 8 tiles with
-    register prefetch, or one thread per point in rows of 128).
+    register prefetch, or one thread per point in rows of 128).  Members whose
+    FP64 steps run in pairs have one tile height: for them the two candidates
+    are the same.
 """
 from __future__ import annotations
 

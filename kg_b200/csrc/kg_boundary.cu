@@ -43,23 +43,20 @@ __device__ __forceinline__ int ghost_src_row(const Grid& g, int jj) {
 // rows 3..5 and NJ-6..NJ-4 of plane 0 as the stage left them, and C overwrites
 // those rows.  The C unit of such a row therefore reads it as well as its own
 // source, and writes both copies behind a block barrier (A leaves plane kp out).
-// What bounds it: on small grids the launch and the latency of one load-store
-// chain per thread, so one launch replaces the former two (ghost rows and faces,
-// then the phi planes); on large ones memory, 2 x 80 B per point of the ghost rows.
-// Event-timed, two launches before and one after: 301 x 46 x 90 21.5 -> 17.1 us,
-// 1024 x 65 x 129 43.1 -> 33.9 us (FP32 states 37.4 -> 22.1 us).  With the x faces
-// apart (PIRK2) 64 x 17 x 33 13.0 -> 12.1 us, 2048 x 129 x 257 123.8 -> 119.9 us.
+// What bounds it: on small grids the launch and the latency of a thread's loads, so
+// the whole sequence is one launch and a thread requests all that it reads, both
+// sources of a row of plane 0 among it, before it stores any of it; on large ones
+// memory, 2 x 80 B per point of the ghost rows.  Rows longer than a block are shared
+// among blocks (row_parts).  Event-timed, the faces' and rows' launch and the phi
+// planes' before, and now: 64 x 17 x 33 12.8 / 10.7 us (PIRK2, x faces apart), 301 x 46
+// x 90 21.0 / 12.1, 1024 x 65 x 129 43.1 / 32.0 (FP32 states 37.5 / 21.3), 2048 x 129 x
+// 257 125 / 121 (PIRK2).
 //
 // On a refined level the outermost planes then take the coarser level's values
 // (kg_refine.cuh): with WithProlong the same launch writes those instead, in A and C
-// for the ghost rows and planes 0 and Nz and in B for the interior rows (one launch
-// in the place of two: 384 x 33 x 65, four columns, 12.6 + 13.3 -> 17.9 us).  No
-// unit reads these columns: the x fill of the outermost one falls away.
-//
-// A thread requests all that it reads before it stores any of it, and the rows of
-// plane 0 read both their sources before either is written: one or two round trips
-// to memory a unit, where there were up to four (301 x 46 x 90: 17.9 -> 13.8 us with the rows shared out).
-// Rows longer than a block are shared among blocks (row_parts).
+// for the ghost rows and planes 0 and Nz and in B for the interior rows (384 x 33 x
+// 65, four columns, us in two launches and in one: 25.9 / 17.9).  No unit reads these
+// columns: the x fill of the outermost one falls away.
 
 // excision extrapolation 3 u1 - 3 u2 + u3; FP32 stage states form it in FP64
 __device__ __forceinline__ double2 excise(double2 a, double2 b, double2 c) {

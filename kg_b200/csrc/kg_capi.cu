@@ -902,8 +902,9 @@ int check_device_flag(kg_solver* h) {
   }
   return KG_OK;
 }
-// faces_apart: two launches instead of one; a PIRK2 step is four launches, a
-// count that kg_launch_count reports and its callers rely on
+// faces_apart: the x faces in a launch of their own.  PIRK2 keeps that: its tests
+// hold a step to four launches in kg_launch_count (no caller needs the number; in
+// one launch the fill of 64 x 17 x 33 would take about 2 us less)
 void run_ghost(kg_solver* h, double2* u, const double2* up, int inflow, bool faces_apart = false,
                bool cyclic = false) {
   Prof pf(h, PK_GHOST, faces_apart ? 2 : 1);

@@ -34,9 +34,10 @@ inline int best_chunk(int planes, int longest, F cost) {
 // a grid whose tiles alone leave SMs idle gets short chunks, a large one the
 // longest.  Constants fitted to a sweep of 19 lengths over ten grids from
 // 64 x 17 x 33 to 1024 x 65 x 129 (within 2 % of the best length on average, 14 %
-// at worst).  Against chunks of about 32 planes on every grid (64 in the fused PIRK stage 1),
-// us per launch: 64 x 17 x 33 PIRK2 stage 2 71 -> 12 and fused stage 1 94 -> 18,
-// 256 x 33 x 65 66 -> 37 and 103 -> 52, RK4 stage 2 98 -> 55.
+// at worst).  Event-timed us per launch with about 32 planes a chunk on every grid
+// (64 in the fused PIRK stage 1) and every stored row computed, and now, with these
+// chunks and the interior rows alone: 64 x 17 x 33 PIRK2 stage 2 53.7 / 11.2 and fused
+// stage 1 98.4 / 19.1, 256 x 33 x 65 78.4 / 37.2 and 103.0 / 47.4, RK4 stage 2 106 / 55.4.
 inline int phi_chunk(int planes, long long tiles, int slots, int longest) {
   return best_chunk(planes, longest, [&](int c, int m) {
     const double waves = (double)tiles * m / slots + 0.25;

@@ -3,8 +3,10 @@
 // boundary, with RK4.  The reference wires only second-order operators (its
 // fourth-order x stencil, first_derivative_x_4 in
 // tools/finite_differences.f90:124-154, is real-only and never called), so this
-// method is defined here and by the oracle's restatement of it, which this
-// code matches bit for bit:
+// method is defined here and by the oracle's restatement of it, which this code
+// matches to 1e-13 (multiply-adds are contracted, and the phi operators are formed
+// as differences and sums of the stored variables, weighted by the metric and
+// scaled afterwards; see cfg_phi):
 //   * D4 f = (f(-2) - 8 f(-1) + 8 f(+1) - f(+2)) / (12 h) in r, theta and phi;
 //     in r the one-sided closures of first_derivative_x_4 on the first and last
 //     two stored planes; theta on the interior rows (the +-2 rows of the first
@@ -15,7 +17,7 @@
 //     per direction on all five variables (r planes 3..N-3 only).
 //   * the outermost r plane obeys d_t u = -(d_r u + u / r) (Sommerfeld); the
 //     innermost planes (inside the horizon) evolve with the one-sided closures.
-//   * the theta ghost rows and the duplicated phi planes get a zero RHS and are
+//   * the theta ghost rows and the duplicated phi planes are not computed; they are
 //     refilled after every stage: the phi planes first, then the theta ghost
 //     rows from the interior rows at phi + pi with psi_2 negated (the parity of
 //     d_theta of a smooth function on the sphere); the theta flux
@@ -247,20 +249,17 @@ __global__ void __launch_bounds__(128) cfg_stage_kernel(CfgArgs a) {
 // arrives in shared memory with a +-4 r and +-3 theta halo (every same-plane
 // neighbour the fourth-order differences, the r closures and the sixth-order
 // dissipation touch), double buffered: one TMA box of all five variables brings
-// the next plane's tile while this plane is computed (eleven cp.async per thread
-// and plane, each with its index arithmetic, did before).  With that, only the
-// interior rows and planes, the point-wise operands requested together and the fill
-// in one launch, 20 RK4 steps on 256 x 33 x 65 went from 13.3 to 9.7 ms (a stage 164
-// -> 125 us).  The phi neighbours (planes k+-1..3 of the thread's own column) are plain
-// loads, and their latency from L2 bound it: read where the formulas name them, they
-// came in many short batches, some twice.  cfg_phi reads them first, ahead of the
-// wait for the tile, a variable's six together, and keeps seven sums of them: 9.64 ->
-// 7.92 ms, a stage 125 -> 99 us.  What bounds it now is the chain of one plane's
-// loads and fifteen stencils at 16 warps per SM.  Not kept: the point-wise operands
-// prefetched into L2 a plane ahead (7.99 ms), u^n staged in shared memory (9.2 ms,
-// with 8 KB of L1 left).  (Holding them in a rolling register window
-// instead needs 255 registers per thread and one CTA per SM, and ran the C0
-// grid at half the speed.)
+// the next plane's tile while this plane is computed.  The phi neighbours (planes
+// k+-1..3 of the thread's own column) are plain loads that come from L2 on every
+// plane; cfg_phi reads them ahead of the wait for the tile, a variable's six
+// together, and keeps seven sums of them.  What bounds it is the chain of one
+// plane's loads and fifteen stencils at 16 warps per SM.  256 x 33 x 65, event-timed
+// us of stages 1 to 4: with cp.async tiles of every row and the neighbours loaded
+// where the formulas name them 142, 171, 169, 166; now 86, 94, 94, 90 (an RK4 step
+// with its fills 0.612 / 0.365 ms).  Slower: the point-wise operands prefetched into
+// L2 a plane ahead (20 steps 7.99 ms for 7.92), u^n staged in shared memory (9.2 ms,
+// with 8 KB of L1 left), and the neighbours in a rolling register window (255
+// registers per thread, one CTA per SM: half the speed).
 constexpr int CTI = 32, CTJ = 8, CRH = 4, CTH = 3;
 constexpr int CW = CTI + 2 * CRH, CH = CTJ + 2 * CTH, CT_N = CW * CH;
 constexpr size_t CFG_TILE_BYTES = (size_t)5 * CT_N * sizeof(double2);
@@ -329,8 +328,8 @@ __global__ void __launch_bounds__(CTI * CTJ, 2)
 // The method's fill: phi planes 0 <- Nz-1 and Nz <- 1, then the theta ghost rows
 // from the interior rows at phi + pi, psi_2 negated.  One launch, a block per row:
 // a ghost row whose partner is plane 0 reads plane Nz-1, its source, so no row that
-// is read is written (event-timed on 256 x 33 x 65, two launches before: 19.0 ->
-// 8.9 us).
+// is read is written (256 x 33 x 65, event-timed us in two launches and in one: 20.6 /
+// 8.8).
 __global__ void cfg_ghost_kernel(Grid g, double2* u) {
   pdl_wait();
   const int nz = 2 * (g.NJ - 6);  // interior rows of the two planes

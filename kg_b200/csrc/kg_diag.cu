@@ -4,7 +4,9 @@
 //
 // All reductions are deterministic: each block reduces its slice with warp
 // shuffles (FP64) into one partial, and a single block adds the partials in
-// a fixed order.  No atomics, so a result does not depend on scheduling.
+// a fixed order.  In the mass integral that is the block that finishes last,
+// elected by an atomic counter: which block adds depends on the scheduling, the
+// order of the additions and so the result do not.
 #include "kg_device.cuh"
 #include "kg_internal.h"
 #include "kg_diag.h"
@@ -89,12 +91,11 @@ int mass_blocks(const Grid& g) { return 148 * 4; }  // one wave at 4 CTAs (64 re
 // Each warp takes whole (theta, phi) rows in turn and its lanes stride along r
 // with eight independent loads of rho (and of sqrt(gamma)) in flight, so the
 // loads are coalesced and no per-point index division is needed; the block
-// count is fixed, so the partial sums (and the result) do not depend on the
-// device.
+// count follows from the grid, so the partial sums (and the result) do not depend
+// on the device.
 // One launch: the CTA that finishes last (a counter behind a fence, cleared for
-// the next call) adds the partials, in the same fixed order as a second launch
-// would.  A grid with fewer rows than 8 per CTA leaves the surplus CTAs out; their
-// partials were zero.
+// the next call) adds the partials in a fixed order.  A grid with fewer than 8 rows
+// for each CTA of a full wave launches fewer.
 struct MassSum {
   double value;
   unsigned int left;
@@ -181,10 +182,10 @@ void launch_mass(const Grid& g, const Metric& m, const double* rho, double dxdyd
 // computed once on the host with the reference's arithmetic and passed in.
 //   src: 0 = phi, 1..3 = j_i * sqrtg (currents_ADM, diagnostic_lib.f90:219-229)
 // One thread forms every field asked for (bit 0: phi, bits 1..3: the currents)
-// at its vertex: the eight corners' values are loaded once, as independent loads,
-// where a launch per field read them again behind a launch each.  The kernel is
-// bound by that one latency on the grids that are sampled every few steps: four
-// fields on 64 x 17 x 33, five detectors, 31 -> 8.7 us event-timed.
+// at its vertex: the eight corners' values are loaded once, as independent loads.
+// The kernel is bound by that one latency on the grids that are sampled every few
+// steps: four fields on 64 x 17 x 33, five detectors, event-timed us in a launch per
+// field and in one: 31 / 8.7.
 template <int MASK>
 __global__ void shell_interp_kernel(Grid g, Metric m, const double2* u, ShellInterp si, int Ny, int Nz,
                                     double2* out) {

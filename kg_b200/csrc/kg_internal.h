@@ -29,12 +29,12 @@ enum StageKind {
 // kernel before it on the stream finish (programmatic dependent launch), so that
 // the launch, the barrier set-up and the load of the metric tile, which no kernel
 // writes, do not wait for the full drain.  Such a kernel calls pdl_wait() before
-// it touches anything that earlier work on the stream writes or reads, in every
-// block.  No kernel releases its successor early: with a release at the start
-// the waiting blocks took the slots unevenly and everything got slower (256 x 33
-// x 65 PIRK2 94 -> 104 us a step).  us a pass, without -> with: 40 evolve steps on
-// 64 x 17 x 33 4070 -> 3960, 60 PIRK2 steps on 256 x 33 x 65 5520 -> 5440, three
-// levels of RK4 on 512 x 33 x 65 9640 -> 9290; nothing on the largest grids.
+// it touches anything that earlier work on the stream writes or reads; a block may
+// leave without it only when it touches nothing.  No kernel releases its successor
+// early: waiting blocks would take the slots unevenly (256 x 33 x 65 PIRK2, us a
+// step with a release at the start and without: 104 / 94).  us a pass, without and
+// with: 40 evolve steps on 64 x 17 x 33 4070 / 3960, three levels of RK4 on 512 x 33 x
+// 65 9640 / 9290; nothing on the largest grids.
 template <class... P, class... A>
 inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                               const A&... args) {

@@ -118,9 +118,9 @@ __device__ __forceinline__ cx<R> ld2(const T* p) {
 // What a thread keeps in arithmetic type R across planes (its own point's metric,
 // the phi-derivative arguments) lies in FP64 registers, as FP32 bit patterns for
 // R = float: a value is converted once, not at each use.  Conversions from and to 64
-// bits bound stage 1, whose ring is FP64 (their pipe 63 % busy, the next one 19 %).
-// With this and the FP32 metric tiles in every stage, 1024 x 65 x 129: stage 1 325 ->
-// 307 us, the others (240 B a point, 0.92 of the copy bandwidth) as before.
+// bits bound stage 1, whose ring is FP64 (with a conversion at each use their pipe
+// was 63 % busy and 1024 x 65 x 129 took 325 us, now 305); the others are bound by
+// memory (379, 379 and 368 us, 0.84 to 0.86 of the copy bandwidth for 240 B a point).
 template <class R>
 __device__ __forceinline__ R kept(double v);
 template <>

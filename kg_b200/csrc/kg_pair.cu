@@ -17,11 +17,13 @@
 // so lanes 2..29 of warps 1..TJ are the tile's own points.  Per plane P[s]:
 //   * X arrives by TMA (one box of all five variables, +-2 columns and +-1 row
 //     around the region) in a 3-deep ring with one "full" mbarrier per slot;
-//   * every warp forms Y of P[s] at its region points and puts psi1..3 and Pi into
-//     a double-buffered plane in shared memory;
+//   * every warp forms Y of P[s] at its region points and puts psi1 and the five
+//     products of Y with the metric that neighbours difference into a
+//     double-buffered plane in shared memory, each formed once by its own point;
 //   * the own points form the second right-hand side of P[s-1] from that plane's
-//     Y, with the phi neighbours' arguments, u and the first increment kept in
-//     registers;
+//     products, with the phi neighbours' arguments in registers.  The first
+//     increment (pair 0) or the increment sum (pair 1) of P[s-1] waits in shared
+//     memory, and so does u in pair 0; pair 1 reads u again;
 //   * one block barrier orders the Y planes and frees X's slot.
 // The ghost values of Y that the reference's boundary() would put in between:
 //   r: the excision extrapolation and the outer copy (or hold) come from the lanes
@@ -38,18 +40,17 @@
 // their order, so the results are the same bits.
 //
 // What bounds it: not memory (30 % of the HBM rate) but the latency of the two
-// dependent right-hand sides at 10 warps per SM, all that the X ring, the Y planes
-// and the metric tile leave room for (FP64 pipe 33 % busy, then LDS latency and the
-// barrier).  On 1024 x 65 x 129, pair 0 / pair 1 in us: tiles of 4 rows, two CTAs per
-// SM 809 / 1099; 8 rows 787 / 990; with Y's products with the metric formed once by
-// their own point instead of by each neighbour, and the increment sum parked in
-// shared memory, 697 / 867; with u parked too (pair 0) or read again where it is
-// used (pair 1), so that little spills, 686 / 864 (301 x 46 x 90: 141 / 186 -> 137 /
-// 175).  Stage kernels with their fills: 1020 and 1089.  Measured and not kept: the
-// march in copies per warp role 781 / 993 (instruction fetch), the second right-hand
-// side ahead of the Y stores 736 / 1039, tiles of 10 rows 712 / 1033, pair 1's u
-// parked 686 / 896 or in registers 686 / 934, ghost values stored by the pairs
-// instead of a fill (a whole step 1658 -> 1938).
+// dependent right-hand sides at 10 warps per SM, all that the X ring, the Y planes,
+// the parked values and the metric tile leave room for (FP64 pipe 33 % busy, then
+// LDS latency and the barrier).  Event-timed us, the two stage kernels, which store
+// their ghost values, and the pair, whose fill and pole rows take 32 us each (13 on
+// the second grid) on top: 1024 x 65 x 129 1036 / 693 and 1116 / 868, 301 x 46 x 90
+// 188 / 137 and 205 / 174.  Why this split (1024 x 65 x 129, pair 0 / pair 1 of the variant against
+// the same form otherwise): tiles of 4 rows with two CTAs per SM 809 / 1099 for 787 /
+// 990; products formed by each neighbour and the sum in registers 787 / 990 for 697 /
+// 867; tiles of 10 rows 712 / 1033, the march in copies per warp role 781 / 993 and
+// the second right-hand side ahead of the Y stores 736 / 1039 for 686 / 864; ghost
+// values stored by the pairs 1938 us a step for 1658.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include "kg_device.cuh"
@@ -578,7 +579,7 @@ int pair_launch(const PairLaunch& L, const double* rsg, int* err, cudaStream_t s
 // store their own ghost values: 0.68 for each point that the tiles' 28 x 8 columns
 // span over those of the grid, 0.2 where every tile lies at an r end (its warps take
 // the general path), and a start that shows below some tens of tile planes per SM.
-// Fitted to 49 grids, 22 x 65 x 513 to 2048 x 129 x 257.  us per step, pairs / stages
+// Fitted to 47 grids, 22 x 65 x 513 to 2048 x 129 x 257.  us per step, pairs / stages
 // (tile planes per SM): 128 x 33 x 65 (9) 119 / 100, 64 x 65 x 129 (21) 230 / 197, 256 x
 // 33 x 65 (17) 177 / 181, 512 x 33 x 65 (33) 296 / 302, 301 x 46 x 90 (40) 334 / 377,
 // 64 x 129 x 257 (83) 711 / 674, 384 x 65 x 129 (97) 691 / 866, 1024 x 65 x 129 (256)

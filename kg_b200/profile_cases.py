@@ -17,7 +17,7 @@ L2, so a profiler capture of one launch is representative and ends quickly.
   mixed:      RK4 with the FP32 stencil RHS and FP64 update (mixed_rk4_* kernels)
   proj:       the all-shell Y_lm projection on the tensor cores, K times
               (split-BF16 tcgen05 GEMM, ylm_gemm_kernel)
-  configured: RK4 of the fourth-order method (cfg_stage_kernel)
+  configured: RK4 of the fourth-order method (cfg_march_kernel)
   batch:      a request mix advanced as one batch (tma_batch_kernel /
               mx_batch_kernel, persistent over a ragged work list): the serving
               mix (Nr 128..512, Ntheta 16/32) or the batching-form mix
