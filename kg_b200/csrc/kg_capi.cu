@@ -2111,7 +2111,7 @@ int kg_load_checkpoint(kg_solver* h, const char* path) {
     why = "checkpoint method (scheme, Kreiss-Oliger eps) differs from the handle's; call kg_set_scheme first";
   else if (hd.precision != h->precision)
     why = "checkpoint precision mode differs from the handle's; call kg_set_precision first";
-  else if (hd.has_stage < 0 || hd.has_stage > 1 || hd.has_stage2 < 0 || hd.has_stage2 > 1)
+  else if (hd.has_stage < 0 || hd.has_stage > 1 || hd.has_stage2 < 0 || hd.has_stage2 > 1 || !(hd.dt > 0.0))
     why = "checkpoint header is corrupt";
   if (!why.empty()) {
     fclose(f);
@@ -2152,8 +2152,7 @@ int kg_load_checkpoint(kg_solver* h, const char* path) {
   }
   KG_CK(cudaStreamSynchronize(h->stream));
   h->t = hd.t;
-  h->dt = hd.dt;
-  return KG_OK;
+  return kg_set_dt(h, hd.dt);
 }
 
 int kg_get_detectors(kg_solver* h, double* r_det, int* index_det) {

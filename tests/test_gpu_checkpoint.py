@@ -121,3 +121,20 @@ def test_truncated_checkpoint_leaves_the_handle_untouched(tmp_path):
         b.read_from_check_point(cut)
     assert np.array_equal(b.u, before)
     assert b.t == t_before
+
+
+def test_resume_takes_the_time_step_of_the_file(tmp_path):
+    """a checkpoint of a solve with a time step of its own, into a handle with the
+    reference's: the steps, not the clock alone, take the file's"""
+    a = _solver()
+    a.dt = 0.5 * a.dt
+    a.rk4(nsteps=3)
+    path = tmp_path / "ckpt.bin"
+    a.check_point(path)
+    a.rk4(nsteps=4)
+    b = _solver()
+    b.rk4(nsteps=5)  # the graph of its own time step is there already
+    b.read_from_check_point(path)
+    b.rk4(nsteps=4)
+    assert np.array_equal(a.u, b.u)
+    assert a.t == b.t
