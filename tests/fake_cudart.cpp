@@ -13,7 +13,6 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
-#include <set>
 #include <string>
 #include <utility>
 #include <vector>
@@ -41,11 +40,10 @@ thread_local std::vector<Config> pushed;
 
 std::map<const void*, std::string> names;                // host stub -> kernel
 std::map<std::pair<int, const void*>, size_t> smem_set;  // (device, kernel) -> bytes
-std::map<const void*, int> alloc_device;
 std::map<std::string, int> launched;
-std::string refused_kernel, log_text;
+std::string refused_kernel;
 size_t refused_size = 0;
-int refused_count = 0, capture_allocs = 0, device_syncs = 0;
+int refused_count = 0, capture_allocs = 0;
 uintptr_t next_addr = (uintptr_t)1 << 44;
 
 cudaError_t fail(cudaError_t e) {
@@ -87,7 +85,6 @@ void* address(size_t n) {
   std::lock_guard<std::recursive_mutex> lock(mu);
   const uintptr_t p = next_addr;
   next_addr += (n + 511) / 256 * 256;
-  alloc_device[reinterpret_cast<void*>(p)] = device;
   return reinterpret_cast<void*>(p);
 }
 
@@ -100,7 +97,7 @@ void fake_reset() {
   std::lock_guard<std::recursive_mutex> lock(mu);
   refused_kernel.clear();
   refused_size = 0;
-  refused_count = capture_allocs = device_syncs = 0;
+  refused_count = capture_allocs = 0;
   launched.clear();
   last = cudaSuccess;
 }
@@ -121,7 +118,8 @@ int fake_last_error() { return (int)last; }
 void** __cudaRegisterFatBinary(void* f) { return reinterpret_cast<void**>(f); }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
-void __cudaRegisterFunction(void**, const char* stub, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*) {
+void __cudaRegisterFunction(void**, const char* stub, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*,
+                            int*) {
   names[stub] = name;
 }
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
@@ -169,10 +167,7 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
   *v = a == cudaDevAttrComputeCapabilityMajor ? 10 : a == cudaDevAttrMultiProcessorCount ? 148 : 0;
   return cudaSuccess;
 }
-cudaError_t cudaDeviceSynchronize() {
-  ++device_syncs;
-  return cudaSuccess;
-}
+cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
 cudaError_t cudaGetLastError() {
   const cudaError_t e = last;
   last = cudaSuccess;
